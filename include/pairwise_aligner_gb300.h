@@ -243,9 +243,10 @@ pa_status pa_mlp_adam(float *w, void *w16, const float *grad, float *m1, float *
                       void *stream);
 pa_status pa_mlp_to_bf16(const float *src, int rows, int cols, int ld_dst, void *dst, void *stream);
 
-/* Pairs with at least `cells` = m * n cells are computed by whole thread blocks
- * (the warps of a block pipeline the pair's row passes) instead of one group of
- * lanes; default 2^20.  1 sends every pair there, UINT64_MAX none. */
+/* Pairs with at least `cells` = m * n cells are long: their row passes are spread over
+ * many warps (unitary DNA scores: one queue of passes for the whole GPU; other scores:
+ * the warps of a block) instead of running on one group of lanes; default 2^20.  1 makes
+ * every pair long, UINT64_MAX none. */
 pa_status pa_set_cta_threshold(pa_ctx *ctx, uint64_t cells);
 
 /* Calls the context keeps captured as CUDA graphs (replayed when a call repeats the
@@ -253,21 +254,21 @@ pa_status pa_set_cta_threshold(pa_ctx *ctx, uint64_t cells);
  * replayed is dropped first).  No counterpart in the reference. */
 pa_status pa_get_graph_count(const pa_ctx *ctx, uint32_t *out);
 
-/* Polls a CTA-mode progress wait makes after its first look before it gives up
+/* Polls a wait between the passes of a long pair makes after its first look before it gives up
  * (default 2^24, with a short sleep between polls).  A wait that gives up marks its
  * pair PA_RESULT_ERROR and the call returns PA_ERR_TIMEOUT; 0 gives up at the first
  * look (tests use it to exercise that path).  No counterpart in the reference. */
 pa_status pa_set_wait_limit(pa_ctx *ctx, uint32_t polls);
 
-/* Of those, pairs whose sequence2 has at most `max_rows` rows (few 512-row passes) run on
- * teams of 4 warps, two pairs per block, instead of all 8 warps of a block (beside
- * them, on the SMs their blocks release); default 12288 (24 passes), 0 keeps every
- * such pair on whole blocks. */
+/* Of the long pairs scored by byte comparison or a substitution matrix, those whose sequence2
+ * has at most `max_rows` rows (few 512-row passes) run on teams of 4 warps, two pairs per
+ * block, instead of all 8 warps of a block; default 12288 (24 passes), 0 keeps every such
+ * pair on whole blocks.  Also the row limit of team_full_frac in band mode. */
 pa_status pa_set_team_threshold(pa_ctx *ctx, uint32_t max_rows);
 
-/* Of those, pairs with at least `cells` cells and `min_rows` rows of sequence2 are
- * computed by clusters of 4 thread blocks (co-scheduled; their 32 warps pipeline the
- * pair's passes); defaults 2^28 and 8192. */
+/* Of the same pairs, and of the pairs band mode tries, those with at least `cells` cells and
+ * `min_rows` rows of sequence2 are computed by clusters of 4 thread blocks (co-scheduled;
+ * their 32 warps pipeline the pair's passes); defaults 2^28 and 8192. */
 pa_status pa_set_cluster_threshold(pa_ctx *ctx, uint64_t cells, uint32_t min_rows);
 
 /* Substitution-matrix scoring (configuration/score_model_matrix.hpp:203-222,
@@ -288,9 +289,8 @@ pa_status pa_set_substitution_matrix(pa_ctx *ctx, const uint8_t *symbols, uint32
  * computed by the full DP.  margin scales the learned starting width;
  * straight_w0 is the starting width of band_mode 2.  Pairs of at most
  * pa_set_team_threshold rows use team_full_frac instead of full_frac (0: full_frac):
- * their full DP runs on teams of 4 warps, fast enough that a band pays only when it
- * is much narrower than the matrix.  The full DP of long pairs is routed as in the
- * plain path (teams, whole blocks, clusters, at the same time). */
+ * their full DP is fast enough that a band pays only when it is much narrower than the
+ * matrix.  The full DP of long pairs runs as in the plain path. */
 typedef struct pa_band_options {
     float margin;               /* default 1.25 */
     int32_t w_min;              /* default 16   */

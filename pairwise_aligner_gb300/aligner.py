@@ -62,15 +62,15 @@ class Context:
             pass
 
     def set_cta_threshold(self, cells: int):
-        """Pairs with at least `cells` m*n cells run on whole thread blocks (1: all pairs)."""
+        """Pairs with at least `cells` m*n cells are long: many warps share their passes (1: all pairs)."""
         _lib.check(self.lib.pa_set_cta_threshold(self.ptr, int(cells)), self.ptr)
 
     def set_cluster_threshold(self, cells: int, min_rows: int = 8192):
-        """Of the block-mode pairs, those with at least `cells` cells and `min_rows` rows run on clusters."""
+        """Long pairs (byte comparison, matrix, band mode) of at least `cells` cells and `min_rows` rows run on clusters."""
         _lib.check(self.lib.pa_set_cluster_threshold(self.ptr, int(cells), int(min_rows)), self.ptr)
 
     def set_team_threshold(self, max_rows: int):
-        """Block-mode pairs whose sequence2 has at most `max_rows` rows run on 4-warp teams (0: none)."""
+        """Long pairs (byte comparison, matrix) of at most `max_rows` rows run on 4-warp teams (0: none)."""
         _lib.check(self.lib.pa_set_team_threshold(self.ptr, int(max_rows)), self.ptr)
 
     def graph_count(self) -> int:
@@ -80,7 +80,7 @@ class Context:
         return n.value
 
     def set_wait_limit(self, polls: int):
-        """Polls a CTA-mode progress wait makes before it gives up (default 2^24; 0: at the first look)."""
+        """Polls a wait between the passes of a long pair makes before it gives up (default 2^24; 0: at the first look)."""
         _lib.check(self.lib.pa_set_wait_limit(self.ptr, int(polls)), self.ptr)
 
     def set_substitution_matrix(self, symbols: bytes, scores):

@@ -160,20 +160,6 @@ __global__ void k_band_windows(const uint64_t *__restrict__ off1, const uint64_t
     }
 }
 
-// The full DP's work kind of each listed pair, as the plain path's classifier routes long
-// pairs: 2 clusters (m * n >= huge_cells and n >= huge_min_n), 0 teams of 4 warps (at most
-// team_max_n rows), 1 whole blocks.
-__global__ void k_size_code(const uint64_t *__restrict__ off1, const uint64_t *__restrict__ off2,
-                            const uint32_t *__restrict__ list, uint32_t count, int32_t team_max_n, int64_t huge_cells,
-                            int32_t huge_min_n, uint8_t *__restrict__ code)
-{
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const uint32_t id = list[k];
-    const int64_t m = (int64_t)(off1[id + 1] - off1[id]), n = (int64_t)(off2[id + 1] - off2[id]);
-    code[k] = (m * n >= huge_cells && n >= huge_min_n) ? 2 : (n <= team_max_n ? 0 : 1);
-}
-
 // Network outputs (16 floats per pair, 9 used) -> band: checkpoint diagonals
 // out[c] * (m + n) / 4 and, from the predicted deficit c2 = 2^(16 out[8]) - 1
 // (= smax (m + n) - 2 S), the starting half-width.  A path that leaves the band
@@ -373,14 +359,6 @@ void band_windows_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *
     if (count)
         k_band_windows<<<blocks((uint64_t)count * 32, 128), 128, 0, st>>>(
             off1, off2, list, count, spec, rows, shift, full_frac, team_frac, team_max_n, win, code, width_stats);
-}
-
-void size_code_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *off2, const uint32_t *list,
-                      uint32_t count, int32_t team_max_n, int64_t huge_cells, int32_t huge_min_n, uint8_t *code)
-{
-    if (count)
-        k_size_code<<<blocks(count, 256), 256, 0, st>>>(off1, off2, list, count, team_max_n, huge_cells, huge_min_n,
-                                                         code);
 }
 
 void band_decode_launch(cudaStream_t st, const float *out, const uint64_t *off1, const uint64_t *off2,

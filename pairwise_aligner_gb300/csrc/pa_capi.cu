@@ -6,9 +6,9 @@
 //   1. k_classify    class, bucket key, score tables and empty-pair results
 //   2. k_scan_*      exclusive scan of the bucket histogram (2^18 buckets)
 //   3. k_scatter     bucket sort of the pair ids (order inside a bucket is free)
-//   4. dp_kernel     persistent DP kernels per class (s16x2, s32, byte-compare),
-//                    each pulling warp units from its own device queue, longest first
-//   5. dp_kernel     s32 recomputation of s16 global results that failed their check
+//   4. persistent DP kernels per class (s16x2, s32, byte-compare), each pulling work from its own
+//      device queue, longest first: dp_short / dp_kernel for short pairs, dp_long for long ones
+//   5. s32 recomputation of s16 global results that failed their check
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,6 +54,7 @@ struct GraphKey {
     pa_config cfg;
     int32_t G[3], variant[3];      // the launch shapes the call was captured with
     uint32_t wait_limit;
+    uint32_t use_long;
     bool operator<(const GraphKey &o) const { return std::memcmp(this, &o, sizeof(GraphKey)) < 0; }
 };
 
@@ -61,6 +62,7 @@ struct GraphKey {
 struct GraphEntry {
     cudaGraphExec_t exec;
     uint64_t last_use;
+    uint64_t launches;
 };
 constexpr size_t kMaxGraphs = 8;   // captured calls kept per context; the least recently used goes first
 
@@ -72,9 +74,9 @@ struct pa_ctx {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
     cudaEvent_t ev_dp0 = nullptr, ev_dp1 = nullptr;   // bracket the DP kernels of the last call
-    cudaStream_t side = nullptr;                      // cluster-mode kernels run beside the others
+    cudaStream_t side = nullptr;                      // s16x2 long pairs (highest priority)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaStream_t side2 = nullptr;                     // team kernels run beside the CTA kernels
+    cudaStream_t side2 = nullptr;                     // s32 and byte-compare pairs
     cudaEvent_t ev_join2 = nullptr;
     uint8_t *pinned = nullptr;                        // page-locked host words for band mode's reads
     pa_options opt{};
@@ -82,13 +84,17 @@ struct pa_ctx {
     // device work buffers (grow only)
     DevBuf keys, order, hist, starts, cursor, sums, ranges, counts, qtab, boundary, rerun, counters, pstats;
     DevBuf slots;                 // short-pair kernel: 16-byte column slots, (seq1_bytes + n_pairs)
+    // long pairs (dp_long): queue words and launch counter, boundary cells, and per queue (s16x2,
+    // s32) the units' first tickets, finished passes, failed waits and records
+    DevBuf long_words, long_cells16, long_start[2], long_done[2], long_fail[2], long_rec[2];
+    bool use_long = false;        // this call's batch may hold long pairs
     DevBuf ring, rerun_long;      // CTA mode: boundary rows per block; s16 long pairs to redo in s32
     int32_t ring_m = 0;           // longest sequence1 the ring rows hold (0: no CTA mode yet)
     int ring_grid = 0;            // blocks of every CTA-mode launch
-    int64_t long_cells = 1ll << 20;   // pairs with at least this many cells use CTA mode
-    int64_t huge_cells = 1ll << 28;   // ... and with this many (and n >= huge_min_n) cluster mode
+    int64_t long_cells = 1ll << 20;   // pairs with at least this many cells are long
+    int64_t huge_cells = 1ll << 28;   // byte-compare and banded: ... and this many (and n >= huge_min_n): clusters
     int32_t huge_min_n = 8192;
-    int32_t team_max_n = 12288;       // CTA-mode pairs with at most this many rows run on 4-warp teams
+    int32_t team_max_n = 12288;       // byte-compare long pairs of at most this many rows run on teams
     uint32_t wait_limit = kSpinLimit; // polls of a CTA-mode progress wait before it gives up
     int64_t want_ring_m = 0;          // the next call's longest CTA-mode sequence1 (host: exact)
     DevBuf in_seq1, in_off1, in_seq2, in_off2, in_out;   // staging for the host-buffer entry points
@@ -219,7 +225,7 @@ pa_status check_config(pa_ctx *c, const pa_config *cfg, DpParams &P, ClassCfg &C
     C.huge_cells = c->huge_cells;
     C.huge_min_n = c->huge_min_n;
     C.team_max_n = c->team_max_n;
-    C.long_max_m = c->ring.p ? c->ring_m : 0;
+    C.long_max_m = c->use_long && c->ring.p ? c->ring_m : 0;
     C.qtab_s16 = 1;
     return PA_OK;
 }
@@ -260,6 +266,27 @@ void dp_short_launch_global(int G, int form, int grid, cudaStream_t st, const Dp
 int dp_short_occupancy_free(int G);
 void dp_short_launch_free(int G, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
 
+int dp_long_occupancy_local(bool lanes16);
+int dp_long_occupancy_global(bool lanes16);
+int dp_long_occupancy_free(bool lanes16);
+void dp_long_launch_local(bool, int, cudaStream_t, const DpLaunch &, const LongQueue &, const DpParams &);
+void dp_long_launch_global(bool, int, cudaStream_t, const DpLaunch &, const LongQueue &, const DpParams &);
+void dp_long_launch_free(bool, int, cudaStream_t, const DpLaunch &, const LongQueue &, const DpParams &);
+
+int dp_long_occupancy(bool lanes16, int mode)
+{
+    return mode == M_LOCAL ? dp_long_occupancy_local(lanes16)
+         : mode == M_GLOBAL ? dp_long_occupancy_global(lanes16) : dp_long_occupancy_free(lanes16);
+}
+
+void dp_long_launch(bool lanes16, int mode, int grid, cudaStream_t st, const DpLaunch &L, const LongQueue &Q,
+                    const DpParams &P)
+{
+    if (mode == M_LOCAL) dp_long_launch_local(lanes16, grid, st, L, Q, P);
+    else if (mode == M_GLOBAL) dp_long_launch_global(lanes16, grid, st, L, Q, P);
+    else dp_long_launch_free(lanes16, grid, st, L, Q, P);
+}
+
 int dp_short_occupancy(int G, int form, int mode)
 {
     return mode == M_LOCAL ? dp_short_occupancy_local(G, form)
@@ -297,8 +324,6 @@ void band_windows_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *
                          uint32_t count, const BandSpec *spec, int32_t rows, int shift, float full_frac,
                          float team_frac, int32_t team_max_n, int2 *win, uint8_t *code,
                          unsigned long long *width_stats);
-void size_code_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *off2, const uint32_t *list,
-                      uint32_t count, int32_t team_max_n, int64_t huge_cells, int32_t huge_min_n, uint8_t *code);
 void band_decode_launch(cudaStream_t st, const float *out, const uint64_t *off1, const uint64_t *off2,
                         uint64_t n_pairs, const DpParams &P, float margin, int32_t w_min, BandSpec *spec);
 void band_straight_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *off2, uint64_t n_pairs,
@@ -339,7 +364,8 @@ void warm_occupancy()
             for (int mode = 0; mode < 3; ++mode) dp_short_occupancy(g, form, mode);
 }
 
-void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const DpLaunch &L, const DpParams &P)
+void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const DpLaunch &L, const DpParams &P,
+                  cudaStream_t st)
 {
     int v = c->variant[slot];
     if (v >= kShortVariant) {
@@ -351,7 +377,7 @@ void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const D
             int per_sm = dp_short_occupancy(L.G, form, mode);
             if (c->opt.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)c->opt.blocks_per_sm);
             c->grid[slot] = per_sm * c->sm_count;
-            dp_short_launch(L.G, form, mode, c->grid[slot], c->stream, L, P);
+            dp_short_launch(L.G, form, mode, c->grid[slot], st, L, P);
             c->last_launches++;
             return;
         }
@@ -360,7 +386,57 @@ void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const D
     int per_sm = dp_occupancy(v, lanes16, gen, mode);
     if (c->opt.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)c->opt.blocks_per_sm);
     c->grid[slot] = per_sm * c->sm_count;
-    dp_launch(v, lanes16, gen, mode, c->grid[slot], c->stream, L, P);
+    dp_launch(v, lanes16, gen, mode, c->grid[slot], st, L, P);
+    c->last_launches++;
+}
+
+// Buffers of the long-pair kernel for a batch; the boundary cells start zeroed, so that no cell
+// carries a tag that a launch did not write.
+pa_status ensure_long(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
+{
+    pa_status s;
+    const void *words = c->long_words.p, *cells = c->long_cells16.p;
+    if ((s = ensure(c, c->long_words, 2 * sizeof(LongWords) + 8))) return s;
+    if (c->long_words.p != words) PA_CUDA(c, cudaMemsetAsync(c->long_words.p, 0, c->long_words.cap, c->stream));
+    if ((s = ensure(c, c->long_cells16, (b1 + n_pairs) * 16))) return s;
+    if (c->long_cells16.p != cells) PA_CUDA(c, cudaMemsetAsync(c->long_cells16.p, 0, c->long_cells16.cap, c->stream));
+    for (int k = 0; k < 2; ++k) {
+        const uint64_t units = k == 0 ? (n_pairs + 1) / 2 : n_pairs;
+        if ((s = ensure(c, c->long_start[k], (units + 1) * 4))) return s;
+        if ((s = ensure(c, c->long_done[k], units * 4))) return s;
+        if ((s = ensure(c, c->long_fail[k], units * 4))) return s;
+        if ((s = ensure(c, c->long_rec[k], units * sizeof(LongRecord)))) return s;
+    }
+    return PA_OK;
+}
+
+LongQueue long_queue(pa_ctx *c, int k, const DpParams &P)
+{
+    auto lane = [&](int32_t x) { return (uint32_t)std::abs(x) * (k == 0 ? 0x10001u : 1u); };
+    LongQueue q;
+    q.goea = lane(P.gap_open + P.gap_ext);
+    q.exta = lane(P.gap_ext);
+    q.goeh = lane(P.gap_open + P.gap_ext - P.shift);
+    q.exth = lane(P.gap_ext - P.shift);
+    q.words = (LongWords *)c->long_words.p + k;
+    q.start = (uint32_t *)c->long_start[k].p;
+    q.done = (uint32_t *)c->long_done[k].p;
+    q.fail = (uint32_t *)c->long_fail[k].p;
+    q.rec = (LongRecord *)c->long_rec[k].p;
+    q.cells = (ulonglong2 *)c->long_cells16.p;
+    return q;
+}
+
+int long_grid(pa_ctx *c, bool lanes16, int mode) { return dp_long_occupancy(lanes16, mode) * c->sm_count; }
+
+// The pass queues of one or two lists (s16x2 units, s32 units); a null list gets no block.
+void plan_long(pa_ctx *c, cudaStream_t st, const uint64_t *o1, const uint64_t *o2, int mode, const LongPlan *p16, const LongPlan *p32)
+{
+    unsigned long long *epoch = (unsigned long long *)((LongWords *)c->long_words.p + 2);
+    const LongPlan &a = p16 ? *p16 : *p32;
+    k_long_plan<<<p16 && p32 ? 2 : 1, 1024, 0, st>>>(a, p32 ? *p32 : a, o1, o2,
+                                                     (uint32_t)long_grid(c, true, mode) * (kBlock / 32),
+                                                     mode == M_LOCAL ? 8 : 4, epoch);
     c->last_launches++;
 }
 
@@ -401,17 +477,11 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
 {
     cudaStream_t st = c->stream;
     // counters: [0..3] group queues, [4] rerun count, [5] zero, [6] long rerun count, [8] error
-    // bits, [9..12] CTA queues, [13..15] cluster queues, [16..21] routing of the largest pairs
+    // bits, [9..12] long queues (s16x2, s32, byte-compare blocks, redo), [13] cluster and [14]
+    // team queue, [16..17] routing of the largest byte-compare pairs
     uint32_t *counters = (uint32_t *)c->counters.p;
     pa_status ps = enqueue_prep(c, P, C, s1, o1, b1, s2, o2, b2, out, n_pairs);
     if (ps) return ps;
-    const int cl_grid = c->ring.p ? dp_cluster_grid(true, false, P.local ? M_LOCAL : M_GLOBAL, c->ring_grid) : 0;
-    if (c->ring.p) {
-        k_route_huge<<<1, 1, 0, st>>>((const uint32_t *)c->counts.p, (uint32_t)(cl_grid / kClusterBlocks),
-                                      counters + 16);
-        c->last_launches++;
-    }
-
     const int mode = P.local ? M_LOCAL : ((P.last_column_free || P.last_row_free) ? M_GLOBAL_FREE : M_GLOBAL);
     DpLaunch L;
     std::memset(&L, 0, sizeof(L));
@@ -438,75 +508,80 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
     // inside a capture the record must become a graph node to fire on every replay
     const unsigned ev_flags = capturing == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     PA_CUDA(c, cudaEventRecordWithFlags(c->ev_dp0, st, ev_flags));
-    // s16x2 class
-    L.begin_ptr = ranges + K_S16; L.count_ptr = counts + K_S16; L.unit_counter = counters + 0; L.G = c->G[K_S16];
-    launch_class(c, K_S16, mode, true, false, L, P);
-    // s32 class
-    L.begin_ptr = ranges + K_S32; L.count_ptr = counts + K_S32; L.unit_counter = counters + 1; L.G = c->G[K_S32];
-    launch_class(c, K_S32, mode, false, false, L, P);
-    // byte-compare class
-    L.begin_ptr = ranges + K_GEN; L.count_ptr = counts + K_GEN; L.unit_counter = counters + 2; L.G = c->G[K_GEN];
-    launch_class(c, K_GEN, mode, false, true, L, P);
-    // the largest pairs, on the side stream forked after the group kernels: clusters of blocks
-    // per pair, beside the CTA-mode kernels below, which fill the SMs the clusters leave free
+    // Three branches run side by side after the bucket sort; each kernel finds its list empty or
+    // not on the device.  The long pairs' passes go to the side stream of the highest priority,
+    // so that they take the SMs first and the short pairs fill what their last passes leave.
+    const bool use_long = C.pass_queue != 0;
+    LongPlan plan[2];
+    if (use_long) {
+        for (int k = 0; k < 2; ++k)
+            plan[k] = LongPlan{(const uint32_t *)c->order.p, ranges + (k == 0 ? K_S16L : K_S32L),
+                               counts + (k == 0 ? K_S16L : K_S32L), k == 0 ? 2 : 1, long_queue(c, k, P)};
+        plan_long(c, st, o1, o2, mode, &plan[0], &plan[1]);
+    }
+    PA_CUDA(c, cudaEventRecord(c->ev_fork, st));
+    PA_CUDA(c, cudaStreamWaitEvent(c->side2, c->ev_fork, 0));
     DpLaunch LL = L;
-    if (c->ring.p) {
-        LL.ring = (Cell *)c->ring.p;
-        LL.ring_stride = (uint64_t)c->ring_m + 2;
-        LL.error = counters + 8;
-        LL.rerun_list = (uint32_t *)c->rerun_long.p;
-        LL.rerun_count = counters + 6;
-        LL.G = 32;
-        PA_CUDA(c, cudaEventRecord(c->ev_fork, st));
+    LL.error = counters + 8;
+    LL.rerun_list = (uint32_t *)c->rerun_long.p;
+    LL.rerun_count = counters + 6;
+    LL.G = 32;
+    if (use_long) {
         PA_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-        DpLaunch LC = LL;
-        LC.ring = cluster_ring(c);
-        const Klass hc[3] = {K_S16H, K_S32H, K_GENH};
-        for (int k = 0; k < 3; ++k) {
-            LC.begin_ptr = ranges + hc[k]; LC.count_ptr = counters + 16 + k; LC.unit_counter = counters + 13 + k;
-            PA_CUDA(c, dp_cluster_launch(k == 0, k == 2, mode, dp_cluster_grid(k == 0, k == 2, mode, c->ring_grid),
-                                         c->side, LC, P));
+        for (int k = 0; k < 2; ++k) {
+            LL.begin_ptr = plan[k].begin; LL.count_ptr = plan[k].count; LL.unit_counter = counters + 9 + k;
+            dp_long_launch(k == 0, mode, long_grid(c, k == 0, mode), k == 0 ? c->side : c->side2, LL, plan[k].Q, P);
+            c->last_launches++;
         }
         PA_CUDA(c, cudaEventRecord(c->ev_join, c->side));
     }
-    // long pairs: whole blocks per pair; their s16 results that fail the check are redone in s32
-    if (c->ring.p) {
-        const Klass lc[3] = {K_S16L, K_S32L, K_GENL}, hl[3] = {K_S16H, K_S32H, K_GENH};
-        for (int k = 0; k < 3; ++k) {
-            LL.begin_ptr = ranges + lc[k]; LL.count_ptr = counts + lc[k]; LL.unit_counter = counters + 9 + k;
-            LL.lead_order = (const uint32_t *)c->order.p;          // the largest pairs the router left here
-            LL.lead_begin_ptr = ranges + hl[k];
-            LL.lead_count_ptr = counters + 19 + k;
-            dp_cta_launch(k == 0, k == 2, mode, c->ring_grid, st, LL, P);
-        }
+    // s16x2 class
+    L.begin_ptr = ranges + K_S16; L.count_ptr = counts + K_S16; L.unit_counter = counters + 0; L.G = c->G[K_S16];
+    launch_class(c, K_S16, mode, true, false, L, P, st);
+    // s32 class
+    L.begin_ptr = ranges + K_S32; L.count_ptr = counts + K_S32; L.unit_counter = counters + 1; L.G = c->G[K_S32];
+    launch_class(c, K_S32, mode, false, false, L, P, c->side2);
+    // byte-compare class, its long pairs on clusters, whole blocks (which take the largest pairs
+    // that the router left them first) and teams of 4 warps
+    L.begin_ptr = ranges + K_GEN; L.count_ptr = counts + K_GEN; L.unit_counter = counters + 2; L.G = c->G[K_GEN];
+    launch_class(c, K_GEN, mode, false, true, L, P, c->side2);
+    if (use_long && c->ring.p) {
+        const int cl_grid = dp_cluster_grid(mode, c->ring_grid);
+        k_route_huge<<<1, 1, 0, c->side2>>>(counts, (uint32_t)(cl_grid / kClusterBlocks), counters + 16);
+        LL.ring_stride = (uint64_t)c->ring_m + 2;
+        LL.ring = cluster_ring(c);
+        LL.begin_ptr = ranges + K_GENH; LL.count_ptr = counters + 16; LL.unit_counter = counters + 13;
+        PA_CUDA(c, dp_cluster_launch(mode, cl_grid, c->side2, LL, P));
+        LL.ring = (Cell *)c->ring.p;
+        LL.begin_ptr = ranges + K_GENL; LL.count_ptr = counts + K_GENL; LL.unit_counter = counters + 11;
+        LL.lead_order = (const uint32_t *)c->order.p;
+        LL.lead_begin_ptr = ranges + K_GENH;
+        LL.lead_count_ptr = counters + 17;
+        dp_cta_launch(mode, c->ring_grid, c->side2, LL, P);
         LL.lead_order = nullptr;
-        LL.lead_begin_ptr = nullptr;
-        LL.lead_count_ptr = nullptr;
-        // long pairs with few passes: teams of 4 warps on a second side stream with their own
-        // ring rows, launched after the CTA-mode kernels so that those take the SMs first; the
-        // teams fill the SMs that the blocks of the longer pairs release
+        LL.lead_begin_ptr = LL.lead_count_ptr = nullptr;
+        c->last_launches += 3;
         if (C.team_max_n > 0) {
-            PA_CUDA(c, cudaStreamWaitEvent(c->side2, c->ev_fork, 0));
-            DpLaunch LT = LL;
-            LT.ring = team_ring(c);
-            const Klass mc[3] = {K_S16M, K_S32M, K_GENM};
-            for (int k = 0; k < 3; ++k) {
-                LT.begin_ptr = ranges + mc[k]; LT.count_ptr = counts + mc[k]; LT.unit_counter = counters + 22 + k;
-                dp_team_launch(k == 0, k == 2, mode, c->ring_grid, c->side2, LT, P);
-            }
-            PA_CUDA(c, cudaEventRecord(c->ev_join2, c->side2));
-            PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join2, 0));   // the team kernels' results and redo list
+            LL.ring = team_ring(c);
+            LL.begin_ptr = ranges + K_GENM; LL.count_ptr = counts + K_GENM; LL.unit_counter = counters + 14;
+            dp_team_launch(mode, c->ring_grid, c->side2, LL, P);
+            c->last_launches++;
         }
-        PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));   // the cluster kernels' results and redo list
+    }
+    PA_CUDA(c, cudaEventRecord(c->ev_join2, c->side2));
+    PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join2, 0));
+    if (use_long) {
+        PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));   // the long pairs' results and redo list
         if (mode != M_LOCAL) {
-            LL.order = (const uint32_t *)c->rerun_long.p;
-            LL.begin_ptr = counters + 5;
-            LL.count_ptr = counters + 6;
-            LL.unit_counter = counters + 12;
+            // s16 results of long pairs that failed the exactness check, recomputed in s32
+            LongPlan redo{(const uint32_t *)c->rerun_long.p, counters + 5, counters + 6, 1, long_queue(c, 1, P)};
+            plan_long(c, st, o1, o2, mode, nullptr, &redo);
+            LL.order = redo.order;
+            LL.begin_ptr = redo.begin; LL.count_ptr = redo.count; LL.unit_counter = counters + 12;
             LL.rerun = 1;
-            dp_cta_launch(false, false, mode, c->ring_grid, st, LL, P);
+            dp_long_launch(false, mode, long_grid(c, false, mode), st, LL, redo.Q, P);
+            c->last_launches++;
         }
-        c->last_launches += (mode != M_LOCAL ? 7 : 6) + (C.team_max_n > 0 ? 3 : 0);
     }
     // s16 global results that failed the exactness check, recomputed in s32
     if (mode != M_LOCAL) {
@@ -516,7 +591,7 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
         L.unit_counter = counters + 3;
         L.rerun = 1;
         L.G = c->G[K_S32];
-        launch_class(c, K_S32, mode, false, false, L, P);
+        launch_class(c, K_S32, mode, false, false, L, P, st);
     }
     PA_CUDA(c, cudaEventRecordWithFlags(c->ev_dp1, st, ev_flags));
     PA_CUDA(c, cudaGetLastError());
@@ -532,18 +607,13 @@ pa_status ensure_ring(pa_ctx *c, int64_t max_m)
     if (c->ring.p && c->ring_m >= max_m) return PA_OK;
     int per_sm = 1;
     for (int mode = 0; mode < 3; ++mode) {
-        per_sm = std::max(per_sm, dp_cta_occupancy(true, false, mode));
-        per_sm = std::max(per_sm, dp_cta_occupancy(false, false, mode));
-        per_sm = std::max(per_sm, dp_cta_occupancy(false, true, mode));
-        per_sm = std::max(per_sm, dp_team_occupancy(true, false, mode));
-        per_sm = std::max(per_sm, dp_team_occupancy(false, false, mode));
-        per_sm = std::max(per_sm, dp_team_occupancy(false, true, mode));
+        per_sm = std::max(per_sm, dp_cta_occupancy(mode));
+        per_sm = std::max(per_sm, dp_team_occupancy(mode));
     }
     per_sm = std::max(per_sm, band_cta_occupancy());
     per_sm = std::max(per_sm, band_labels_cta_occupancy());
     const int grid = per_sm * c->sm_count;
     const int32_t m = (int32_t)std::max<int64_t>(max_m, c->ring_m);
-    // two regions: CTA-mode blocks and cluster-mode blocks run at the same time
     // three regions: CTA-mode blocks, cluster-mode blocks and team blocks run at the same time
     pa_status s = ensure(c, c->ring, (size_t)3 * grid * 8 * ((size_t)m + 2) * sizeof(Cell));
     if (s) return s;
@@ -682,6 +752,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     if (!s1 || !o1 || !s2 || !o2 || !out) return fail(c, PA_ERR_INVALID_ARGUMENT, "null buffer");
     if (n_pairs >= (1ull << 31)) return fail(c, PA_ERR_TOO_LARGE, "n_pairs must be < 2^31");
     if ((s = prepare_buffers(c, n_pairs, b1))) return s;
+    if (c->use_long && (s = ensure_long(c, n_pairs, b1))) return s;
     const uint64_t np = n_pairs;
     // the band work classes: {lanes16, cta} -> s16 groups, s32 groups, s16 blocks, s32 blocks
     // the band work classes: s16x2 / s32 lanes x one group / one block / one cluster per unit
@@ -759,7 +830,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
                 F.count_ptr = (const uint32_t *)c->counts.p + gk[k];
                 F.unit_counter = counters + k;
                 F.G = c->G[gk[k]];
-                launch_class(c, gk[k], M_GLOBAL, k == 0, false, F, P);
+                launch_class(c, gk[k], M_GLOBAL, k == 0, false, F, P, st);
             }
         }
         PA_CUDA(c, cudaEventSynchronize(c->ev_join));
@@ -787,36 +858,22 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     }
     // the largest pairs go to clusters only when their units fit in two waves of clusters
     if (c->ring.p) {
-        const int slots = dp_cluster_grid(true, false, M_BAND, c->ring_grid) / kClusterBlocks;
+        const int slots = dp_cluster_grid(M_BAND, c->ring_grid) / kClusterBlocks;
         if ((counts[K_S16H] + 1) / 2 + counts[K_S32H] > 2u * (uint32_t)slots) bc[4].kind = bc[5].kind = 1;
     }
 
-    // the full DP of a list: group kernels (with the s16 -> s32 redo list), whole blocks or clusters
-    auto full_dp = [&](int k, const uint32_t *list, uint32_t *count_word, uint32_t *queue) -> pa_status {
+    // the full DP of a list of group-class pairs (with the s16 -> s32 redo list)
+    auto full_dp = [&](int k, const uint32_t *list, uint32_t *count_word, uint32_t *queue) {
         DpLaunch F = L;
         F.order = list;
         F.begin_ptr = ctr + 0;
         F.count_ptr = count_word;
         F.unit_counter = queue;
         F.rerun = 0;
-        F.team = 0;                                   // whole blocks per pair
-        F.rerun_list = (uint32_t *)(bc[k].kind ? c->rerun_long.p : c->rerun.p);
-        F.rerun_count = counters + (bc[k].kind ? 6 : 4);
-        if (bc[k].kind == 2) {
-            F.G = 32;
-            F.ring = cluster_ring(c);
-            PA_CUDA(c, dp_cluster_launch(bc[k].lanes16, false, M_GLOBAL,
-                                         dp_cluster_grid(bc[k].lanes16, false, M_GLOBAL, c->ring_grid), st, F, P));
-            c->last_launches++;
-        } else if (bc[k].kind == 1) {
-            F.G = 32;
-            dp_cta_launch(bc[k].lanes16, false, M_GLOBAL, c->ring_grid, st, F, P);
-            c->last_launches++;
-        } else {
-            F.G = c->G[bc[k].klass];
-            launch_class(c, bc[k].klass, M_GLOBAL, bc[k].lanes16, false, F, P);
-        }
-        return PA_OK;
+        F.rerun_list = (uint32_t *)c->rerun.p;
+        F.rerun_count = counters + 4;
+        F.G = c->G[bc[k].klass];
+        launch_class(c, bc[k].klass, M_GLOBAL, bc[k].lanes16, false, F, P, st);
     };
     // byte-compare classes: the full DP
     {
@@ -828,7 +885,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
         F.count_ptr = (const uint32_t *)c->counts.p + K_GEN;
         F.unit_counter = counters + 2;
         F.G = c->G[K_GEN];
-        launch_class(c, K_GEN, M_GLOBAL, false, true, F, P);
+        launch_class(c, K_GEN, M_GLOBAL, false, true, F, P, st);
         if (counts[K_GENL]) {
             F.begin_ptr = (const uint32_t *)c->ranges.p + K_GENL;
             F.count_ptr = (const uint32_t *)c->counts.p + K_GENL;
@@ -836,7 +893,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
             F.G = 32;
             F.rerun_list = (uint32_t *)c->rerun_long.p;
             F.rerun_count = counters + 6;
-            dp_cta_launch(false, true, M_GLOBAL, c->ring_grid, st, F, P);
+            dp_cta_launch(M_GLOBAL, c->ring_grid, st, F, P);
             c->last_launches++;
         }
         if (counts[K_GENH]) {
@@ -847,8 +904,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
             F.ring = cluster_ring(c);
             F.rerun_list = (uint32_t *)c->rerun_long.p;
             F.rerun_count = counters + 6;
-            PA_CUDA(c, dp_cluster_launch(false, true, M_GLOBAL, dp_cluster_grid(false, true, M_GLOBAL, c->ring_grid),
-                                         st, F, P));
+            PA_CUDA(c, dp_cluster_launch(M_GLOBAL, dp_cluster_grid(M_GLOBAL, c->ring_grid), st, F, P));
             c->last_launches++;
         }
     }
@@ -947,8 +1003,8 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
         LB.rerun = S.rerun ? 1 : 0;
         if (B.kind == 2) {
             LB.ring = cluster_ring(c);
-            PA_CUDA(c, dp_cluster_launch(B.lanes16, false, M_BAND, dp_cluster_grid(B.lanes16, false, M_BAND, c->ring_grid),
-                                         S.stream, LB, P));
+            PA_CUDA(c, dp_cluster_launch(M_BAND, dp_cluster_grid(M_BAND, c->ring_grid, B.lanes16), S.stream, LB, P,
+                                         B.lanes16));
         } else {
             LB.ring = S.ring;
             band_dp_launch(B.lanes16, B.kind == 1,
@@ -1055,7 +1111,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
             ncur[k] = nn[k];
         }
     }
-    L.team = 0;                                       // the full DP below: whole blocks per pair
+    L.team = 0;
     // still open after the last round: full DP
     uint32_t hc[NB];
     for (int k = 0; k < NB; ++k) {
@@ -1072,79 +1128,38 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
         PA_CUDA(c, cudaMemcpyAsync(ctr + 6, h_hc, sizeof(hc), cudaMemcpyHostToDevice, st));
     }
     for (int k = 0; k < 2; ++k)                      // group classes
-        if (nfull[k] && (s = full_dp(k, full[k], ctr + 6 + k, ctr + 16 + k))) return s;
-    // Long classes: the full DP routed as the plain path routes it -- teams of 4 warps for pairs
-    // of at most team_max_n rows, clusters for the largest pairs when their units fit in two
-    // waves of clusters (else whole blocks take them first), whole blocks for the rest -- the
-    // three kinds at the same time, on the call's two side streams.
-    for (int l = 0; l < 2; ++l) {
-        const int kl = 2 + l, kh = 4 + l;
-        const uint32_t total = nfull[kl] + nfull[kh];
-        if (!total) continue;
-        const bool lanes16 = l == 0;
-        uint32_t *all = cur[kl], *lc = cur[kh], *lb = nxt[kl], *lt = nxt[kh];   // free after the rounds
-        // the largest pairs first: the cluster-class list, then the block-class list
-        if (nfull[kh]) PA_CUDA(c, cudaMemcpyAsync(all, full[kh], nfull[kh] * 4ull, cudaMemcpyDeviceToDevice, st));
-        if (nfull[kl])
-            PA_CUDA(c, cudaMemcpyAsync(all + nfull[kh], full[kl], nfull[kl] * 4ull, cudaMemcpyDeviceToDevice, st));
-        uint32_t *cnt = ctr + 40 + 3 * l, *queue = ctr + 48 + 3 * l;
-        size_code_launch(st, o1, o2, all, total, c->team_max_n, c->huge_cells, c->huge_min_n, code);
-        compact_launch(st, all, code, total, 2, bsum, lc, cnt + 0);
-        compact_launch(st, all, code, total, 1, bsum, lb, cnt + 1);
-        compact_launch(st, all, code, total, 0, bsum, lt, cnt + 2);
-        c->last_launches += 10;
-        uint32_t *h = (uint32_t *)(c->pinned + 224);
-        PA_CUDA(c, cudaMemcpyAsync(h, cnt, 12, cudaMemcpyDeviceToHost, st));
-        PA_CUDA(c, cudaStreamSynchronize(st));
+        if (nfull[k]) full_dp(k, full[k], ctr + 6 + k, ctr + 16 + k);
+    // Long classes: the full DP of what is left, as the plain path runs it (the pass queue of
+    // dp_long), s16x2 pairs first; the queue takes its list from the end, the largest pairs
+    auto long_full = [&](bool lanes16, const uint32_t *list, const uint32_t *begin, const uint32_t *count,
+                         uint32_t *queue, bool rerun) {
+        LongPlan plan{list, begin, count, lanes16 ? 2 : 1, long_queue(c, lanes16 ? 0 : 1, P)};
+        plan_long(c, st, o1, o2, M_GLOBAL, lanes16 ? &plan : nullptr, lanes16 ? nullptr : &plan);
         DpLaunch F = L;
-        F.begin_ptr = ctr + 0;
-        F.rerun = 0;
+        F.order = list;
+        F.begin_ptr = begin;
+        F.count_ptr = count;
+        F.unit_counter = queue;
+        F.rerun = rerun ? 1 : 0;
         F.team = 0;
-        F.G = 32;
         F.rerun_list = (uint32_t *)c->rerun_long.p;
         F.rerun_count = counters + 6;
-        const int slots = dp_cluster_grid(lanes16, false, M_GLOBAL, c->ring_grid) / kClusterBlocks;
-        const uint32_t cl_units = lanes16 ? (h[0] + 1) / 2 : h[0];
-        const bool clusters = h[0] > 0 && slots > 0 && cl_units <= 2u * (uint32_t)slots;
-        PA_CUDA(c, cudaEventRecord(c->ev_fork, st));
-        if (clusters) {
-            PA_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-            DpLaunch FC = F;
-            FC.order = lc;
-            FC.count_ptr = cnt + 0;
-            FC.unit_counter = queue + 0;
-            FC.ring = cluster_ring(c);
-            PA_CUDA(c, dp_cluster_launch(lanes16, false, M_GLOBAL,
-                                         dp_cluster_grid(lanes16, false, M_GLOBAL, c->ring_grid), c->side, FC, P));
-            PA_CUDA(c, cudaEventRecord(c->ev_join, c->side));
-            c->last_launches++;
-        }
-        if (h[2]) {
-            PA_CUDA(c, cudaStreamWaitEvent(c->side2, c->ev_fork, 0));
-            DpLaunch FT = F;
-            FT.order = lt;
-            FT.count_ptr = cnt + 2;
-            FT.unit_counter = queue + 2;
-            FT.ring = team_ring(c);
-            dp_team_launch(lanes16, false, M_GLOBAL, c->ring_grid, c->side2, FT, P);
-            PA_CUDA(c, cudaEventRecord(c->ev_join2, c->side2));
-            c->last_launches++;
-        }
-        if (h[1] || (h[0] && !clusters)) {
-            DpLaunch FB = F;
-            FB.order = lb;
-            FB.count_ptr = cnt + 1;
-            FB.unit_counter = queue + 1;
-            if (h[0] && !clusters) {                  // the largest pairs ahead of the block list
-                FB.lead_order = lc;
-                FB.lead_begin_ptr = ctr + 0;
-                FB.lead_count_ptr = cnt + 0;
-            }
-            dp_cta_launch(lanes16, false, M_GLOBAL, c->ring_grid, st, FB, P);
-            c->last_launches++;
-        }
-        if (clusters) PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));
-        if (h[2]) PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join2, 0));
+        dp_long_launch(lanes16, M_GLOBAL, long_grid(c, lanes16, M_GLOBAL), st, F, plan.Q, P);
+        c->last_launches++;
+    };
+    uint32_t h_total[2];
+    for (int l = 0; l < 2; ++l) {
+        const int kl = 2 + l, kh = 4 + l;
+        h_total[l] = nfull[kl] + nfull[kh];
+        if (!h_total[l]) continue;
+        uint32_t *all = cur[kl];                      // free after the rounds
+        if (nfull[kl]) PA_CUDA(c, cudaMemcpyAsync(all, full[kl], nfull[kl] * 4ull, cudaMemcpyDeviceToDevice, st));
+        if (nfull[kh])
+            PA_CUDA(c, cudaMemcpyAsync(all + nfull[kl], full[kh], nfull[kh] * 4ull, cudaMemcpyDeviceToDevice, st));
+        uint32_t *h = (uint32_t *)(c->pinned + 224) + l;
+        *h = h_total[l];
+        PA_CUDA(c, cudaMemcpyAsync(ctr + 40 + l, h, 4, cudaMemcpyHostToDevice, st));
+        long_full(l == 0, all, ctr + 0, ctr + 40 + l, ctr + 48 + l, false);
     }
     if (nfull[0] || (short_full && counts[K_S16])) {  // s16 group results that failed their check
         DpLaunch F = L;
@@ -1154,19 +1169,10 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
         F.unit_counter = counters + 3;
         F.rerun = 1;
         F.G = c->G[K_S32];
-        launch_class(c, K_S32, M_GLOBAL, false, false, F, P);
+        launch_class(c, K_S32, M_GLOBAL, false, false, F, P, st);
     }
-    if (nfull[2] || nfull[4]) {                       // the same for s16 long and largest pairs
-        DpLaunch F = L;
-        F.order = (const uint32_t *)c->rerun_long.p;
-        F.begin_ptr = counters + 5;
-        F.count_ptr = counters + 6;
-        F.unit_counter = counters + 12;
-        F.rerun = 1;
-        F.G = 32;
-        dp_cta_launch(false, false, M_GLOBAL, c->ring_grid, st, F, P);
-        c->last_launches++;
-    }
+    if (h_total[0])                                   // the same for s16 long and largest pairs
+        long_full(false, (const uint32_t *)c->rerun_long.p, counters + 5, counters + 6, counters + 12, true);
     mark_full_launch(st, out, np);
     c->last_launches++;
     PA_CUDA(c, cudaEventRecord(c->ev1, st));
@@ -1264,6 +1270,8 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
     if (!s1 || !o1 || !s2 || !o2 || !out) return fail(c, PA_ERR_INVALID_ARGUMENT, "null buffer");
     if (n_pairs >= (1ull << 31)) return fail(c, PA_ERR_TOO_LARGE, "n_pairs must be < 2^31");
     if ((s = prepare_buffers(c, n_pairs, b1))) return s;
+    if (c->use_long && (s = ensure_long(c, n_pairs, b1))) return s;
+    C.pass_queue = c->use_long;
     c->last_launches = 0;
     const bool use_graph = c->opt.use_graphs >= 0;
     PA_CUDA(c, cudaEventRecord(c->ev0, c->stream));
@@ -1275,6 +1283,7 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
         key.n_pairs = n_pairs; key.b1 = b1; key.b2 = b2; key.cfg = *cfg;
         for (int k = 0; k < 3; ++k) { key.G[k] = c->G[k]; key.variant[k] = c->variant[k]; }
         key.wait_limit = c->wait_limit;
+        key.use_long = c->use_long;
         auto it = c->graphs.find(key);
         if (it == c->graphs.end()) {
             if (c->graphs.size() >= kMaxGraphs) {
@@ -1295,9 +1304,9 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
             ce = cudaGraphInstantiate(&ex, g, 0);
             cudaGraphDestroy(g);
             if (ce != cudaSuccess) return fail(c, PA_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(ce));
-            it = c->graphs.emplace(key, GraphEntry{ex, 0}).first;
+            it = c->graphs.emplace(key, GraphEntry{ex, 0, c->last_launches}).first;
         } else {
-            c->last_launches = 6 + 3 + (P.local ? 0 : 1) + (c->ring.p ? (P.local ? 7 : 8) + (C.team_max_n > 0 ? 3 : 0) : 0);
+            c->last_launches = it->second.launches;
         }
         it->second.last_use = ++c->graph_clock;
         PA_CUDA(c, cudaGraphLaunch(it->second.exec, c->stream));
@@ -1404,13 +1413,15 @@ pa_status pa_create(pa_ctx **out, int device_ordinal, const pa_options *options)
     pa_ctx *c = new pa_ctx();
     c->device = device_ordinal;
     if (options) c->opt = *options;
+    int high = 0;
     if (cudaSetDevice(device_ordinal) != cudaSuccess ||
         cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device_ordinal) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaEventCreate(&c->ev2) != cudaSuccess || cudaEventCreate(&c->ev3) != cudaSuccess ||
         cudaEventCreate(&c->ev_dp0) != cudaSuccess || cudaEventCreate(&c->ev_dp1) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaDeviceGetStreamPriorityRange(nullptr, &high) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, high) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -1454,7 +1465,9 @@ pa_status pa_destroy(pa_ctx *c)
                       &c->in_seq1, &c->in_off1, &c->in_seq2, &c->in_off2, &c->in_out,
                       &c->band_spec, &c->band_win, &c->band_code, &c->band_bsum, &c->band_ctr, &c->band_in,
                       &c->mlp_feat, &c->mlp_x, &c->mlp_h1, &c->mlp_h2, &c->mlp_out,
-                      &c->ring, &c->rerun_long, &c->mat_rank, &c->mat_scores,
+                      &c->ring, &c->rerun_long, &c->long_words, &c->long_cells16, &c->long_start[0], &c->long_start[1],
+                      &c->long_done[0], &c->long_done[1], &c->long_fail[0], &c->long_fail[1], &c->long_rec[0],
+                      &c->long_rec[1], &c->mat_rank, &c->mat_scores,
                       &c->io_tab, &c->io_ctr, &c->in_words1, &c->in_words2,
                       &c->tb_dir, &c->tb_dir_off, &c->tb_aln, &c->tb_ops};
     for (DevBuf *b : bufs)
@@ -1487,8 +1500,10 @@ pa_status pa_align_batch_device(pa_ctx *ctx, const pa_config *config, const uint
 {
     if (!ctx) return PA_ERR_INVALID_ARGUMENT;
     if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, PA_ERR_CUDA, "cudaSetDevice");
-    // sequence lengths are on the device: CTA mode covers sequence1 up to the default ring
-    ctx->want_ring_m = std::max<int64_t>(ctx->ring_m, kDefaultRingM);
+    // sequence lengths are on the device: a batch may hold long pairs unless its bytes are too
+    // few for one; CTA mode then covers sequence1 up to the default ring
+    ctx->use_long = (double)seq1_bytes * (double)seq2_bytes >= (double)ctx->long_cells;
+    ctx->want_ring_m = ctx->use_long ? std::max<int64_t>(ctx->ring_m, kDefaultRingM) : 0;
     cudaStream_t user = (cudaStream_t)stream;
     if (user && user != ctx->stream) {
         // order the context stream after the caller's work, and the caller's after ours
@@ -1727,6 +1742,7 @@ static pa_status align_host(pa_ctx *ctx, const pa_config *config, const uint8_t 
         if (m * n >= ctx->long_cells) long_m = std::max(long_m, m);
     }
     ctx->want_ring_m = long_m;      // exact: the ring rows hold the longest CTA-mode sequence1
+    ctx->use_long = long_m > 0;
     if (config && config->band_mode) {
         s = run_band(ctx, config, (const uint8_t *)ctx->in_seq1.p, (const uint64_t *)ctx->in_off1.p, b1,
                      (const uint8_t *)ctx->in_seq2.p, (const uint64_t *)ctx->in_off2.p, b2, n_pairs,

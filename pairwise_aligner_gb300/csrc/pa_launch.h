@@ -20,21 +20,62 @@ int dp_short_occupancy(int G, int form, int mode);
 void dp_short_launch(int G, int form, int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
 inline bool dp_short_supports(int G) { return G == 4 || G == 8 || G == 16 || G == 32; }
 
-// CTA mode (long pairs): whole blocks per pair; L.ring must hold grid * 8 rows of
-// L.ring_stride cells.
-int dp_cta_occupancy(bool lanes16, bool gen, int mode);
-void dp_cta_launch(bool lanes16, bool gen, int mode, int grid, cudaStream_t stream, const DpLaunch &L,
-                   const DpParams &P);
-// The same pairs on teams of 4 warps (two units per block, same ring rows as CTA mode).
-int dp_team_occupancy(bool lanes16, bool gen, int mode);
-void dp_team_launch(bool lanes16, bool gen, int mode, int grid, cudaStream_t stream, const DpLaunch &L,
+// Rows per thread of a unit's full passes.  24 rows spread a column's fixed cost best without
+// spilling registers (mixed stream of 32,768 pairs: 113.3 ms; 32 rows, which spill, 116.8; 16
+// rows 121.5; 8 rows 159).  A pass is one warp's serial work, so the passes of the longest units
+// must not outlast the rest of the queue: rows x columns of a pass stay within the budget that
+// k_long_plan sets from the launch's work.  The floor is 4 rows, and 8 in local mode, whose
+// columns cost more (90 contig pairs: 5.1 ms with 8 rows, 6.3 with 4; 60 global long reads the
+// other way round, 3.2 and 2.7).
+constexpr int kLongRows = 24;
+__device__ inline int32_t long_rows(uint32_t budget, int32_t floor_rows, int32_t columns)
+{
+    const int32_t r = (int32_t)min(budget / (uint32_t)(columns > 0 ? columns : 1), (uint32_t)kLongRows) & ~3;
+    return r < floor_rows ? floor_rows : r;
+}
+
+// The queue of a launch: unit u's passes are tickets start[u] .. start[u + 1] - 1.
+struct LongWords {
+    uint32_t tasks;                // tickets
+    uint32_t budget;               // rows per thread x columns a pass may cover (long_rows)
+    int32_t floor_rows;
+    uint32_t pad;
+    uint64_t epoch;                // names the launch in the cell tags
+};
+struct LongRecord {                // a unit's best candidates between its passes
+    int32_t s[2], i[2], j[2];
+    int32_t pad[2];
+};
+struct LongQueue {
+    LongWords *words;
+    uint32_t *start;
+    uint32_t *done;                // passes finished per unit
+    uint32_t *fail;                // per unit: a wait ran out
+    LongRecord *rec;
+    // gap constants of the lanes: |open + ext|, |ext|, and the same for steps to the next column
+    uint32_t goea, exta, goeh, exth;
+    ulonglong2 *cells;             // (seq1_bytes + n_pairs) boundary cells, pair k's at off1[k] + k
+};
+
+// Long pairs with unitary DNA scores (pa_long.cuh): the row passes of all units in one queue.
+int dp_long_occupancy(bool lanes16, int mode);
+void dp_long_launch(bool lanes16, int mode, int grid, cudaStream_t stream, const DpLaunch &L, const LongQueue &Q,
                     const DpParams &P);
 
+// CTA mode (long pairs of the byte-compare class): whole blocks per pair; L.ring must hold grid * 8 rows of
+// L.ring_stride cells.
+int dp_cta_occupancy(int mode);
+void dp_cta_launch(int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
+// The same pairs on teams of 4 warps (two units per block, same ring rows as CTA mode).
+int dp_team_occupancy(int mode);
+void dp_team_launch(int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
+
 // Cluster mode (the largest pairs): clusters of kClusterBlocks blocks per pair; the grid is a
-// multiple of the cluster size and L.ring holds grid * 8 rows.  mode may be M_BAND.
-int dp_cluster_grid(bool lanes16, bool gen, int mode, int max_blocks);
-cudaError_t dp_cluster_launch(bool lanes16, bool gen, int mode, int grid, cudaStream_t stream, const DpLaunch &L,
-                              const DpParams &P);
+// multiple of the cluster size and L.ring holds grid * 8 rows.  The byte-compare class, or with
+// mode M_BAND the banded DP (band16: s16x2 lanes, else s32).
+int dp_cluster_grid(int mode, int max_blocks, bool band16 = true);
+cudaError_t dp_cluster_launch(int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P,
+                              bool band16 = true);
 
 // Traceback (pa_traceback.cu): one warp per pair, direction words of pair q at dir + dir_off[q],
 // passes * (m + 31) * 32 words with passes = ceil(n / kTracebackPassRows).

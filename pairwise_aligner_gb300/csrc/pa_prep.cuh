@@ -5,7 +5,7 @@
 // keeps its own length; pairs are only grouped so that the lanes and groups of
 // one warp get matrices of nearly the same shape.
 #pragma once
-#include "pa_common.cuh"
+#include "pa_launch.h"
 
 namespace pa {
 
@@ -22,6 +22,7 @@ struct ClassCfg {
     int32_t long_max_m;      // the longest sequence1 the ring rows hold
     int32_t huge_min_n;
     int32_t team_max_n;      // CTA-mode pairs with n at most this run on teams of 4 warps (0: none)
+    int32_t pass_queue;      // long s16x2 / s32 pairs all take the long class (dp_long's pass queue)
     int32_t qtab_s16;        // write class K_S16's score tables (0: its kernel builds its own)
     const int8_t *rank_map;  // substitution-matrix scoring: symbol -> rank (null: unitary scores)
 };
@@ -152,10 +153,12 @@ __global__ void k_classify(const uint8_t *__restrict__ seq1, const uint64_t *__r
         // the clamp floor (checked after the DP), so any length may try s16 first
         else if (!C.force32 && C.s16_params && (!C.local || (int64_t)P.smax * min(m, n) <= 30000)) klass = K_S16;
         else klass = K_S32;
-        if (klass != K_NONE && m * n >= C.long_cells && m <= C.long_max_m && n <= (1 << 20))
-            klass += (m * n >= C.huge_cells && n >= C.huge_min_n) ? kHugeOffset
-                     : (n <= C.team_max_n)                        ? kMediumOffset
-                                                                  : kLongOffset;
+        if (klass != K_NONE && m * n >= C.long_cells && n <= (1 << 20) &&
+            m <= (C.pass_queue && klass != K_GEN ? (1 << 20) : C.long_max_m))
+            klass += (C.pass_queue && klass != K_GEN)               ? kLongOffset
+                     : (m * n >= C.huge_cells && n >= C.huge_min_n) ? kHugeOffset
+                     : (n <= C.team_max_n)                          ? kMediumOffset
+                                                                    : kLongOffset;
         if ((klass == K_S16 && C.qtab_s16) || klass == K_S32 || klass == K_S16L || klass == K_S32L ||
             klass == K_S16H || klass == K_S32H || klass == K_S16M || klass == K_S32M) {
             uint32_t *qt = qtab + q0 + p;
@@ -284,21 +287,90 @@ __global__ void k_scatter(const uint32_t *__restrict__ keys, uint64_t n_pairs, u
     order[pos] = (uint32_t)p;
 }
 
-// Who computes the largest pairs: clusters of blocks when their units fit in two waves of
-// the clusters that can be resident (their run time would otherwise be one block's), else
-// the CTA-mode kernel, ahead of the long pairs (more units than clusters: blocks, which
-// quantise a pair's passes more finely, keep the GPU as busy).  words[0..2] are the
-// cluster kernels' counts of K_S16H, K_S32H, K_GENH, words[3..5] the CTA kernels' lead counts.
+// The pass queues of one or two long-pair launches (dp_long) that run side by side: start[u] for
+// the units of a list, largest first (the list is ascending), the budget of a pass, and the
+// launch's epoch.  Block b plans list b.
+struct LongPlan {
+    const uint32_t *order, *begin, *count;
+    int32_t lanes;                 // pairs per unit
+    LongQueue Q;
+};
+
+// The longer pair's lengths of unit u of a list.
+__device__ __forceinline__ uint2 long_shape(const LongPlan &p, const uint64_t *off1, const uint64_t *off2,
+                                            uint32_t count, uint32_t units, uint32_t u)
+{
+    const uint32_t lanes = (uint32_t)p.lanes, first = (units - 1 - u) * lanes;
+    uint2 s = make_uint2(0u, 0u);
+    for (uint32_t l = 0; l < lanes && first + l < count; ++l) {
+        const uint32_t id = p.order[*p.begin + first + l];
+        s.x = max(s.x, (uint32_t)(off1[id + 1] - off1[id]));
+        s.y = max(s.y, (uint32_t)(off2[id + 1] - off2[id]));
+    }
+    return s;
+}
+
+__global__ void __launch_bounds__(1024) k_long_plan(LongPlan a, LongPlan b, const uint64_t *__restrict__ off1,
+                                                    const uint64_t *__restrict__ off2, uint32_t warps,
+                                                    int32_t floor_rows, unsigned long long *epoch)
+{
+    __shared__ uint32_t sh[32];
+    __shared__ unsigned long long work;
+    if (threadIdx.x == 0) work = 0;
+    __syncthreads();
+    unsigned long long mine = 0;
+    for (uint32_t k = 0; k < gridDim.x; ++k) {
+        const LongPlan &p = k == 0 ? a : b;
+        const uint32_t count = *p.count, units = (count + p.lanes - 1) / p.lanes;
+        for (uint32_t u = threadIdx.x; u < units; u += 1024) {
+            const uint2 s = long_shape(p, off1, off2, count, units, u);
+            mine += (unsigned long long)s.x * s.y;
+        }
+    }
+    if (mine) atomicAdd(&work, mine);
+    __syncthreads();
+    // A pass may cover one warp's share of the work, in thread rows x columns.  Half of that ran
+    // the larger batches 7 % slower (smaller passes), one and a half times 18 % slower at 2,400
+    // long reads (the longest pair's passes outlast the others).
+    const uint32_t budget = (uint32_t)min(work / (32ull * warps), 0xffffffffull);
+    const LongPlan &p = blockIdx.x == 0 ? a : b;
+    const uint32_t count = *p.count, units = (count + p.lanes - 1) / p.lanes;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < units; base += 1024) {
+        const uint32_t u = base + threadIdx.x;
+        uint32_t total, v = 0;
+        if (u < units) {
+            const uint2 s = long_shape(p, off1, off2, count, units, u);
+            const uint32_t rows = 32u * (uint32_t)long_rows(budget, floor_rows, (int32_t)s.x);
+            v = (s.y + rows - 1) / rows;
+        }
+        const uint32_t ex = block_exclusive_scan(v, sh, total);
+        if (u < units) {
+            p.Q.start[u] = carry + ex;
+            p.Q.done[u] = 0u;
+            p.Q.fail[u] = 0u;
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) {
+        p.Q.start[units] = carry;
+        p.Q.words->tasks = carry;
+        p.Q.words->budget = budget;
+        p.Q.words->floor_rows = floor_rows;
+        p.Q.words->epoch = (uint64_t)atomicAdd(epoch, 1ull) + 1ull;
+    }
+}
+
+// Who computes the largest byte-compare pairs: clusters of blocks when their units fit in two
+// waves of the clusters that can be resident (their run time would otherwise be one block's),
+// else the CTA-mode kernel, ahead of its long pairs.  words[0] is the cluster kernel's count,
+// words[1] the CTA kernel's lead count.
 __global__ void k_route_huge(const uint32_t *__restrict__ counts, uint32_t cluster_slots, uint32_t *__restrict__ words)
 {
-    const uint32_t c16 = counts[K_S16H], c32 = counts[K_S32H], cg = counts[K_GENH];
-    const bool clusters = (c16 + 1) / 2 + c32 + cg <= 2 * cluster_slots;
-    words[0] = clusters ? c16 : 0u;
-    words[1] = clusters ? c32 : 0u;
-    words[2] = clusters ? cg : 0u;
-    words[3] = clusters ? 0u : c16;
-    words[4] = clusters ? 0u : c32;
-    words[5] = clusters ? 0u : cg;
+    const uint32_t c = counts[K_GENH];
+    const bool clusters = c <= 2 * cluster_slots;
+    words[0] = clusters ? c : 0u;
+    words[1] = clusters ? 0u : c;
 }
 
 }  // namespace pa

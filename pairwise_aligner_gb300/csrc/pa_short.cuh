@@ -33,16 +33,20 @@ struct ShortUnit {
     Slot *slot;                    // slots 1..ms of the unit (slot 0 unused)
 };
 
-template <int MODE>
-struct ShortConst {
-    static constexpr int32_t Kt = MODE == M_LOCAL ? 2048 : 32767 - 512;   // stored = true + Kt (+ shift)
-    static constexpr int32_t clampt = 2048;
-    static constexpr int32_t floor_true = MODE == M_LOCAL ? 0 : 2048 - Kt;
+// Stored values of a lane type: true value + Kt (global modes: of H - shift * column), clamped
+// at clampt; a global s16 result at or below floor_true may have met the clamp.
+template <class V, int MODE>
+struct StripConst {
+    static constexpr bool S16 = V::LANES == 2;
+    static constexpr int32_t Kt = !S16 ? 0 : MODE == M_LOCAL ? 2048 : 32767 - 512;
+    static constexpr int32_t clampt = S16 ? 2048 : MODE == M_LOCAL ? 0 : INT32_MIN;
+    static constexpr int32_t floor_true = !S16 ? INT32_MIN : MODE == M_LOCAL ? 0 : 2048 - Kt;
 };
 
-// Per-thread shared-memory state: result candidates (score, end1, end2) of both lanes and,
+// Per-thread shared-memory state: result candidates (score, end1, end2) of every lane and,
 // in local mode, the column of each lane's last improvement in the current pass.
-struct ShortShared {
+template <class V>
+struct StripShared {
     int32_t (*c)[3][kBlock];       // [lane][field][thread]
     int32_t (*bi)[kBlock];         // [lane][thread]
     __device__ __forceinline__ int32_t &s(int l) { return c[l][0][threadIdx.x]; }
@@ -54,13 +58,63 @@ struct ShortShared {
     }
 };
 
+// Results of a finished unit from its candidates (one thread): the free-end borders, the s16
+// exactness check (a result at the floor goes to the s32 redo list), the failed waits.
+template <class V, int MODE>
+__device__ __forceinline__ void strip_emit(const DpLaunch &L, const DpParams &P, const uint32_t *id, const int32_t *m,
+                                           const int32_t *n, bool has_b, int32_t *cs, int32_t *ci, int32_t *cj,
+                                           bool failed)
+{
+    using KC = StripConst<V, MODE>;
+#pragma unroll
+    for (int l = 0; l < V::LANES; ++l) {
+        if (l == 1 && !has_b) continue;
+        pa_result r;
+        if (failed) {
+            // a boundary cell was used before it was there: the score is not valid
+            r.score = INT32_MIN;
+            r.end1 = r.end2 = 0;
+            r.width = V::WIDTH;
+            r.flags = PA_RESULT_ERROR;
+            r.band_rounds = 0;
+            L.out[id[l]] = r;
+            continue;
+        }
+        if (MODE == M_GLOBAL_FREE) {
+            if (P.last_column_free) {            // H(0, n)
+                const int32_t x = border(P, P.first_row_free, n[l]);
+                if (better(x, 0, n[l], cs[l], ci[l], cj[l])) { cs[l] = x; ci[l] = 0; cj[l] = n[l]; }
+            }
+            if (P.last_row_free) {               // H(m, 0)
+                const int32_t x = border(P, P.first_column_free, m[l]);
+                if (better(x, m[l], 0, cs[l], ci[l], cj[l])) { cs[l] = x; ci[l] = m[l]; cj[l] = 0; }
+            }
+        }
+        if (V::LANES == 2 && MODE != M_LOCAL &&
+            (int64_t)cs[l] - (int64_t)P.shift * ci[l] <= (int64_t)KC::floor_true) {
+            // a clamp may have reached this result: recompute it in s32
+            const uint32_t slot = atomicAdd(L.rerun_count, 1u);
+            L.rerun_list[slot] = id[l];
+            continue;
+        }
+        r.score = cs[l];
+        r.end1 = ci[l];
+        r.end2 = cj[l];
+        r.width = V::WIDTH;
+        r.flags = V::LANES == 1 && L.rerun ? PA_RESULT_RERUN : 0;
+        r.band_rounds = 0;
+        if (MODE == M_LOCAL && cs[l] <= 0) { r.end1 = 0; r.end2 = 0; }
+        L.out[id[l]] = r;
+    }
+}
+
 // One pass p of the unit: rows p*G*R + t*RA + 1 .. + RA (1-based) on thread t.
 template <int MODE, int G, int R, int RA>
 __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P, const ShortUnit &u, int p, int t,
-                                           unsigned gmask, uint4 *snap, ShortShared sh)
+                                           unsigned gmask, uint4 *snap, StripShared<L16> sh)
 {
     using V = L16;
-    using KC = ShortConst<MODE>;
+    using KC = StripConst<L16, MODE>;
     constexpr bool SHIFTED = MODE != M_LOCAL;      // local mode has no column shift (P.shift == 0)
     const int32_t rows_full = G * R;
     const int32_t j0 = p * rows_full + t * RA;
@@ -221,14 +275,14 @@ __global__ void __launch_bounds__(kBlock, 2) dp_short(DpLaunch L, DpParams P)
 {
     static_assert(R % kChunk == 0 && R <= 32, "R must be a multiple of the chunk");
     using V = L16;
-    using KC = ShortConst<MODE>;
+    using KC = StripConst<L16, MODE>;
     constexpr int NGROUPS = kBlock / G;
     __shared__ uint4 snap_store[MODE == M_LOCAL ? 2 * (R / 4) * kBlock : 1];
     __shared__ ShortUnit s_unit[NGROUPS];
     __shared__ int32_t s_cand[2][3][kBlock];
     __shared__ int32_t s_bi[MODE == M_LOCAL ? 2 : 1][kBlock];
     uint4 *snap = snap_store + threadIdx.x;
-    ShortShared sh{s_cand, s_bi};
+    StripShared<L16> sh{s_cand, s_bi};
     const int lane = threadIdx.x & 31;
     const int t = lane & (G - 1);
     const int g = lane / G;
@@ -321,35 +375,7 @@ __global__ void __launch_bounds__(kBlock, 2) dp_short(DpLaunch L, DpParams P)
         }
         if (t == 0) {
             const ShortUnit u = su;
-#pragma unroll
-            for (int l = 0; l < 2; ++l) {
-                if (l == 1 && !u.has_b) continue;
-                if (MODE == M_GLOBAL_FREE) {
-                    if (P.last_column_free) {            // H(0, n)
-                        const int32_t x = border(P, P.first_row_free, u.n[l]);
-                        if (better(x, 0, u.n[l], cs[l], ci[l], cj[l])) { cs[l] = x; ci[l] = 0; cj[l] = u.n[l]; }
-                    }
-                    if (P.last_row_free) {               // H(m, 0)
-                        const int32_t x = border(P, P.first_column_free, u.m[l]);
-                        if (better(x, u.m[l], 0, cs[l], ci[l], cj[l])) { cs[l] = x; ci[l] = u.m[l]; cj[l] = 0; }
-                    }
-                }
-                if (MODE != M_LOCAL && (int64_t)cs[l] - (int64_t)P.shift * ci[l] <= (int64_t)KC::floor_true) {
-                    // a clamp may have reached this result: recompute it in s32
-                    const uint32_t slot = atomicAdd(L.rerun_count, 1u);
-                    L.rerun_list[slot] = u.id[l];
-                    continue;
-                }
-                pa_result r;
-                r.score = cs[l];
-                r.end1 = ci[l];
-                r.end2 = cj[l];
-                r.width = 16;
-                r.flags = 0;
-                r.band_rounds = 0;
-                if (MODE == M_LOCAL && cs[l] <= 0) { r.end1 = 0; r.end2 = 0; }
-                L.out[u.id[l]] = r;
-            }
+            strip_emit<V, MODE>(L, P, u.id, u.m, u.n, u.has_b != 0, cs, ci, cj, false);
         }
         __syncwarp(gmask);
     }
