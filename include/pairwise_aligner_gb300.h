@@ -266,9 +266,9 @@ pa_status pa_set_wait_limit(pa_ctx *ctx, uint32_t polls);
  * pair on whole blocks.  Also the row limit of team_full_frac in band mode. */
 pa_status pa_set_team_threshold(pa_ctx *ctx, uint32_t max_rows);
 
-/* Of the same pairs, and of the pairs band mode tries, those with at least `cells` cells and
- * `min_rows` rows of sequence2 are computed by clusters of 4 thread blocks (co-scheduled;
- * their 32 warps pipeline the pair's passes); defaults 2^28 and 8192. */
+/* Of the same pairs, those with at least `cells` cells and `min_rows` rows of sequence2 are
+ * computed by clusters of 4 thread blocks (co-scheduled; their 32 warps pipeline the
+ * pair's passes); defaults 2^28 and 8192. */
 pa_status pa_set_cluster_threshold(pa_ctx *ctx, uint64_t cells, uint32_t min_rows);
 
 /* Substitution-matrix scoring (configuration/score_model_matrix.hpp:203-222,

@@ -66,7 +66,7 @@ class Context:
         _lib.check(self.lib.pa_set_cta_threshold(self.ptr, int(cells)), self.ptr)
 
     def set_cluster_threshold(self, cells: int, min_rows: int = 8192):
-        """Long pairs (byte comparison, matrix, band mode) of at least `cells` cells and `min_rows` rows run on clusters."""
+        """Long pairs (byte comparison, matrix) of at least `cells` cells and `min_rows` rows run on clusters."""
         _lib.check(self.lib.pa_set_cluster_threshold(self.ptr, int(cells), int(min_rows)), self.ptr)
 
     def set_team_threshold(self, max_rows: int):

@@ -72,8 +72,7 @@ __device__ __forceinline__ int32_t half_width(const BandSpec &B, int32_t i, int3
 __global__ void k_band_windows(const uint64_t *__restrict__ off1, const uint64_t *__restrict__ off2,
                                const uint32_t *__restrict__ list, uint32_t count, const BandSpec *__restrict__ spec,
                                int32_t rows, int shift, float full_frac, float team_frac, int32_t team_max_n,
-                               int2 *__restrict__ win, uint8_t *__restrict__ code,
-                               unsigned long long *__restrict__ width_stats)
+                               int2 *__restrict__ win, uint8_t *__restrict__ code)
 {
     const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -154,10 +153,6 @@ __global__ void k_band_windows(const uint64_t *__restrict__ off1, const uint64_t
     const float frac = (n <= team_max_n && team_frac > 0.f) ? team_frac : full_frac;
     const bool full = (double)cells > (double)frac * (double)m * (double)n;
     code[k] = full ? 2 : 0;
-    if (!full && width_stats) {          // mean window width of the banded pairs (team size)
-        atomicAdd(width_stats, (unsigned long long)(cells / rows));
-        atomicAdd(width_stats + 1, (unsigned long long)P);
-    }
 }
 
 // Network outputs (16 floats per pair, 9 used) -> band: checkpoint diagonals
@@ -300,16 +295,13 @@ __global__ void k_mark_full(pa_result *__restrict__ out, uint64_t n_pairs)
 namespace {
 constexpr int kBandVar = 36;     // branch-free top input, one-op vertical-gap chain, no table prefetch
 
-template <class V, bool CTA>
+template <class V>
 int band_occ()
 {
     static int per_sm = -1;
     if (per_sm < 0) {
         int v = 0;
-        if (CTA)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, dp_kernel_team<V, 16, M_BAND, false, kBandVar, 1>, kBlock, 0);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, dp_kernel<V, 16, M_BAND, false, kBandVar, 2>, kBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, dp_kernel<V, 16, M_BAND, false, kBandVar, 2>, kBlock, 0);
         per_sm = v < 1 ? 1 : v;
     }
     return per_sm;
@@ -317,48 +309,23 @@ int band_occ()
 inline unsigned blocks(uint64_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }
 }  // namespace
 
-int band_dp_occupancy(bool lanes16, bool cta)
+int band_dp_occupancy(bool lanes16) { return lanes16 ? band_occ<L16>() : band_occ<L32>(); }
+
+// Short pairs with caller-given bands: one group per pair (long pairs: dp_long_band_launch).
+void band_dp_launch(bool lanes16, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
 {
-    if (cta) return lanes16 ? band_occ<L16, true>() : band_occ<L32, true>();
-    return lanes16 ? band_occ<L16, false>() : band_occ<L32, false>();
+    if (lanes16) dp_kernel<L16, 16, M_BAND, false, kBandVar, 2><<<grid, kBlock, 0, st>>>(L, P);
+    else dp_kernel<L32, 16, M_BAND, false, kBandVar, 2><<<grid, kBlock, 0, st>>>(L, P);
 }
 
-int band_cta_occupancy() { return std::max(band_dp_occupancy(true, true), band_dp_occupancy(false, true)); }
-
-// CTA launches use the ring rows of L (grid blocks of 8 rows each).
-void band_dp_launch(bool lanes16, bool cta, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
-{
-    if (cta) {
-        // teams of L.team warps per pair (narrow bands keep few passes in flight)
-        if (lanes16) {
-            if (L.team == 1) dp_kernel_team<L16, 16, M_BAND, false, kBandVar, 1><<<grid, kBlock, 0, st>>>(L, P);
-            else if (L.team == 2) dp_kernel_team<L16, 16, M_BAND, false, kBandVar, 2><<<grid, kBlock, 0, st>>>(L, P);
-            else if (L.team == 4) dp_kernel_team<L16, 16, M_BAND, false, kBandVar, 4><<<grid, kBlock, 0, st>>>(L, P);
-            else dp_kernel_cta<L16, 16, M_BAND, false, kBandVar><<<grid, kBlock, 0, st>>>(L, P);
-        } else {
-            if (L.team == 1) dp_kernel_team<L32, 16, M_BAND, false, kBandVar, 1><<<grid, kBlock, 0, st>>>(L, P);
-            else if (L.team == 2) dp_kernel_team<L32, 16, M_BAND, false, kBandVar, 2><<<grid, kBlock, 0, st>>>(L, P);
-            else if (L.team == 4) dp_kernel_team<L32, 16, M_BAND, false, kBandVar, 4><<<grid, kBlock, 0, st>>>(L, P);
-            else dp_kernel_cta<L32, 16, M_BAND, false, kBandVar><<<grid, kBlock, 0, st>>>(L, P);
-        }
-    } else if (lanes16) {
-        dp_kernel<L16, 16, M_BAND, false, kBandVar, 2><<<grid, kBlock, 0, st>>>(L, P);
-    } else {
-        dp_kernel<L32, 16, M_BAND, false, kBandVar, 2><<<grid, kBlock, 0, st>>>(L, P);
-    }
-}
-
-// width_stats (2 device words, may be null) accumulates the window widths and passes of
-// the pairs that stay banded.
 void band_windows_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *off2, const uint32_t *list,
                          uint32_t count, const BandSpec *spec, int32_t rows, int shift, float full_frac,
-                         float team_frac, int32_t team_max_n, int2 *win, uint8_t *code,
-                         unsigned long long *width_stats)
+                         float team_frac, int32_t team_max_n, int2 *win, uint8_t *code)
 {
     // one warp per pair
     if (count)
         k_band_windows<<<blocks((uint64_t)count * 32, 128), 128, 0, st>>>(
-            off1, off2, list, count, spec, rows, shift, full_frac, team_frac, team_max_n, win, code, width_stats);
+            off1, off2, list, count, spec, rows, shift, full_frac, team_frac, team_max_n, win, code);
 }
 
 void band_decode_launch(cudaStream_t st, const float *out, const uint64_t *off1, const uint64_t *off2,

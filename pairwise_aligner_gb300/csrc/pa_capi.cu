@@ -86,7 +86,7 @@ struct pa_ctx {
     DevBuf slots;                 // short-pair kernel: 16-byte column slots, (seq1_bytes + n_pairs)
     // long pairs (dp_long): queue words and launch counter, boundary cells, and per queue (s16x2,
     // s32) the units' first tickets, finished passes, failed waits and records
-    DevBuf long_words, long_cells16, long_start[2], long_done[2], long_fail[2], long_rec[2];
+    DevBuf long_words, long_cells16, long_tasks, long_start[2], long_done[2], long_fail[2], long_rec[2];
     bool use_long = false;        // this call's batch may hold long pairs
     DevBuf ring, rerun_long;      // CTA mode: boundary rows per block; s16 long pairs to redo in s32
     int32_t ring_m = 0;           // longest sequence1 the ring rows hold (0: no CTA mode yet)
@@ -109,7 +109,7 @@ struct pa_ctx {
     // band mode
     pa_band_options band_opt{1.25f, 16, 64, 0.85f, 2, 0.65f, {0, 0}};
     DevBuf band_spec, band_win, band_code, band_bsum, band_ctr, band_in;
-    DevBuf band_list[22];
+    DevBuf band_list[14];
     DevBuf mlp_w[6], mlp_feat, mlp_x, mlp_h1, mlp_h2, mlp_out;
     bool has_model = false;
     // substitution matrix (PA_SCORE_MATRIX): int8 rank per byte (-1: not a symbol), int32 scores
@@ -317,13 +317,11 @@ void band_labels_launch(bool reverse, int grid, cudaStream_t st, const DpLaunch 
 void band_labels_cta_launch(bool reverse, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
 int band_labels_occupancy();
 int band_labels_cta_occupancy();
-int band_dp_occupancy(bool lanes16, bool cta);
-int band_cta_occupancy();
-void band_dp_launch(bool lanes16, bool cta, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
+int band_dp_occupancy(bool lanes16);
+void band_dp_launch(bool lanes16, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
 void band_windows_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *off2, const uint32_t *list,
                          uint32_t count, const BandSpec *spec, int32_t rows, int shift, float full_frac,
-                         float team_frac, int32_t team_max_n, int2 *win, uint8_t *code,
-                         unsigned long long *width_stats);
+                         float team_frac, int32_t team_max_n, int2 *win, uint8_t *code);
 void band_decode_launch(cudaStream_t st, const float *out, const uint64_t *off1, const uint64_t *off2,
                         uint64_t n_pairs, const DpParams &P, float margin, int32_t w_min, BandSpec *spec);
 void band_straight_launch(cudaStream_t st, const uint64_t *off1, const uint64_t *off2, uint64_t n_pairs,
@@ -420,6 +418,7 @@ LongQueue long_queue(pa_ctx *c, int k, const DpParams &P)
     q.exth = lane(P.gap_ext - P.shift);
     q.words = (LongWords *)c->long_words.p + k;
     q.start = (uint32_t *)c->long_start[k].p;
+    q.tasks = (uint2 *)c->long_tasks.p;
     q.done = (uint32_t *)c->long_done[k].p;
     q.fail = (uint32_t *)c->long_fail[k].p;
     q.rec = (LongRecord *)c->long_rec[k].p;
@@ -430,13 +429,15 @@ LongQueue long_queue(pa_ctx *c, int k, const DpParams &P)
 int long_grid(pa_ctx *c, bool lanes16, int mode) { return dp_long_occupancy(lanes16, mode) * c->sm_count; }
 
 // The pass queues of one or two lists (s16x2 units, s32 units); a null list gets no block.
+// The word that counts long-pair launches.
+unsigned long long *long_epoch(pa_ctx *c) { return (unsigned long long *)((LongWords *)c->long_words.p + 2); }
+
 void plan_long(pa_ctx *c, cudaStream_t st, const uint64_t *o1, const uint64_t *o2, int mode, const LongPlan *p16, const LongPlan *p32)
 {
-    unsigned long long *epoch = (unsigned long long *)((LongWords *)c->long_words.p + 2);
     const LongPlan &a = p16 ? *p16 : *p32;
     k_long_plan<<<p16 && p32 ? 2 : 1, 1024, 0, st>>>(a, p32 ? *p32 : a, o1, o2,
                                                      (uint32_t)long_grid(c, true, mode) * (kBlock / 32),
-                                                     mode == M_LOCAL ? 8 : 4, epoch);
+                                                     mode == M_LOCAL ? 8 : 4, long_epoch(c));
     c->last_launches++;
 }
 
@@ -610,7 +611,6 @@ pa_status ensure_ring(pa_ctx *c, int64_t max_m)
         per_sm = std::max(per_sm, dp_cta_occupancy(mode));
         per_sm = std::max(per_sm, dp_team_occupancy(mode));
     }
-    per_sm = std::max(per_sm, band_cta_occupancy());
     per_sm = std::max(per_sm, band_labels_cta_occupancy());
     const int grid = per_sm * c->sm_count;
     const int32_t m = (int32_t)std::max<int64_t>(max_m, c->ring_m);
@@ -752,20 +752,20 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     if (!s1 || !o1 || !s2 || !o2 || !out) return fail(c, PA_ERR_INVALID_ARGUMENT, "null buffer");
     if (n_pairs >= (1ull << 31)) return fail(c, PA_ERR_TOO_LARGE, "n_pairs must be < 2^31");
     if ((s = prepare_buffers(c, n_pairs, b1))) return s;
-    if (c->use_long && (s = ensure_long(c, n_pairs, b1))) return s;
+    if (c->use_long && ((s = ensure_long(c, n_pairs, b1)) ||
+                        (s = ensure(c, c->long_tasks, (b2 / (32 * kR) + n_pairs + 1) * sizeof(uint2)))))
+        return s;
+    C.pass_queue = c->use_long;
     const uint64_t np = n_pairs;
-    // the band work classes: {lanes16, cta} -> s16 groups, s32 groups, s16 blocks, s32 blocks
-    // the band work classes: s16x2 / s32 lanes x one group / one block / one cluster per unit
+    // the band work classes: s16x2 / s32 lanes x one group per unit / the long pairs' pass queue
     struct BandClass {
-        bool lanes16;
-        int kind;                 // 0 groups, 1 CTA mode, 2 cluster mode
+        bool lanes16, queue;
         Klass klass;
         int rows;
     };
-    constexpr int NB = 6;
-    BandClass bc[NB] = {{true, 0, K_S16, c->G[K_S16] * kR}, {false, 0, K_S32, c->G[K_S32] * kR},
-                        {true, 1, K_S16L, 32 * kR},         {false, 1, K_S32L, 32 * kR},
-                        {true, 2, K_S16H, 32 * kR},         {false, 2, K_S32H, 32 * kR}};
+    constexpr int NB = 4;
+    BandClass bc[NB] = {{true, false, K_S16, c->G[K_S16] * kR}, {false, false, K_S32, c->G[K_S32] * kR},
+                        {true, true, K_S16L, 32 * kR},          {false, true, K_S32L, 32 * kR}};
     const int min_rows = std::min(std::min(bc[0].rows, bc[1].rows), 32 * kR);
     if ((s = ensure(c, c->band_spec, np * sizeof(BandSpec)))) return s;
     if ((s = ensure(c, c->band_win, (b2 / min_rows + np + 1) * sizeof(int2)))) return s;
@@ -794,8 +794,6 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     L.band = spec;
     L.band_code = (uint8_t *)c->band_code.p;
     L.dp_cells = (unsigned long long *)(ctr + 32);
-    L.ring = (Cell *)c->ring.p;
-    L.ring_stride = (uint64_t)c->ring_m + 2;
     L.error = counters + 8;
     L.spin_limit = c->wait_limit;
     // Predicted bands (modes 1 and 2) are tried on long pairs only, the block and cluster classes
@@ -842,7 +840,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
                         "offsets decrease or run past seq1_bytes / seq2_bytes; no pair was aligned");
         }
     }
-    const uint32_t n_long = counts[K_S16L] + counts[K_S32L] + counts[K_S16H] + counts[K_S32H];
+    const uint32_t n_long = counts[K_S16L] + counts[K_S32L];
     if (short_full && n_long == 0) {
         // nothing to band
     } else if (h_bands) {
@@ -856,12 +854,6 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     } else if ((s = band_predict(c, P, s1, o1, s2, o2, np, spec))) {
         return s;
     }
-    // the largest pairs go to clusters only when their units fit in two waves of clusters
-    if (c->ring.p) {
-        const int slots = dp_cluster_grid(M_BAND, c->ring_grid) / kClusterBlocks;
-        if ((counts[K_S16H] + 1) / 2 + counts[K_S32H] > 2u * (uint32_t)slots) bc[4].kind = bc[5].kind = 1;
-    }
-
     // the full DP of a list of group-class pairs (with the s16 -> s32 redo list)
     auto full_dp = [&](int k, const uint32_t *list, uint32_t *count_word, uint32_t *queue) {
         DpLaunch F = L;
@@ -891,6 +883,8 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
             F.count_ptr = (const uint32_t *)c->counts.p + K_GENL;
             F.unit_counter = counters + 11;
             F.G = 32;
+            F.ring = (Cell *)c->ring.p;
+            F.ring_stride = (uint64_t)c->ring_m + 2;
             F.rerun_list = (uint32_t *)c->rerun_long.p;
             F.rerun_count = counters + 6;
             dp_cta_launch(M_GLOBAL, c->ring_grid, st, F, P);
@@ -902,6 +896,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
             F.unit_counter = counters + 15;
             F.G = 32;
             F.ring = cluster_ring(c);
+            F.ring_stride = (uint64_t)c->ring_m + 2;
             F.rerun_list = (uint32_t *)c->rerun_long.p;
             F.rerun_count = counters + 6;
             PA_CUDA(c, dp_cluster_launch(M_GLOBAL, dp_cluster_grid(M_GLOBAL, c->ring_grid), st, F, P));
@@ -920,7 +915,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     uint64_t short_pairs = 0;                         // group-class pairs already on the full DP
     for (int k = 0; k < NB; ++k) {
         const uint32_t cnt = counts[bc[k].klass];
-        if (short_full && bc[k].kind == 0) {          // short pairs: no band rounds (launched above)
+        if (short_full && !bc[k].queue) {             // short pairs: no band rounds (launched above)
             ncur[k] = 0;
             short_pairs += cnt;
             continue;
@@ -934,141 +929,51 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     uint8_t *code = (uint8_t *)c->band_code.p;
     uint32_t *bsum = (uint32_t *)c->band_bsum.p;
     const float full_frac = c->band_opt.full_frac;
-    // One round of work class k over `list`: pairs to widen go to `next`, s16 results to redo in
-    // s32 to `redo_out` (or nowhere).  A step has its own list, code, counter and stream slots,
-    // so that two steps can run their banded DP at the same time: open() queues the windows and
-    // their compaction, read() collects the counts (host wait), dp() launches the banded DP on
-    // the step's stream and ring rows, close() compacts its outcome, collect() reads it.
-    struct Step {
-        int k = 0;
-        const uint32_t *list = nullptr;
-        uint32_t count = 0;
-        bool rerun = false;
-        uint32_t *next = nullptr, *n_next = nullptr, *redo_out = nullptr;
-        uint32_t n_redo = 0;
-        uint32_t *tmpl = nullptr;                    // the pairs that run the banded DP
-        uint8_t *code = nullptr;                     // per list position
-        uint32_t *cw = nullptr;                      // 5 device words: full, banded, queue, widen, redo
-        unsigned long long *ws = nullptr;            // 2 device words: window cells, passes
-        cudaStream_t stream = nullptr;
-        Cell *ring = nullptr;
-        size_t pin = 0;                              // its page-locked host words (32 bytes)
-        uint32_t nb = 0;
-        int team = 1;
-    };
+    // One round of work class k over `list`: the windows and their compaction, the banded DP of the
+    // pairs that stay banded, the compaction of its outcome: pairs to widen go to `next`, s16
+    // results to redo in s32 to `redo_out` (or nowhere).  The host waits for the counts twice.
     const auto *opt = &c->band_opt;
-    auto step_open = [&](Step &S, int r) -> pa_status {
-        const BandClass &B = bc[S.k];
-        PA_CUDA(c, cudaMemsetAsync(S.ws, 0, 16, st));
-        band_windows_launch(st, o1, o2, S.list, S.count, spec, B.rows, r, full_frac, opt->team_full_frac,
-                            c->team_max_n, (int2 *)c->band_win.p, S.code, S.ws);
-        compact_launch(st, S.list, S.code, S.count, 2, bsum, full[S.k] + nfull[S.k], S.cw + 0);
-        compact_launch(st, S.list, S.code, S.count, 0, bsum, S.tmpl, S.cw + 1);
-        c->last_launches += 7;
-        return PA_OK;
-    };
-    auto step_read = [&](Step &S) -> pa_status {
-        const BandClass &B = bc[S.k];
-        uint32_t *h = (uint32_t *)(c->pinned + S.pin);
-        unsigned long long *w = (unsigned long long *)(c->pinned + S.pin + 8);
-        PA_CUDA(c, cudaMemcpyAsync(h, S.cw, 8, cudaMemcpyDeviceToHost, st));
-        PA_CUDA(c, cudaMemcpyAsync(w, S.ws, 16, cudaMemcpyDeviceToHost, st));
-        PA_CUDA(c, cudaStreamSynchronize(st));
-        nfull[S.k] += h[0];
-        S.nb = h[1];
-        // CTA mode: a team of warps per pair, at most half the passes a window keeps in flight
-        // (a window of W columns keeps about W / rows passes going); more pairs with fewer
-        // warps each beat fewer pairs with waiting warps.  Measured on 262,144 config-5 pairs:
-        // for the 1,000-10,000-base class (mean window 1,600-2,500 columns) one warp per pair
-        // was 1-2 % faster than two or four and eight was 1.30x slower; for the largest pairs
-        // (mean window 8,900-14,800) eight warps were 1.16x faster than four, 1.83x than two
-        const double mean_width = w[1] ? (double)w[0] / (double)w[1] : 0.0;
-        S.team = mean_width >= 16.0 * B.rows ? 8 : mean_width >= 8.0 * B.rows ? 4 : mean_width >= 4.0 * B.rows ? 2 : 1;
-        return PA_OK;
-    };
-    auto step_dp = [&](Step &S, int r) -> pa_status {
-        if (S.nb == 0) return PA_OK;
-        const BandClass &B = bc[S.k];
-        DpLaunch LB = L;
-        PA_CUDA(c, cudaMemsetAsync(S.cw + 2, 0, 4, S.stream));
-        LB.team = S.team;
-        LB.order = S.tmpl;
-        LB.begin_ptr = ctr + 0;
-        LB.count_ptr = S.cw + 1;
-        LB.unit_counter = S.cw + 2;
-        LB.band_code = S.code;
-        LB.G = B.kind ? 32 : c->G[B.klass];
-        LB.band_rows = B.rows;
-        LB.band_round = r;
-        LB.rerun = S.rerun ? 1 : 0;
-        if (B.kind == 2) {
-            LB.ring = cluster_ring(c);
-            PA_CUDA(c, dp_cluster_launch(M_BAND, dp_cluster_grid(M_BAND, c->ring_grid, B.lanes16), S.stream, LB, P,
-                                         B.lanes16));
-        } else {
-            LB.ring = S.ring;
-            band_dp_launch(B.lanes16, B.kind == 1,
-                           B.kind ? c->ring_grid : band_dp_occupancy(B.lanes16, false) * c->sm_count, S.stream, LB, P);
-        }
-        c->last_launches++;
-        return PA_OK;
-    };
-    auto step_close = [&](Step &S) -> pa_status {
-        if (S.nb == 0) return PA_OK;
-        compact_launch(st, S.tmpl, S.code, S.nb, 1, bsum, S.next + *S.n_next, S.cw + 3);
-        compact_launch(st, S.tmpl, S.code, S.nb, 3, bsum, S.redo_out ? S.redo_out : S.tmpl, S.cw + 4);
-        c->last_launches += 6;
-        return PA_OK;
-    };
-    auto step_collect = [&](Step &S) -> pa_status {
-        if (S.nb == 0) return PA_OK;
-        uint32_t *h = (uint32_t *)(c->pinned + S.pin + 24);
-        PA_CUDA(c, cudaMemcpyAsync(h, S.cw + 3, 8, cudaMemcpyDeviceToHost, st));
-        PA_CUDA(c, cudaStreamSynchronize(st));
-        PA_CUDA(c, cudaGetLastError());
-        *S.n_next += h[0];
-        S.n_redo = S.redo_out ? h[1] : 0;
-        banded += S.nb - h[0] - h[1];
-        return PA_OK;
-    };
-    uint32_t *tmp2 = (uint32_t *)c->band_list[3 * NB + 2].p, *redo2 = (uint32_t *)c->band_list[3 * NB + 3].p;
-    // slot 0: the call's stream and the block-mode ring rows; slot 1: the first side stream and
-    // the team region of the ring (cluster steps use the cluster region in either slot)
-    auto make_step = [&](int slot, int k, const uint32_t *list, uint32_t count, bool rerun, uint32_t *next,
-                         uint32_t *n_next, uint32_t *redo_out, uint32_t code_off) {
-        Step S;
-        S.k = k; S.list = list; S.count = count; S.rerun = rerun;
-        S.next = next; S.n_next = n_next; S.redo_out = redo_out;
-        S.tmpl = slot ? tmp2 : tmp;
-        S.code = code + code_off;
-        S.cw = slot ? ctr + 22 : ctr + 1;
-        S.ws = (unsigned long long *)(slot ? ctr + 28 : ctr + 36);
-        S.stream = slot ? c->side : st;
-        S.pin = slot ? 192 : 160;
-        S.ring = slot ? team_ring(c) : (Cell *)c->ring.p;
-        return S;
-    };
-    // one step alone, on slot 0
+    uint32_t *cw = ctr + 1;                           // 5 words: full, banded, queue, widen, redo
+    uint32_t *h_cw = (uint32_t *)(c->pinned + 160);
     auto band_step = [&](int k, const uint32_t *list, uint32_t count, int r, bool rerun, uint32_t *next,
                          uint32_t &n_next, uint32_t *redo_out, uint32_t &n_redo) -> pa_status {
-        Step S = make_step(0, k, list, count, rerun, next, &n_next, redo_out, 0);
-        pa_status e;
-        if ((e = step_open(S, r)) || (e = step_read(S)) || (e = step_dp(S, r)) || (e = step_close(S)) ||
-            (e = step_collect(S)))
-            return e;
-        n_redo = S.n_redo;
-        return PA_OK;
-    };
-    // two steps whose banded DPs run at the same time (the long and the largest pairs)
-    auto band_pair = [&](Step &A, Step &B, int r) -> pa_status {
-        pa_status e;
-        if ((e = step_open(A, r)) || (e = step_open(B, r)) || (e = step_read(A)) || (e = step_read(B))) return e;
-        PA_CUDA(c, cudaEventRecord(c->ev_fork, st));
-        PA_CUDA(c, cudaStreamWaitEvent(B.stream, c->ev_fork, 0));
-        if ((e = step_dp(A, r)) || (e = step_dp(B, r))) return e;
-        PA_CUDA(c, cudaEventRecord(c->ev_join, B.stream));
-        PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));
-        if ((e = step_close(A)) || (e = step_close(B)) || (e = step_collect(A)) || (e = step_collect(B))) return e;
+        const BandClass &B = bc[k];
+        band_windows_launch(st, o1, o2, list, count, spec, B.rows, r, full_frac, opt->team_full_frac, c->team_max_n,
+                            (int2 *)c->band_win.p, code);
+        compact_launch(st, list, code, count, 2, bsum, full[k] + nfull[k], cw + 0);
+        compact_launch(st, list, code, count, 0, bsum, tmp, cw + 1);
+        c->last_launches += 7;
+        PA_CUDA(c, cudaMemcpyAsync(h_cw, cw, 8, cudaMemcpyDeviceToHost, st));
+        PA_CUDA(c, cudaStreamSynchronize(st));
+        nfull[k] += h_cw[0];
+        const uint32_t nb = h_cw[1];
+        if (nb == 0) return PA_OK;
+        DpLaunch LB = L;
+        PA_CUDA(c, cudaMemsetAsync(cw + 2, 0, 4, st));
+        LB.order = tmp;
+        LB.begin_ptr = ctr + 0;
+        LB.count_ptr = cw + 1;
+        LB.unit_counter = cw + 2;
+        LB.G = B.queue ? 32 : c->G[B.klass];
+        LB.band_rows = B.rows;
+        LB.band_round = r;
+        LB.rerun = rerun ? 1 : 0;
+        if (B.queue) {
+            dp_long_band_launch(B.lanes16, dp_long_band_occupancy(B.lanes16) * c->sm_count, st, LB,
+                                long_queue(c, B.lanes16 ? 0 : 1, P), P, long_epoch(c));
+            c->last_launches++;
+        } else {
+            band_dp_launch(B.lanes16, band_dp_occupancy(B.lanes16) * c->sm_count, st, LB, P);
+        }
+        compact_launch(st, tmp, code, nb, 1, bsum, next + n_next, cw + 3);
+        compact_launch(st, tmp, code, nb, 3, bsum, redo_out ? redo_out : tmp, cw + 4);
+        c->last_launches += 7;
+        PA_CUDA(c, cudaMemcpyAsync(h_cw, cw + 3, 8, cudaMemcpyDeviceToHost, st));
+        PA_CUDA(c, cudaStreamSynchronize(st));
+        PA_CUDA(c, cudaGetLastError());
+        n_next += h_cw[0];
+        n_redo = redo_out ? h_cw[1] : 0;
+        banded += nb - h_cw[0] - h_cw[1];
         return PA_OK;
     };
     auto open_pairs = [&]() {
@@ -1079,28 +984,11 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     for (int r = 0; r < opt->max_rounds && open_pairs(); ++r) {
         ++rounds;
         uint32_t nn[NB] = {};
-        uint32_t nredo[NB] = {}, none = 0;
-        uint32_t *redo_of[NB] = {redo, nullptr, redo, nullptr, redo2, nullptr};
-        // the s16 group class (caller-given bands only), then its s32 redo and the s32 groups
-        if (ncur[0] && (s = band_step(0, cur[0], ncur[0], r, false, nxt[0], nn[0], redo, nredo[0]))) return s;
-        if (nredo[0] && (s = band_step(1, redo, nredo[0], r, true, nxt[1], nn[1], nullptr, none))) return s;
-        if (ncur[1] && (s = band_step(1, cur[1], ncur[1], r, false, nxt[1], nn[1], nullptr, none))) return s;
-        // the s16 long and largest classes: both banded DPs at once when both have pairs
-        if (ncur[2] && ncur[4]) {
-            Step A = make_step(0, 2, cur[2], ncur[2], false, nxt[2], &nn[2], redo_of[2], 0);
-            Step B = make_step(1, 4, cur[4], ncur[4], false, nxt[4], &nn[4], redo_of[4], ncur[2]);
-            if ((s = band_pair(A, B, r))) return s;
-            nredo[2] = A.n_redo;
-            nredo[4] = B.n_redo;
-        } else {
-            for (int k16 : {2, 4})
-                if (ncur[k16] &&
-                    (s = band_step(k16, cur[k16], ncur[k16], r, false, nxt[k16], nn[k16], redo_of[k16], nredo[k16])))
-                    return s;
-        }
-        for (int k16 : {2, 4}) {                      // their s32 redo, then the s32 classes
-            if (nredo[k16] && (s = band_step(k16 + 1, redo_of[k16], nredo[k16], r, true, nxt[k16 + 1], nn[k16 + 1],
-                                             nullptr, none)))
+        for (int k16 = 0; k16 < NB; k16 += 2) {       // an s16 class, its s32 redo, the s32 class
+            uint32_t nredo = 0, none = 0;
+            if (ncur[k16] && (s = band_step(k16, cur[k16], ncur[k16], r, false, nxt[k16], nn[k16], redo, nredo)))
+                return s;
+            if (nredo && (s = band_step(k16 + 1, redo, nredo, r, true, nxt[k16 + 1], nn[k16 + 1], nullptr, none)))
                 return s;
             if (ncur[k16 + 1] && (s = band_step(k16 + 1, cur[k16 + 1], ncur[k16 + 1], r, false, nxt[k16 + 1],
                                                 nn[k16 + 1], nullptr, none)))
@@ -1111,7 +999,6 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
             ncur[k] = nn[k];
         }
     }
-    L.team = 0;
     // still open after the last round: full DP
     uint32_t hc[NB];
     for (int k = 0; k < NB; ++k) {
@@ -1141,26 +1028,13 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
         F.count_ptr = count;
         F.unit_counter = queue;
         F.rerun = rerun ? 1 : 0;
-        F.team = 0;
         F.rerun_list = (uint32_t *)c->rerun_long.p;
         F.rerun_count = counters + 6;
         dp_long_launch(lanes16, M_GLOBAL, long_grid(c, lanes16, M_GLOBAL), st, F, plan.Q, P);
         c->last_launches++;
     };
-    uint32_t h_total[2];
-    for (int l = 0; l < 2; ++l) {
-        const int kl = 2 + l, kh = 4 + l;
-        h_total[l] = nfull[kl] + nfull[kh];
-        if (!h_total[l]) continue;
-        uint32_t *all = cur[kl];                      // free after the rounds
-        if (nfull[kl]) PA_CUDA(c, cudaMemcpyAsync(all, full[kl], nfull[kl] * 4ull, cudaMemcpyDeviceToDevice, st));
-        if (nfull[kh])
-            PA_CUDA(c, cudaMemcpyAsync(all + nfull[kl], full[kh], nfull[kh] * 4ull, cudaMemcpyDeviceToDevice, st));
-        uint32_t *h = (uint32_t *)(c->pinned + 224) + l;
-        *h = h_total[l];
-        PA_CUDA(c, cudaMemcpyAsync(ctr + 40 + l, h, 4, cudaMemcpyHostToDevice, st));
-        long_full(l == 0, all, ctr + 0, ctr + 40 + l, ctr + 48 + l, false);
-    }
+    for (int l = 0; l < 2; ++l)
+        if (nfull[2 + l]) long_full(l == 0, full[2 + l], ctr + 0, ctr + 8 + l, ctr + 18 + l, false);
     if (nfull[0] || (short_full && counts[K_S16])) {  // s16 group results that failed their check
         DpLaunch F = L;
         F.order = (const uint32_t *)c->rerun.p;
@@ -1171,7 +1045,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
         F.G = c->G[K_S32];
         launch_class(c, K_S32, M_GLOBAL, false, false, F, P, st);
     }
-    if (h_total[0])                                   // the same for s16 long and largest pairs
+    if (nfull[2])                                     // the same for s16 long pairs
         long_full(false, (const uint32_t *)c->rerun_long.p, counters + 5, counters + 6, counters + 12, true);
     mark_full_launch(st, out, np);
     c->last_launches++;
@@ -1465,7 +1339,7 @@ pa_status pa_destroy(pa_ctx *c)
                       &c->in_seq1, &c->in_off1, &c->in_seq2, &c->in_off2, &c->in_out,
                       &c->band_spec, &c->band_win, &c->band_code, &c->band_bsum, &c->band_ctr, &c->band_in,
                       &c->mlp_feat, &c->mlp_x, &c->mlp_h1, &c->mlp_h2, &c->mlp_out,
-                      &c->ring, &c->rerun_long, &c->long_words, &c->long_cells16, &c->long_start[0], &c->long_start[1],
+                      &c->ring, &c->rerun_long, &c->long_words, &c->long_cells16, &c->long_tasks, &c->long_start[0], &c->long_start[1],
                       &c->long_done[0], &c->long_done[1], &c->long_fail[0], &c->long_fail[1], &c->long_rec[0],
                       &c->long_rec[1], &c->mat_rank, &c->mat_scores,
                       &c->io_tab, &c->io_ctr, &c->in_words1, &c->in_words2,

@@ -975,14 +975,12 @@ __global__ void __launch_bounds__(kBlock, 2) dp_kernel_cta(DpLaunch L, DpParams 
     }
 }
 
-// Teams mode (band mode on long pairs): the warps of a block form teams of T warps
-// (1, 2, 4 or 8); each team takes one unit (one pair, two in s16x2 lanes) at a time and its warps
+// Teams mode (byte-compare long pairs with few passes): the warps of a block form teams of T
+// warps; each team takes one unit (one pair, two in s16x2 lanes) at a time and its warps
 // take the unit's passes round robin: pass p runs on team warp p % T, reads the boundary
 // row of pass p - 1 from that warp's ring row and writes its own, column by column, behind
 // published progress.  A team's ring row k is reused by pass p + T only after pass p + 1
-// has read it: pass p + T reaches column c only after every pass between did.  Teams
-// smaller than the block suit banded pairs, whose narrow windows keep only a few passes in
-// flight at once.
+// has read it: pass p + T reaches column c only after every pass between did.
 template <class V, int R, int MODE, bool GEN, int VAR, int T>
 __global__ void __launch_bounds__(kBlock, 2) dp_kernel_team(DpLaunch L, DpParams P)
 {

@@ -1,23 +1,21 @@
 // pa_kern_cluster.cu -- instantiations and launchers of the cluster-mode DP kernel
-// (the largest pairs: a cluster of kClusterBlocks co-scheduled blocks pipelines the
-// row passes of one pair): the byte-compare class in the plain modes, and the band mode.
+// (the largest byte-compare pairs: a cluster of kClusterBlocks co-scheduled blocks pipelines
+// the row passes of one pair).
 #include "pa_dp.cuh"
 
 namespace pa {
 namespace {
 constexpr int kRowsCl = 16;
 
-template <class V, int MODE, bool GEN>
+template <int MODE>
 void *cluster_fn()
 {
-    return (void *)dp_kernel_cluster<V, kRowsCl, MODE, GEN, 36, kClusterBlocks>;
+    return (void *)dp_kernel_cluster<L32, kRowsCl, MODE, true, 36, kClusterBlocks>;
 }
 
-void *pick(int mode, bool band16)
+void *pick(int mode)
 {
-    if (mode == M_BAND) return band16 ? cluster_fn<L16, M_BAND, false>() : cluster_fn<L32, M_BAND, false>();
-    return mode == M_LOCAL ? cluster_fn<L32, M_LOCAL, true>()
-                           : mode == M_GLOBAL ? cluster_fn<L32, M_GLOBAL, true>() : cluster_fn<L32, M_GLOBAL_FREE, true>();
+    return mode == M_LOCAL ? cluster_fn<M_LOCAL>() : mode == M_GLOBAL ? cluster_fn<M_GLOBAL>() : cluster_fn<M_GLOBAL_FREE>();
 }
 
 cudaLaunchConfig_t config_of(int grid, cudaStream_t st, cudaLaunchAttribute *attr)
@@ -39,12 +37,12 @@ cudaLaunchConfig_t config_of(int grid, cudaStream_t st, cudaLaunchAttribute *att
 
 // Blocks (a multiple of the cluster size) of a cluster-mode launch that are resident at once,
 // at most `max_blocks`.
-int dp_cluster_grid(int mode, int max_blocks, bool band16)
+int dp_cluster_grid(int mode, int max_blocks)
 {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = config_of(max_blocks, nullptr, attr);
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, pick(mode, band16), &cfg) != cudaSuccess || clusters < 1) {
+    if (cudaOccupancyMaxActiveClusters(&clusters, pick(mode), &cfg) != cudaSuccess || clusters < 1) {
         cudaGetLastError();
         clusters = 1;
     }
@@ -53,14 +51,14 @@ int dp_cluster_grid(int mode, int max_blocks, bool band16)
     return grid < cap ? grid : (cap > 0 ? cap : kClusterBlocks);
 }
 
-cudaError_t dp_cluster_launch(int mode, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P, bool band16)
+cudaError_t dp_cluster_launch(int mode, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
 {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = config_of(grid, st, attr);
     DpLaunch l = L;
     DpParams p = P;
     void *args[2] = {&l, &p};
-    return cudaLaunchKernelExC(&cfg, pick(mode, band16), args);
+    return cudaLaunchKernelExC(&cfg, pick(mode), args);
 }
 
 }  // namespace pa

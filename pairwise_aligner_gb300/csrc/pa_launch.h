@@ -44,11 +44,12 @@ struct LongWords {
 };
 struct LongRecord {                // a unit's best candidates between its passes
     int32_t s[2], i[2], j[2];
-    int32_t pad[2];
+    int32_t ub[2];                 // band mode: the largest exit bound
 };
 struct LongQueue {
     LongWords *words;
     uint32_t *start;
+    uint2 *tasks;                  // band mode: {unit, pass} per ticket
     uint32_t *done;                // passes finished per unit
     uint32_t *fail;                // per unit: a wait ran out
     LongRecord *rec;
@@ -61,6 +62,10 @@ struct LongQueue {
 int dp_long_occupancy(bool lanes16, int mode);
 void dp_long_launch(bool lanes16, int mode, int grid, cudaStream_t stream, const DpLaunch &L, const LongQueue &Q,
                     const DpParams &P);
+// The banded DP of long pairs on the same queue: plan and run the list of L.
+int dp_long_band_occupancy(bool lanes16);
+void dp_long_band_launch(bool lanes16, int grid, cudaStream_t stream, const DpLaunch &L, const LongQueue &Q,
+                         const DpParams &P, unsigned long long *epoch);
 
 // CTA mode (long pairs of the byte-compare class): whole blocks per pair; L.ring must hold grid * 8 rows of
 // L.ring_stride cells.
@@ -70,12 +75,10 @@ void dp_cta_launch(int mode, int grid, cudaStream_t stream, const DpLaunch &L, c
 int dp_team_occupancy(int mode);
 void dp_team_launch(int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
 
-// Cluster mode (the largest pairs): clusters of kClusterBlocks blocks per pair; the grid is a
-// multiple of the cluster size and L.ring holds grid * 8 rows.  The byte-compare class, or with
-// mode M_BAND the banded DP (band16: s16x2 lanes, else s32).
-int dp_cluster_grid(int mode, int max_blocks, bool band16 = true);
-cudaError_t dp_cluster_launch(int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P,
-                              bool band16 = true);
+// Cluster mode (the largest of them): clusters of kClusterBlocks blocks per pair; the grid is a
+// multiple of the cluster size and L.ring holds grid * 8 rows.
+int dp_cluster_grid(int mode, int max_blocks);
+cudaError_t dp_cluster_launch(int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
 
 // Traceback (pa_traceback.cu): one warp per pair, direction words of pair q at dir + dir_off[q],
 // passes * (m + 31) * 32 words with passes = ceil(n / kTracebackPassRows).
