@@ -21,7 +21,7 @@
 #include <vector>
 
 #include "pa_common.cuh"
-#include "pa_dp.cuh"
+#include "pa_short.cuh"
 #include "pa_prep.cuh"
 #include "pa_launch.h"
 
@@ -408,14 +408,9 @@ pa_status ensure_long(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
     return PA_OK;
 }
 
-LongQueue long_queue(pa_ctx *c, int k, const DpParams &P)
+LongQueue long_queue(pa_ctx *c, int k)
 {
-    auto lane = [&](int32_t x) { return (uint32_t)std::abs(x) * (k == 0 ? 0x10001u : 1u); };
     LongQueue q;
-    q.goea = lane(P.gap_open + P.gap_ext);
-    q.exta = lane(P.gap_ext);
-    q.goeh = lane(P.gap_open + P.gap_ext - P.shift);
-    q.exth = lane(P.gap_ext - P.shift);
     q.words = (LongWords *)c->long_words.p + k;
     q.start = (uint32_t *)c->long_start[k].p;
     q.tasks = (uint2 *)c->long_tasks.p;
@@ -492,6 +487,8 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
     L.out = out;
     L.boundary = (Cell *)c->boundary.p;
     L.slots = (Slot *)c->slots.p;
+    L.gaps16 = strip_gaps(P, true);
+    L.gaps32 = strip_gaps(P, false);
     L.spin_limit = c->wait_limit;
     L.rerun_list = (uint32_t *)c->rerun.p;
     L.rerun_count = counters + 4;
@@ -517,7 +514,7 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
     if (use_long) {
         for (int k = 0; k < 2; ++k)
             plan[k] = LongPlan{(const uint32_t *)c->order.p, ranges + (k == 0 ? K_S16L : K_S32L),
-                               counts + (k == 0 ? K_S16L : K_S32L), k == 0 ? 2 : 1, long_queue(c, k, P)};
+                               counts + (k == 0 ? K_S16L : K_S32L), k == 0 ? 2 : 1, long_queue(c, k)};
         plan_long(c, st, o1, o2, mode, &plan[0], &plan[1]);
     }
     PA_CUDA(c, cudaEventRecord(c->ev_fork, st));
@@ -575,7 +572,7 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
         PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));   // the long pairs' results and redo list
         if (mode != M_LOCAL) {
             // s16 results of long pairs that failed the exactness check, recomputed in s32
-            LongPlan redo{(const uint32_t *)c->rerun_long.p, counters + 5, counters + 6, 1, long_queue(c, 1, P)};
+            LongPlan redo{(const uint32_t *)c->rerun_long.p, counters + 5, counters + 6, 1, long_queue(c, 1)};
             plan_long(c, st, o1, o2, mode, nullptr, &redo);
             LL.order = redo.order;
             LL.begin_ptr = redo.begin; LL.count_ptr = redo.count; LL.unit_counter = counters + 12;
@@ -790,6 +787,8 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     L.out = out;
     L.boundary = (Cell *)c->boundary.p;
     L.slots = (Slot *)c->slots.p;
+    L.gaps16 = strip_gaps(P, true);
+    L.gaps32 = strip_gaps(P, false);
     L.band_win = (const int2 *)c->band_win.p;
     L.band = spec;
     L.band_code = (uint8_t *)c->band_code.p;
@@ -960,7 +959,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
         LB.rerun = rerun ? 1 : 0;
         if (B.queue) {
             dp_long_band_launch(B.lanes16, dp_long_band_occupancy(B.lanes16) * c->sm_count, st, LB,
-                                long_queue(c, B.lanes16 ? 0 : 1, P), P, long_epoch(c));
+                                long_queue(c, B.lanes16 ? 0 : 1), P, long_epoch(c));
             c->last_launches++;
         } else {
             band_dp_launch(B.lanes16, band_dp_occupancy(B.lanes16) * c->sm_count, st, LB, P);
@@ -1020,7 +1019,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     // dp_long), s16x2 pairs first; the queue takes its list from the end, the largest pairs
     auto long_full = [&](bool lanes16, const uint32_t *list, const uint32_t *begin, const uint32_t *count,
                          uint32_t *queue, bool rerun) {
-        LongPlan plan{list, begin, count, lanes16 ? 2 : 1, long_queue(c, lanes16 ? 0 : 1, P)};
+        LongPlan plan{list, begin, count, lanes16 ? 2 : 1, long_queue(c, lanes16 ? 0 : 1)};
         plan_long(c, st, o1, o2, M_GLOBAL, lanes16 ? &plan : nullptr, lanes16 ? nullptr : &plan);
         DpLaunch F = L;
         F.order = list;
@@ -1202,38 +1201,27 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
 }
 
 // ---------------------------------------------------------------------------
-// roofline microkernel: the cell-update instruction mix of dp_kernel on
-// registers only (no memory, no shuffles), timed over the whole chip.  TRACK adds
-// what local scoring needs on top of the recurrence: the column maximum of the
-// thread's rows (three-operand max tree) and the test for a strict improvement.
+// roofline microkernel: the cell-update instruction mix of the strip kernels (strip_column) on
+// registers only (no memory, no shuffles), timed over the whole chip.  TRACK adds what local
+// scoring needs on top of the recurrence: the column maximum of the thread's rows
+// (three-operand max tree) and the test for a strict improvement.
 // ---------------------------------------------------------------------------
 template <class V, bool TRACK = false>
-__global__ void __launch_bounds__(256) k_roofline(int steps, uint32_t seed, uint32_t *sink)
+__global__ void __launch_bounds__(256) k_roofline(int steps, uint32_t seed, StripGaps gaps, uint32_t *sink)
 {
     constexpr int R = 16;
     uint32_t H[R], Fr[R], Sel[R];
-    const uint32_t GOEA = V::cabs(-7), EXTA = V::cabs(-1), CLAMP = V::splat(2048);
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         H[k] = V::splat(2048 + (int)((seed + k * 7 + threadIdx.x) & 15));
         Fr[k] = V::splat(2040);
-        Sel[k] = V::selector((k + threadIdx.x) & 3, (k * 3 + threadIdx.x) & 3);
+        Sel[k] = strip_selector<V>((k + threadIdx.x) & 3, (k * 3 + threadIdx.x) & 3);
     }
     uint32_t ta = 0x01fcfcfcu ^ (seed & 0x03000000u), tb = 0xfc01fcfcu, up = V::splat(2041), diag0 = V::splat(2048);
     uint32_t best = V::splat(2048), moved = 0;
     for (int s = 0; s < steps; ++s) {
-        uint32_t diag = diag0, Ed = up;
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const uint32_t sc = prmt(ta, tb, Sel[k]);
-            const uint32_t tt = V::addmax(diag, sc, Fr[k]);
-            const uint32_t h = V::hmax(tt, Ed, CLAMP);
-            diag = H[k];
-            H[k] = h;
-            const uint32_t hoe = V::subc(h, GOEA);
-            Fr[k] = V::max2(V::subc(Fr[k], EXTA), hoe);
-            Ed = V::max2(V::subc(Ed, EXTA), hoe);
-        }
+        uint32_t Ed = up;
+        strip_column<V, M_LOCAL, R>(H, Fr, Sel, ta, tb, diag0, Ed, gaps);
         if (TRACK) {
             const uint32_t nb = V::max2(best, tree_max<V, R>(H));
             moved += (nb ^ best) != 0u;
@@ -2052,14 +2040,18 @@ pa_status pa_measure_roofline(pa_ctx *ctx, pa_roofline *out)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_roofline<L32>, 256, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_roofline<L16, true>, 256, 0);
     const int steps = 4096;
+    DpParams P{};
+    P.gap_open = -6;
+    P.gap_ext = -1;
+    const StripGaps g16 = strip_gaps(P, true), g32 = strip_gaps(P, false);
     double best[3] = {0, 0, 0};
     for (int rep = 0; rep < 4; ++rep) {
         for (int w = 0; w < 3; ++w) {
             const int grid = std::max(1, per[w]) * ctx->sm_count;
             PA_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-            if (w == 1) k_roofline<L32><<<grid, 256, 0, ctx->stream>>>(steps, rep, (uint32_t *)sink.p);
-            else if (w == 2) k_roofline<L16, true><<<grid, 256, 0, ctx->stream>>>(steps, rep, (uint32_t *)sink.p);
-            else k_roofline<L16><<<grid, 256, 0, ctx->stream>>>(steps, rep, (uint32_t *)sink.p);
+            if (w == 1) k_roofline<L32><<<grid, 256, 0, ctx->stream>>>(steps, rep, g32, (uint32_t *)sink.p);
+            else if (w == 2) k_roofline<L16, true><<<grid, 256, 0, ctx->stream>>>(steps, rep, g16, (uint32_t *)sink.p);
+            else k_roofline<L16><<<grid, 256, 0, ctx->stream>>>(steps, rep, g16, (uint32_t *)sink.p);
             PA_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
             PA_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
             float ms = 0;

@@ -50,6 +50,24 @@ struct __align__(16) Slot {
     uint32_t ta, tb, h, e;
 };
 
+// The gap constants of a strip in lane form: |open + ext| and -|ext| of a step down a column,
+// and the same of a step to the next column (H is held as H - shift * column in global modes).
+struct StripGaps {
+    uint32_t goe, ext_neg, goe_h, ext_h_neg;
+};
+
+inline StripGaps strip_gaps(const DpParams &P, bool lanes16)
+{
+    const uint32_t lane = lanes16 ? 0x10001u : 1u;
+    auto neg = [&](int32_t x) { return lanes16 ? ((uint32_t)x & 0xffffu) * 0x10001u : (uint32_t)x; };   // x <= 0
+    StripGaps g;
+    g.goe = (uint32_t)-(P.gap_open + P.gap_ext) * lane;
+    g.ext_neg = neg(P.gap_ext);
+    g.goe_h = (uint32_t)-(P.gap_open + P.gap_ext - P.shift) * lane;
+    g.ext_h_neg = neg(P.gap_ext - P.shift);
+    return g;
+}
+
 // Band of one pair (band mode): the centre line runs through (0, 0), the 8
 // checkpoints (i_c, i_c + diag[c]) with i_c = (c + 1) * m / 9, and (m, n); the
 // half-width tapers linearly from w_start at column 0 to w_min at column m.
@@ -105,7 +123,9 @@ struct DpLaunch {
     int32_t mdim;
     // short-pair kernel (pa_short.cuh): (seq1_bytes + n_pairs) column slots, pair k's at off1[k] + k
     Slot *slots;
-    // CTA / team / cluster modes: polls a progress wait makes after its first look before it
+    // short- and long-pair kernels: the gap constants of s16x2 and of s32 lanes
+    StripGaps gaps16, gaps32;
+    // long pairs: polls a wait between the passes makes after its first look before it
     // gives up (pa_set_wait_limit; default 2^24)
     uint32_t spin_limit;
 };

@@ -53,8 +53,6 @@ struct LongQueue {
     uint32_t *done;                // passes finished per unit
     uint32_t *fail;                // per unit: a wait ran out
     LongRecord *rec;
-    // gap constants of the lanes: |open + ext|, |ext|, and the same for steps to the next column
-    uint32_t goea, exta, goeh, exth;
     ulonglong2 *cells;             // (seq1_bytes + n_pairs) boundary cells, pair k's at off1[k] + k
 };
 

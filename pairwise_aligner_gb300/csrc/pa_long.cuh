@@ -101,10 +101,8 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
 {
     using KC = StripConst<V, MODE>;
     constexpr int NL = V::LANES;
-    constexpr bool SHIFTED = MODE != M_LOCAL;
     const int32_t j0 = p * rows_full + t * RA;
-    // the gap constants in lane form, operands from the kernel's parameters
-    const uint32_t GOEA = Q.goea, EXTA = Q.exta, GOEH = SHIFTED ? Q.goeh : Q.goea, EXTH = SHIFTED ? Q.exth : Q.exta;
+    const StripGaps gaps = NL == 2 ? L.gaps16 : L.gaps32;
     const uint32_t CLAMP = V::splat(KC::clampt);
     auto stored = [&](int32_t true_value) { return V::splat(max(true_value + KC::Kt, KC::clampt)); };
 
@@ -120,9 +118,9 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
         const int32_t j = j0 + k;                 // 0-based row of sequence2
         const int ca = j < u.n[0] ? (int)dna_code(L.seq2[u.toff[0] + j]) : -1;
         const int cb = NL == 2 ? (j < u.n[1] ? (int)dna_code(L.seq2[u.toff[1] + j]) : -1) : ca;
-        Sel[k] = V::selector(ca, cb);
+        Sel[k] = strip_selector<V>(ca, cb);
         H[k] = left_out ? NEGV : stored(border(P, P.first_row_free, (int64_t)j + 1));
-        Fr[k] = V::subc(H[k], GOEH);
+        Fr[k] = H[k] - gaps.goe_h;
     }
     const bool t0 = t == 0;
     uint32_t prevH = left_out ? NEGV : stored(border(P, P.first_row_free, j0));
@@ -156,7 +154,7 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
                 h = e = NEGV;
             } else {                              // the top border
                 h = stored(border(P, P.first_column_free, col) - P.shift * col);
-                e = V::subc(h, GOEA);
+                e = h - gaps.goe;
             }
             stage[(c0 + t) & (2 * kStage - 1)] = make_uint4(nA, nB, h, e);
         }
@@ -195,18 +193,7 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
             uint32_t Ed = t0 ? top.w : xE;
             const uint32_t ta = t0 ? top.x : xA;
             const uint32_t tb = NL == 2 ? (t0 ? top.y : xB) : ta;
-            uint32_t tt = V::addmax(prevH, prmt(ta, tb, Sel[0]), Fr[0]);
-#pragma unroll
-            for (int k = 0; k < RA; ++k) {
-                // the next row's diagonal term uses this row's H before it is replaced
-                const uint32_t tn = k + 1 < RA ? V::addmax(H[k], prmt(ta, tb, Sel[k + 1]), Fr[k + 1]) : 0u;
-                const uint32_t h = V::hmax(tt, Ed, CLAMP);
-                H[k] = h;
-                const uint32_t hoe = V::subc(h, GOEA);
-                Fr[k] = V::max2(V::subc(Fr[k], EXTH), SHIFTED ? V::subc(h, GOEH) : hoe);
-                Ed = V::max2(V::subc(Ed, EXTA), hoe);
-                tt = tn;
-            }
+            strip_column<V, MODE, RA>(H, Fr, Sel, ta, tb, prevH, Ed, gaps);
             prevH = upH;
             sH = H[RA - 1];
             sE = Ed;

@@ -58,6 +58,55 @@ struct StripShared {
     }
 };
 
+// A held row's score selector: s16x2 lanes permute the tables of both streamed bases to it
+// (V::selector); s32 lanes hold a one-hot byte, so that one dot product adds the row's score.
+// A padded row (code < 0) scores 0 or -1.
+template <class V>
+__device__ __forceinline__ uint32_t strip_selector(int ca, int cb)
+{
+    if (V::LANES == 2) return V::selector(ca, cb);
+    return ca < 0 ? 0u : 1u << (8 * ca);
+}
+
+// One column step of a strip of RA rows: H and the gap to the next column (Fr) of the rows, the
+// vertical gap Ed running down the strip; prevH is H(i - 1, row above the strip), ta / tb the
+// score tables of the column's bases.  Per row and lane register (whole-chip microbenchmark of
+// the loop alone, 24 rows): s16x2 PRMT, VIADDMNMX (diagonal + score against Fr), VIMNMX3, two
+// VIADDMNMX (both gaps) and a subtraction or two, 8.1 T cells/s with the column shift (7.4 with
+// the gaps as a subtraction and a maximum); s32 IDP4A, VIMNMX3, two VIADDMNMX, 4.8 (4.1 with
+// PRMT, VIADDMNMX and subtract-and-maximum), as IDP4A leaves the ALU pipe free.
+template <class V, int MODE, int RA>
+__device__ __forceinline__ void strip_column(uint32_t *H, uint32_t *Fr, const uint32_t *Sel, uint32_t ta, uint32_t tb,
+                                             uint32_t prevH, uint32_t &Ed, const StripGaps &g)
+{
+    constexpr bool SHIFTED = MODE != M_LOCAL;      // local mode has no column shift (P.shift == 0)
+    const uint32_t CLAMP = V::splat(StripConst<V, MODE>::clampt);
+    // the diagonal term of a row; s16x2 lanes take the maximum with Fr along
+    auto diagonal = [&](uint32_t d, uint32_t sel, uint32_t fr) -> uint32_t {
+        if (V::LANES == 2) return __viaddmax_s16x2(d, prmt(ta, tb, sel), fr);
+        return (uint32_t)__dp4a((int)ta, (int)sel, (int)d);
+    };
+    auto gap = [](uint32_t x, uint32_t ext_neg, uint32_t open) -> uint32_t {
+        if (V::LANES == 2) return __viaddmax_s16x2(x, ext_neg, open);
+        return (uint32_t)__viaddmax_s32((int)x, (int)ext_neg, (int)open);
+    };
+    uint32_t tt = diagonal(prevH, Sel[0], Fr[0]);
+#pragma unroll
+    for (int k = 0; k < RA; ++k) {
+        // the next row's diagonal term uses this row's H before it is replaced
+        const uint32_t tn = k + 1 < RA ? diagonal(H[k], Sel[k + 1], Fr[k + 1]) : 0u;
+        uint32_t h;
+        if (V::LANES == 2) h = V::hmax(tt, Ed, CLAMP);
+        else if (MODE == M_LOCAL) h = (uint32_t)__vimax3_s32_relu((int)tt, (int)Fr[k], (int)Ed);
+        else h = (uint32_t)__vimax3_s32((int)tt, (int)Fr[k], (int)Ed);
+        H[k] = h;
+        const uint32_t hoe = h - g.goe;
+        Fr[k] = SHIFTED ? gap(Fr[k], g.ext_h_neg, h - g.goe_h) : gap(Fr[k], g.ext_neg, hoe);
+        Ed = gap(Ed, g.ext_neg, hoe);
+        tt = tn;
+    }
+}
+
 // Results of a finished unit from its candidates (one thread): the free-end borders, the s16
 // exactness check (a result at the floor goes to the s32 redo list), the failed waits.
 template <class V, int MODE>
@@ -115,14 +164,9 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
 {
     using V = L16;
     using KC = StripConst<L16, MODE>;
-    constexpr bool SHIFTED = MODE != M_LOCAL;      // local mode has no column shift (P.shift == 0)
     const int32_t rows_full = G * R;
     const int32_t j0 = p * rows_full + t * RA;
-    const uint32_t GOEA = V::cabs(P.gap_open + P.gap_ext);
-    const uint32_t EXTA = V::cabs(P.gap_ext);
-    const uint32_t GOEH = SHIFTED ? V::cabs(P.gap_open + P.gap_ext - P.shift) : GOEA;
-    const uint32_t EXTH = SHIFTED ? V::cabs(P.gap_ext - P.shift) : EXTA;
-    const uint32_t CLAMP = V::splat(KC::clampt);
+    const StripGaps gaps = L.gaps16;
     auto stored = [&](int32_t true_value) { return V::splat(max(true_value + KC::Kt, KC::clampt)); };
 
     uint32_t H[RA], Fr[RA], Sel[RA];
@@ -133,7 +177,7 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
         const int cb = j < u.n[1] ? (int)dna_code(L.seq2[u.toff[1] + j]) : -1;
         Sel[k] = V::selector(ca, cb);
         H[k] = stored(border(P, P.first_row_free, (int64_t)j + 1));
-        Fr[k] = V::subc(H[k], GOEH);
+        Fr[k] = H[k] - gaps.goe_h;
     }
     uint32_t prevH = stored(border(P, P.first_row_free, j0));
     const bool writer = t == G - 1 && p + 1 < u.passes;
@@ -173,18 +217,7 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
             const uint32_t ta = t0 ? nx.x : xA;
             const uint32_t tb = t0 ? nx.y : xB;
             if (t0 && i < ms) nx = *reinterpret_cast<const uint4 *>(slot + i + 1);
-            uint32_t tt = V::addmax(prevH, prmt(ta, tb, Sel[0]), Fr[0]);
-#pragma unroll
-            for (int k = 0; k < RA; ++k) {
-                // the next row's diagonal term uses this row's H before it is replaced
-                const uint32_t tn = k + 1 < RA ? V::addmax(H[k], prmt(ta, tb, Sel[k + 1]), Fr[k + 1]) : 0u;
-                const uint32_t h = V::hmax(tt, Ed, CLAMP);
-                H[k] = h;
-                const uint32_t hoe = V::subc(h, GOEA);
-                Fr[k] = V::max2(V::subc(Fr[k], EXTH), SHIFTED ? V::subc(h, GOEH) : hoe);
-                Ed = V::max2(V::subc(Ed, EXTA), hoe);
-                tt = tn;
-            }
+            strip_column<V, MODE, RA>(H, Fr, Sel, ta, tb, prevH, Ed, gaps);
             prevH = upH;
             sH = H[RA - 1];
             sE = Ed;
