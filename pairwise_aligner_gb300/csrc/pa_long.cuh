@@ -473,6 +473,7 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
     const uint32_t count = *L.count_ptr;
     const uint32_t units = (count + NL - 1) / NL;
     const uint32_t total = Q.words->tasks;
+    if (!strip_warp_takes_part(total)) return;
     const uint32_t budget = Q.words->budget;
     const int32_t floor_rows = Q.words->floor_rows;
     const uint64_t epoch = Q.words->epoch;

@@ -301,6 +301,14 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
     }
 }
 
+// With fewer work items than warps, only the first warps of every block take any: otherwise the
+// warps of the blocks that start first would take them all and leave the other SMs empty.  1,024
+// pairs of 150 bp (512 units on 2,432 warps): 136 -> 112 us a call.
+__device__ __forceinline__ bool strip_warp_takes_part(uint32_t items)
+{
+    return (threadIdx.x >> 5) < (items + gridDim.x - 1) / gridDim.x;
+}
+
 // The short-pair kernel: a persistent grid whose warps take units of 32/G groups x two
 // pairs from the class queue, largest shapes first; R rows of sequence2 per thread.
 template <int MODE, int G, int R>
@@ -325,6 +333,7 @@ __global__ void __launch_bounds__(kBlock, 2) dp_short(DpLaunch L, DpParams P)
     const uint32_t *order = L.order + *L.begin_ptr;
     constexpr uint32_t ppw = (uint32_t)(32 / G) * 2;   // pairs per warp unit
     const uint32_t n_units = (count + ppw - 1) / ppw;
+    if (!strip_warp_takes_part(n_units)) return;
     const uint32_t match4 = (uint8_t)(P.match - P.shift) * 0x01010101u;
     const uint32_t mis4 = (uint8_t)(P.mismatch - P.shift) * 0x01010101u;
 
