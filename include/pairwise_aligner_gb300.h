@@ -326,8 +326,9 @@ pa_status pa_align_batch_banded(pa_ctx *ctx, const pa_config *config,
  * 1 short chain, 2 three-operand with at most 85 registers, 3 branch-free top input with
  * L1 prefetch, 4 as 3 with a two-op vertical-gap chain, 5 / 6 as 3 / 4 with one prefetch
  * per 8 columns, 7 / 8 as 3 / 4 without the score-table prefetch), 9 / 10 the short-pair
- * s16x2 kernel with 16 / 32 rows of sequence2 per thread (unitary DNA scores; other
- * classes take the general kernel's default); group_threads: lanes per pair group (1..32,
+ * kernel with 16 / 32 rows of sequence2 per thread (s32 lanes: 16; matrix scores beyond a
+ * signed byte take the general kernel's default).  variant_s32 at its default (0 local, 4
+ * global) selects the short-pair kernel too; group_threads: lanes per pair group (1..32,
  * power of two; 0: the built-in rule, which picks it from the batch size).  Index 0 =
  * local, 1 = global.
  * The s16x2 class also has a table of tuned entries, one per method, batch-size class

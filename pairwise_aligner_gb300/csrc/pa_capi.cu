@@ -39,7 +39,7 @@ constexpr int kDefaultG = 8;       // threads per group
 // counters of a finished call (stage_stats).  Each is read only after a wait on the stream
 // that wrote it, and written only after the previous call's work on that stream finished.
 constexpr size_t kPinnedBytes = 1024;
-constexpr int kShortVariant = 9;   // variants 9, 10: dp_short (s16x2 unitary short pairs), 16 / 32 rows per thread
+constexpr int kShortVariant = 9;   // variants 9, 10: dp_short, 16 / 32 rows per thread
 constexpr int kVariants = kShortVariant + kShortFormCount;   // 0..8: dp_kernel (pa_kern_v*.cu)
 constexpr int kDefaultShortVariant = kShortVariant;          // with the rule below: 16 or 32 rows per thread
 
@@ -226,7 +226,7 @@ pa_status check_config(pa_ctx *c, const pa_config *cfg, DpParams &P, ClassCfg &C
     C.huge_min_n = c->huge_min_n;
     C.team_max_n = c->team_max_n;
     C.long_max_m = c->use_long && c->ring.p ? c->ring_m : 0;
-    C.qtab_s16 = 1;
+    C.qtab_s16 = C.qtab_s32 = 1;
     return PA_OK;
 }
 
@@ -259,12 +259,18 @@ void pack_2bit_launch(const uint8_t *in, uint64_t n, uint32_t *words, unsigned l
 void unpack_2bit_launch(const uint32_t *words, uint64_t first_base, uint64_t n, uint8_t *out, int sm_count,
                         cudaStream_t st);
 
-int dp_short_occupancy_local(int G, int form);
-void dp_short_launch_local(int G, int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
-int dp_short_occupancy_global(int G, int form);
-void dp_short_launch_global(int G, int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
-int dp_short_occupancy_free(int G);
-void dp_short_launch_free(int G, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
+int dp_short_occupancy_local(int form);
+int dp_short_occupancy_global(int form);
+int dp_short_occupancy_free(int form);
+void dp_short_launch_local(int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
+void dp_short_launch_global(int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
+void dp_short_launch_free(int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
+int dp_short32_occupancy_local(int scoring, int dim);
+int dp_short32_occupancy_global(int scoring, int dim);
+int dp_short32_occupancy_free(int scoring, int dim);
+void dp_short32_launch_local(int, int, cudaStream_t, const DpLaunch &, const DpParams &);
+void dp_short32_launch_global(int, int, cudaStream_t, const DpLaunch &, const DpParams &);
+void dp_short32_launch_free(int, int, cudaStream_t, const DpLaunch &, const DpParams &);
 
 int dp_long_occupancy_local(bool lanes16);
 int dp_long_occupancy_global(bool lanes16);
@@ -287,17 +293,42 @@ void dp_long_launch(bool lanes16, int mode, int grid, cudaStream_t st, const DpL
     else dp_long_launch_free(lanes16, grid, st, L, Q, P);
 }
 
-int dp_short_occupancy(int G, int form, int mode)
+static int mode_slot(int mode) { return mode == M_LOCAL ? 0 : mode == M_GLOBAL ? 1 : 2; }
+
+// Resident blocks per SM, looked up once (outside any capture: warm_occupancy and, for the
+// profiles of a matrix, pa_set_substitution_matrix).
+int dp_short_occupancy(int form, int mode)
 {
-    return mode == M_LOCAL ? dp_short_occupancy_local(G, form)
-         : mode == M_GLOBAL ? dp_short_occupancy_global(G, form) : dp_short_occupancy_free(G);
+    static int cache[3][kShortFormCount];
+    int &v = cache[mode_slot(mode)][form];
+    if (!v)
+        v = mode == M_LOCAL ? dp_short_occupancy_local(form)
+          : mode == M_GLOBAL ? dp_short_occupancy_global(form) : dp_short_occupancy_free(form);
+    return v;
 }
 
-void dp_short_launch(int G, int form, int mode, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
+void dp_short_launch(int form, int mode, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
 {
-    if (mode == M_LOCAL) dp_short_launch_local(G, form, grid, st, L, P);
-    else if (mode == M_GLOBAL) dp_short_launch_global(G, form, grid, st, L, P);
-    else dp_short_launch_free(G, grid, st, L, P);
+    if (mode == M_LOCAL) dp_short_launch_local(form, grid, st, L, P);
+    else if (mode == M_GLOBAL) dp_short_launch_global(form, grid, st, L, P);
+    else dp_short_launch_free(form, grid, st, L, P);
+}
+
+int dp_short32_occupancy(int scoring, int mode, int dim)
+{
+    static int cache[3][3][9];                    // profiles: by the symbols rounded up to 4
+    int &v = cache[mode_slot(mode)][scoring][(dim + 3) / 4];
+    if (!v)
+        v = mode == M_LOCAL ? dp_short32_occupancy_local(scoring, dim)
+          : mode == M_GLOBAL ? dp_short32_occupancy_global(scoring, dim) : dp_short32_occupancy_free(scoring, dim);
+    return v;
+}
+
+void dp_short32_launch(int scoring, int mode, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
+{
+    if (mode == M_LOCAL) dp_short32_launch_local(scoring, grid, st, L, P);
+    else if (mode == M_GLOBAL) dp_short32_launch_global(scoring, grid, st, L, P);
+    else dp_short32_launch_free(scoring, grid, st, L, P);
 }
 
 int dp_occupancy(int variant, bool lanes16, bool gen, int mode)
@@ -357,9 +388,22 @@ void warm_occupancy()
             dp_occupancy(v, false, false, mode);
             dp_occupancy(v, false, true, mode);
         }
-    for (int g = 4; g <= 32; g *= 2)
-        for (int form = 0; form < kShortFormCount; ++form)
-            for (int mode = 0; mode < 3; ++mode) dp_short_occupancy(g, form, mode);
+    for (int mode = 0; mode < 3; ++mode) {
+        for (int form = 0; form < kShortFormCount; ++form) dp_short_occupancy(form, mode);
+        dp_short32_occupancy(SC_TABLE, mode, 0);
+        dp_short32_occupancy(SC_BYTES, mode, 0);
+    }
+}
+
+// Whether the short-pair kernel takes a class under these scores: the plain modes, except scores
+// of a matrix that do not fit a signed byte, and local byte comparison with a positive mismatch
+// (its padding rows would score); the default form of dp_kernel takes those.
+bool short_fits(int mode, bool gen, bool matrix, const DpParams &P)
+{
+    if (mode > M_GLOBAL_FREE) return false;
+    if (!gen) return true;
+    if (matrix) return P.match - P.shift <= 127 && P.mismatch - P.shift >= -128 && P.spad - P.shift >= -128;
+    return mode != M_LOCAL || P.mismatch <= 0;
 }
 
 void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const DpLaunch &L, const DpParams &P,
@@ -367,19 +411,19 @@ void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const D
 {
     int v = c->variant[slot];
     if (v >= kShortVariant) {
-        // the short-pair kernel covers s16x2 lanes with unitary scores in the plain modes and
-        // groups of 4..32 lanes; anything else takes the default dp_kernel form
-        if (lanes16 && !gen && mode <= M_GLOBAL_FREE && dp_short_supports(L.G) && L.slots) {
-            // the free-end-gap form keeps 16 rows per thread (32 do not fit its registers)
-            const int form = mode == M_GLOBAL_FREE ? 0 : v - kShortVariant;
-            int per_sm = dp_short_occupancy(L.G, form, mode);
+        if (short_fits(mode, gen, L.matrix != nullptr, P) && dp_short_supports(L.G) && L.slots) {
+            const int scoring = !gen ? SC_TABLE : L.matrix ? SC_PROFILE : SC_BYTES;
+            const int form = v - kShortVariant;
+            int per_sm = lanes16 ? dp_short_occupancy(form, mode)
+                                 : dp_short32_occupancy(scoring, mode, scoring == SC_PROFILE ? L.mdim : 0);
             if (c->opt.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)c->opt.blocks_per_sm);
             c->grid[slot] = per_sm * c->sm_count;
-            dp_short_launch(L.G, form, mode, c->grid[slot], st, L, P);
+            if (lanes16) dp_short_launch(form, mode, c->grid[slot], st, L, P);
+            else dp_short32_launch(scoring, mode, c->grid[slot], st, L, P);
             c->last_launches++;
             return;
         }
-        v = mode == M_LOCAL ? 7 : 4;
+        v = lanes16 ? (mode == M_LOCAL ? 7 : 4) : (mode == M_LOCAL ? 0 : 4);
     }
     int per_sm = dp_occupancy(v, lanes16, gen, mode);
     if (c->opt.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)c->opt.blocks_per_sm);
@@ -657,14 +701,20 @@ int tune_shape_class(uint64_t n_pairs, uint64_t b1, uint64_t b2)
     return PA_TUNE_SHAPES - 1;
 }
 
-// The built-in group size: the smallest group (fewest fill and drain steps per pass) that
-// still gives every resident warp about eight work units, so the persistent queue's tail
-// stays short.  A warp unit holds 32 / G groups of `lanes` pairs.
-int rule_group_threads(const pa_ctx *c, uint64_t n_pairs, int lanes)
+// The built-in group size: the smallest group (fewest fill and drain steps per pass, most rows per
+// column step) that still gives every resident warp about three work units, so that the largest
+// pairs do not outlast the rest, and that holds a pair of mean length in two passes.  A warp unit
+// holds 32 / G groups of `lanes` pairs, a pass G * rows rows.  Measured (GB300, us per call on 8 /
+// 16 / 32 lanes): 65,537 reads of 175 rows 1,353 / 1,502 / 2,005; 16,384 pairs of 64-1,000 rows
+// 1,653 / 935 / 580; 60,000 local pairs of 288 rows 1,316 / 1,244 / 1,464; 32,768 proteins of 335
+// rows (16 per thread) 2,342 / 1,548 / 1,588.  Groups of 4 lanes pay for pairs of at most 128
+// rows, one pass of them: 262,144 local pairs of 288 rows 8,195, on 8 lanes 4,696.
+int rule_group_threads(const pa_ctx *c, uint64_t n_pairs, uint64_t b2, int lanes, int rows)
 {
     const double warps = (double)c->sm_count * (2 * kBlock / 32);
-    for (int g = 4; g < 32; g *= 2)
-        if ((double)n_pairs * g / (32.0 * lanes) >= 8.0 * warps) return g;
+    const double mean = n_pairs ? (double)b2 / (double)n_pairs : 0.0;
+    for (int g = mean <= 4 * rows ? 4 : 8; g < 32; g *= 2)
+        if ((double)n_pairs * g / (32.0 * lanes) >= 3.0 * warps && mean <= 2.0 * g * rows) return g;
     return 32;
 }
 
@@ -675,18 +725,19 @@ void apply_tuning(pa_ctx *c, const pa_config *cfg, uint64_t n_pairs, uint64_t b1
     const pa_tune_entry &e = c->tuning.s16[mi][tune_size_class(n_pairs)][tune_shape_class(n_pairs, b1, b2)];
     if (!c->fixed_variant) {
         c->variant[K_S16] = e.group_threads ? e.variant : c->tuning.variant_s16[mi];
-        c->variant[K_S32] = c->variant[K_GEN] = c->tuning.variant_s32[mi];
+        // the other classes: the short-pair kernel, unless a form of dp_kernel other than the
+        // default (0 local, 4 global) was set
+        const int v32 = c->tuning.variant_s32[mi];
+        c->variant[K_S32] = c->variant[K_GEN] = v32 == (mi == 0 ? 0 : 4) ? kDefaultShortVariant : v32;
     }
     if (!c->fixed_G) {
         int g16 = e.group_threads ? e.group_threads : c->tuning.group_threads_s16[mi];
         int g32 = c->tuning.group_threads_s32[mi];
-        c->G[K_S16] = g16 ? g16 : rule_group_threads(c, n_pairs, 2);
-        c->G[K_S32] = c->G[K_GEN] = g32 ? g32 : rule_group_threads(c, n_pairs, 1);
-        // untuned short-pair kernel: 32 rows per thread where groups are small (large batches;
-        // half the column steps of 16 rows), 16 where they are large (few pairs: 32 rows would
-        // make passes of 512-1,024 rows, mostly padding for short pairs)
+        c->G[K_S16] = g16 ? g16 : rule_group_threads(c, n_pairs, b2, 2, 32);
+        c->G[K_S32] = c->G[K_GEN] = g32 ? g32 : rule_group_threads(c, n_pairs, b2, 1, kR);
+        // untuned short-pair kernel: 32 rows per thread
         if (!e.group_threads && !g16 && !c->fixed_variant && c->tuning.variant_s16[mi] >= kShortVariant)
-            c->variant[K_S16] = c->G[K_S16] <= 8 ? kShortVariant + 1 : kShortVariant;
+            c->variant[K_S16] = kShortVariant + 1;
     }
 }
 
@@ -1133,9 +1184,11 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
     ClassCfg C;
     s = check_config(c, cfg, P, C);
     if (s) return s;
-    // local pairs of the s16x2 class that the short-pair kernel takes (launch_class) never go
-    // back to dp_kernel (no s32 redo in local mode): the kernel builds its own column tables
-    if (P.local && c->variant[K_S16] >= kShortVariant && dp_short_supports(c->G[K_S16])) C.qtab_s16 = 0;
+    // the short-pair kernel (launch_class) builds its own column tables: a class needs none when
+    // neither it nor, for global s16x2 pairs, their s32 redo runs on dp_kernel
+    auto on_short = [&](Klass k) { return c->variant[k] >= kShortVariant && dp_short_supports(c->G[k]); };
+    if (on_short(K_S32)) C.qtab_s32 = 0;
+    if (on_short(K_S16) && (P.local || on_short(K_S32))) C.qtab_s16 = 0;
     if (n_pairs == 0) {
         if (stats) std::memset(stats, 0, sizeof(*stats));
         return PA_OK;
@@ -1221,7 +1274,9 @@ __global__ void __launch_bounds__(256) k_roofline(int steps, uint32_t seed, Stri
     uint32_t best = V::splat(2048), moved = 0;
     for (int s = 0; s < steps; ++s) {
         uint32_t Ed = up;
-        strip_column<V, M_LOCAL, R>(H, Fr, Sel, ta, tb, diag0, Ed, gaps);
+        strip_column<V, M_LOCAL, R>(H, Fr, diag0, Ed, gaps, [&](uint32_t d, int k) {
+            return table_diagonal<V>(d, ta, tb, Sel[k], Fr[k]);
+        });
         if (TRACK) {
             const uint32_t nb = V::max2(best, tree_max<V, R>(H));
             moved += (nb ^ best) != 0u;
@@ -1474,6 +1529,7 @@ pa_status pa_set_substitution_matrix(pa_ctx *ctx, const uint8_t *symbols, uint32
     if ((s = ensure(ctx, ctx->mat_rank, 256)) || (s = ensure(ctx, ctx->mat_scores, 32 * 32 * 4))) return s;
     PA_CUDA(ctx, cudaMemcpy(ctx->mat_rank.p, rank, 256, cudaMemcpyHostToDevice));
     PA_CUDA(ctx, cudaMemcpy(ctx->mat_scores.p, scores, (size_t)dim * dim * 4, cudaMemcpyHostToDevice));
+    for (int mode = 0; mode < 3; ++mode) dp_short32_occupancy(SC_PROFILE, mode, (int)dim);
     ctx->mat_dim = (int32_t)dim;
     ctx->mat_max = hi;
     ctx->mat_min = lo;

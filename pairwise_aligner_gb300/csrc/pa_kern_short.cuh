@@ -1,55 +1,73 @@
-// pa_kern_short.cuh -- launcher body of the short-pair kernel, included by
-// pa_kern_short_local.cu and pa_kern_short_global.cu.
+// pa_kern_short.cuh -- launcher body of the short-pair kernel, included by pa_kern_short_*.cu
+// (s16x2 lanes) and pa_kern_short32_*.cu (s32 lanes), one translation unit per mode.
 #include "pa_short.cuh"
 #include "pa_launch.h"
 
 namespace pa {
 namespace {
 
-// Forms of the kernel: the rows of sequence2 a thread holds (0: 16, 1: 32).
-template <int MODE, int G, int R>
-int occ_short()
+constexpr int kProfileThreads = 128;
+
+// Blocks per SM: the same for every group size (registers and shared memory set it).
+template <class V, int SC, int MODE, int R, int NT>
+int occ_short(int smem)
 {
-    static int per_sm = -1;
-    if (per_sm < 0) {
+    int per_sm = 32;
+    for (int k = 0; k < 4; ++k) {
         int v = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, dp_short<MODE, G, R>, kBlock, 0);
-        per_sm = v < 1 ? 1 : v;
+        const void *f = k == 0   ? (const void *)dp_short<V, SC, MODE, 32, R, NT>
+                        : k == 1 ? (const void *)dp_short<V, SC, MODE, 16, R, NT>
+                        : k == 2 ? (const void *)dp_short<V, SC, MODE, 8, R, NT>
+                                 : (const void *)dp_short<V, SC, MODE, 4, R, NT>;
+        // the limit for any matrix, so that a small one does not lower it for a larger one
+        if (smem > 0) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * NT * 16);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, f, NT, smem);
+        per_sm = v < per_sm ? v : per_sm;
     }
-    return per_sm;
+    cudaGetLastError();
+    return per_sm < 1 ? 1 : per_sm;
 }
 
-template <int MODE, int R>
-int occ_short_g(int G)
+template <class V, int SC, int MODE, int R, int NT>
+void go_short(int grid, int smem, cudaStream_t st, const DpLaunch &L, const DpParams &P)
 {
-    return G == 4 ? occ_short<MODE, 4, R>() : G == 8 ? occ_short<MODE, 8, R>()
-                  : G == 16 ? occ_short<MODE, 16, R>() : occ_short<MODE, 32, R>();
+    if (L.G == 4) dp_short<V, SC, MODE, 4, R, NT><<<grid, NT, smem, st>>>(L, P);
+    else if (L.G == 8) dp_short<V, SC, MODE, 8, R, NT><<<grid, NT, smem, st>>>(L, P);
+    else if (L.G == 16) dp_short<V, SC, MODE, 16, R, NT><<<grid, NT, smem, st>>>(L, P);
+    else dp_short<V, SC, MODE, 32, R, NT><<<grid, NT, smem, st>>>(L, P);
 }
 
-// The free-end-gap mode exists with 16 rows only (32 do not fit its registers).
+// Dynamic shared memory of the profile kernels: a uint4 per thread and symbol.
+inline int profile_bytes(int dim) { return ((dim + 3) & ~3) * kProfileThreads * 16; }
+
+// Lanes and scoring of a class; form 0 holds 16 rows per thread, form 1 (s16x2 only) 32.
 template <int MODE>
-int occ_short_gb(int G, int form)
+int occ_short16(int form)
 {
-    if constexpr (MODE != M_GLOBAL_FREE)
-        if (form == 1) return occ_short_g<MODE, 32>(G);
-    return occ_short_g<MODE, 16>(G);
-}
-
-template <int MODE, int R>
-void go_short_g(int G, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
-{
-    if (G == 4) dp_short<MODE, 4, R><<<grid, kBlock, 0, st>>>(L, P);
-    else if (G == 8) dp_short<MODE, 8, R><<<grid, kBlock, 0, st>>>(L, P);
-    else if (G == 16) dp_short<MODE, 16, R><<<grid, kBlock, 0, st>>>(L, P);
-    else dp_short<MODE, 32, R><<<grid, kBlock, 0, st>>>(L, P);
+    return form == 1 ? occ_short<L16, SC_TABLE, MODE, 32, kBlock>(0) : occ_short<L16, SC_TABLE, MODE, 16, kBlock>(0);
 }
 
 template <int MODE>
-void go_short_gb(int G, int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
+void go_short16(int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
 {
-    if constexpr (MODE != M_GLOBAL_FREE)
-        if (form == 1) return go_short_g<MODE, 32>(G, grid, st, L, P);
-    go_short_g<MODE, 16>(G, grid, st, L, P);
+    if (form == 1) go_short<L16, SC_TABLE, MODE, 32, kBlock>(grid, 0, st, L, P);
+    else go_short<L16, SC_TABLE, MODE, 16, kBlock>(grid, 0, st, L, P);
+}
+
+template <int MODE>
+int occ_short32(int scoring, int dim)
+{
+    if (scoring == SC_TABLE) return occ_short<L32, SC_TABLE, MODE, 16, kBlock>(0);
+    if (scoring == SC_BYTES) return occ_short<L32, SC_BYTES, MODE, 16, kBlock>(0);
+    return occ_short<L32, SC_PROFILE, MODE, 16, kProfileThreads>(profile_bytes(dim));
+}
+
+template <int MODE>
+void go_short32(int scoring, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P)
+{
+    if (scoring == SC_TABLE) go_short<L32, SC_TABLE, MODE, 16, kBlock>(grid, 0, st, L, P);
+    else if (scoring == SC_BYTES) go_short<L32, SC_BYTES, MODE, 16, kBlock>(grid, 0, st, L, P);
+    else go_short<L32, SC_PROFILE, MODE, 16, kProfileThreads>(grid, profile_bytes(L.mdim), st, L, P);
 }
 
 }  // namespace

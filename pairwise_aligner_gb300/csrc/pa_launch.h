@@ -12,12 +12,14 @@ int dp_occupancy(int variant, bool lanes16, bool gen, int mode);
 void dp_launch(int variant, bool lanes16, bool gen, int mode, int grid, cudaStream_t stream, const DpLaunch &L,
                const DpParams &P);
 
-// Short-pair kernel in s16x2 lanes with unitary DNA scores (pa_short.cuh): G in {4, 8, 16,
-// 32} lanes per group, form 0 (16 rows of sequence2 per thread) or 1 (32 rows); L.slots must
-// hold seq1_bytes + n_pairs column slots.
+// Short-pair kernel (pa_short.cuh) on groups of L.G = 4, 8, 16 or 32 lanes; L.slots must hold seq1_bytes + n_pairs column slots.  s16x2 lanes with unitary DNA scores: form
+// 0 (16 rows of sequence2 per thread) or 1 (32 rows).  s32 lanes: scoring is a Scoring (tables,
+// raw bytes, or the int8 profile of a substitution matrix of dim symbols), 16 rows.
 constexpr int kShortFormCount = 2;
-int dp_short_occupancy(int G, int form, int mode);
-void dp_short_launch(int G, int form, int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
+int dp_short_occupancy(int form, int mode);
+void dp_short_launch(int form, int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
+int dp_short32_occupancy(int scoring, int mode, int dim);
+void dp_short32_launch(int scoring, int mode, int grid, cudaStream_t stream, const DpLaunch &L, const DpParams &P);
 inline bool dp_short_supports(int G) { return G == 4 || G == 8 || G == 16 || G == 32; }
 
 // Rows per thread of a unit's full passes.  24 rows spread a column's fixed cost best without

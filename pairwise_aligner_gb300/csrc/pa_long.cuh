@@ -193,52 +193,19 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
             uint32_t Ed = t0 ? top.w : xE;
             const uint32_t ta = t0 ? top.x : xA;
             const uint32_t tb = NL == 2 ? (t0 ? top.y : xB) : ta;
-            strip_column<V, MODE, RA>(H, Fr, Sel, ta, tb, prevH, Ed, gaps);
+            strip_column<V, MODE, RA>(H, Fr, prevH, Ed, gaps, [&](uint32_t d, int k) {
+                return table_diagonal<V>(d, ta, tb, Sel[k], Fr[k]);
+            });
             prevH = upH;
             sH = H[RA - 1];
             sE = Ed;
             sA = ta;
             sB = tb;
             if (writer) store_cell128(u.row + i, (uint64_t)sH | ((uint64_t)sE << 32), u.tag);
-            if (MODE == M_LOCAL) {
-                const uint32_t cm = tree_max<V, RA>(H);
-                const uint32_t nb = V::max2(best, cm);
-                const uint32_t x = nb ^ best;
-                best = nb;
-                if (x != 0u) {
-#pragma unroll
-                    for (int l = 0; l < NL; ++l) {
-                        if (V::improved(x, l)) {
-                            sh.bi[l][threadIdx.x] = i;
-#pragma unroll
-                            for (int v = 0; v < RA / 4; ++v)
-                                snap[(l * (R / 4) + v) * kBlock] =
-                                    make_uint4(H[4 * v], H[4 * v + 1], H[4 * v + 2], H[4 * v + 3]);
-                        }
-                    }
-                }
-            } else if ((MODE == M_GLOBAL_FREE && P.last_column_free && any_own) || i >= mmin) {
-                if (any_own) {
-#pragma unroll
-                    for (int v = 0; v < RA / 4; ++v)
-                        snap[v * kBlock] = make_uint4(H[4 * v], H[4 * v + 1], H[4 * v + 2], H[4 * v + 3]);
-                }
-#pragma unroll
-                for (int l = 0; l < NL; ++l) {
-                    if (l == 1 && !u.has_b) continue;
-                    const int32_t base = P.shift * i - KC::Kt, ml = u.m[l], r = own_row(l);
-                    if (r >= 0 && (i == ml || (MODE == M_GLOBAL_FREE && P.last_column_free && i < ml))) {
-                        // the row's H, read back from the snapshot
-                        const uint32_t *q = reinterpret_cast<const uint32_t *>(snap + (r >> 2) * kBlock);
-                        sh.offer(l, V::get(q[r & 3], l) + base, i, u.n[l]);
-                    }
-                    if (MODE == M_GLOBAL_FREE && P.last_row_free && i == ml) {
-#pragma unroll
-                        for (int k = 0; k < RA; ++k)
-                            if (j0 + k + 1 <= u.n[l]) sh.offer(l, V::get(H[k], l) + base, i, j0 + k + 1);
-                    }
-                }
-            }
+            if (MODE == M_LOCAL)
+                strip_track<V, R, RA>(H, best, i, snap, sh);
+            else if ((MODE == M_GLOBAL_FREE && P.last_column_free && any_own) || i >= mmin)
+                strip_ends<V, MODE, RA>(P, u, H, i, j0, any_own, snap, sh, own_row);
         }
     };
     // fill: thread t starts at step t; steady: every thread active; drain
@@ -253,23 +220,7 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
         const int32_t i = s - t + 1;
         step(s, i >= 1 && i <= ms);
     }
-    if (MODE == M_LOCAL) {
-#pragma unroll
-        for (int l = 0; l < NL; ++l) {
-            const int32_t b = V::get(best, l);
-            if (b > KC::Kt) {                     // improved in this pass: snapshot and column are set
-                int32_t kk = 0;
-                for (int v = RA / 4 - 1; v >= 0; --v) {
-                    const uint4 q = snap[(l * (R / 4) + v) * kBlock];
-                    if (V::get(q.w, l) == b) kk = 4 * v + 3;
-                    if (V::get(q.z, l) == b) kk = 4 * v + 2;
-                    if (V::get(q.y, l) == b) kk = 4 * v + 1;
-                    if (V::get(q.x, l) == b) kk = 4 * v;
-                }
-                sh.offer(l, b - KC::Kt, sh.bi[l][threadIdx.x], j0 + kk + 1);
-            }
-        }
-    }
+    if (MODE == M_LOCAL) strip_track_end<V, R, RA>(best, j0, snap, sh);
     if (BAND) {
         // upper bounds on the paths that leave the window (exit_bound): first through its right
         // edge, cells (iend + 1, j), by a horizontal gap from (iend, j) or diagonally from
