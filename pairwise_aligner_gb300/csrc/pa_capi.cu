@@ -115,8 +115,8 @@ struct pa_ctx {
     // substitution matrix (PA_SCORE_MATRIX): int8 rank per byte (-1: not a symbol), int32 scores
     DevBuf mat_rank, mat_scores;
     int32_t mat_dim = 0, mat_max = 0, mat_min = 0;
-    // input path: rank table, invalid-symbol counter, packed staging of pa_align_batch_packed
-    DevBuf io_tab, io_ctr, in_words1, in_words2;
+    // input path: invalid-symbol counter, packed staging of pa_align_batch_packed
+    DevBuf io_ctr, in_words1, in_words2;
     // traceback: direction words of one chunk, their per-pair offsets, alignments and ops
     DevBuf tb_dir, tb_dir_off, tb_aln, tb_ops;
 };
@@ -1385,7 +1385,7 @@ pa_status pa_destroy(pa_ctx *c)
                       &c->ring, &c->rerun_long, &c->long_words, &c->long_cells16, &c->long_tasks, &c->long_start[0], &c->long_start[1],
                       &c->long_done[0], &c->long_done[1], &c->long_fail[0], &c->long_fail[1], &c->long_rec[0],
                       &c->long_rec[1], &c->mat_rank, &c->mat_scores,
-                      &c->io_tab, &c->io_ctr, &c->in_words1, &c->in_words2,
+                      &c->io_ctr, &c->in_words1, &c->in_words2,
                       &c->tb_dir, &c->tb_dir_off, &c->tb_aln, &c->tb_ops};
     for (DevBuf *b : bufs)
         if (b->p) cudaFree(b->p);
@@ -1811,12 +1811,16 @@ pa_status pa_align_batch_packed(pa_ctx *ctx, const pa_config *config, const uint
 
 // The input-path kernels on the caller's stream (or the context's); a non-null n_invalid waits
 // for the count.  The counter belongs to the context: calls on one context are not concurrent.
-static pa_status io_counter(pa_ctx *ctx, cudaStream_t st)
+// A null n_invalid needs no counter.
+static pa_status io_counter(pa_ctx *ctx, cudaStream_t st, const uint64_t *n_invalid, unsigned long long **ctr)
 {
     if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, PA_ERR_CUDA, "cudaSetDevice");
+    *ctr = nullptr;
+    if (!n_invalid) return PA_OK;
     pa_status s = ensure(ctx, ctx->io_ctr, 8);
     if (s) return s;
     PA_CUDA(ctx, cudaMemsetAsync(ctx->io_ctr.p, 0, 8, st));
+    *ctr = (unsigned long long *)ctx->io_ctr.p;
     return PA_OK;
 }
 
@@ -1844,11 +1848,9 @@ pa_status pa_rank_map_device(pa_ctx *ctx, const uint8_t *symbols, uint32_t n_sym
     for (uint32_t r = 0; r < n_symbols; ++r) table[symbols[r]] = (int8_t)r;   // a repeat keeps its last rank
     const cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     pa_status s;
-    if ((s = io_counter(ctx, st)) || (s = ensure(ctx, ctx->io_tab, 256))) return s;
-    PA_CUDA(ctx, cudaMemcpyAsync(ctx->io_tab.p, table, 256, cudaMemcpyHostToDevice, st));
-    PA_CUDA(ctx, cudaStreamSynchronize(st));      // `table` is a stack array
-    if (n) rank_map_launch(d_in, n, d_out, (const int8_t *)ctx->io_tab.p, (unsigned long long *)ctx->io_ctr.p,
-                           ctx->sm_count, st);
+    unsigned long long *ctr = nullptr;
+    if ((s = io_counter(ctx, st, n_invalid, &ctr))) return s;
+    if (n) rank_map_launch(d_in, n, d_out, table, ctr, ctx->sm_count, st);
     return io_finish(ctx, st, n_invalid);
 }
 
@@ -1859,8 +1861,9 @@ pa_status pa_pack_2bit_device(pa_ctx *ctx, const uint8_t *d_in, uint64_t n, uint
     if (n && (!d_in || !d_words)) return fail(ctx, PA_ERR_INVALID_ARGUMENT, "null buffer");
     const cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     pa_status s;
-    if ((s = io_counter(ctx, st))) return s;
-    if (n) pack_2bit_launch(d_in, n, d_words, (unsigned long long *)ctx->io_ctr.p, ctx->sm_count, st);
+    unsigned long long *ctr = nullptr;
+    if ((s = io_counter(ctx, st, n_invalid, &ctr))) return s;
+    if (n) pack_2bit_launch(d_in, n, d_words, ctr, ctx->sm_count, st);
     return io_finish(ctx, st, n_invalid);
 }
 

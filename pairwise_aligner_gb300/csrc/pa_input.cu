@@ -17,13 +17,102 @@ namespace pa {
 
 constexpr int kUnroll = 4;     // independent 16-byte loads in flight per thread
 
+// Four 3-bit fields at bits 0, 8, 16, 24 of x as the nibbles of a PRMT selector.  The dot products
+// run beside the ALU pipe, which bounds these kernels: shifts and masks in their place cost it 7
+// operations.
+__device__ __forceinline__ uint32_t nibbles(uint32_t x)
+{
+    const uint32_t lo = (uint32_t)__dp4a((int)x, 0x00001001, 0), hi = (uint32_t)__dp4a((int)x, 0x10010000, 0);
+    return hi * 256u + lo;
+}
+
+// 0x80 in every byte of x that is not zero (no carries between bytes).
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t x)
+{
+    return (((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x) & 0x80808080u;
+}
+
+// Count of marked bytes of m (0x80 or 0 each), as -128 per byte, added to acc.
+__device__ __forceinline__ int count_marks(uint32_t m, int acc) { return __dp4a((int)m, 0x01010101, acc); }
+
+// Adds the block's marked bytes to the counter, if the caller wants it.
+__device__ __forceinline__ void add_invalid(int acc, unsigned long long *invalid)
+{
+    if (!invalid) return;
+    unsigned bad = (unsigned)(-acc) >> 7;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
+    if ((threadIdx.x & 31) == 0 && bad) atomicAdd(invalid, (unsigned long long)bad);
+}
+
 // ---------------------------------------------------------------------------------------------
 // rank map: the reference's alphabet_rank_map_scalar keeps a 256-entry table (-1 for bytes that
 // are not symbols, alphabet_conversion/alphabet_rank_map_scalar.hpp); alphabet_rank_map_simd
-// gathers from the same table in SIMD registers (alphabet_rank_map_simd.hpp:31-117).  Here the
-// table is held 32 times in shared memory, word w of lane l at [w * 32 + l], so the 32 lanes of a
-// warp read 32 different banks whatever bytes they look up.
+// gathers from the same table in SIMD registers (alphabet_rank_map_simd.hpp:31-117).
+//
+// Alphabets of up to 8 symbols whose three bits from `shift` on differ (DNA: bits 1-3 of A, C, G,
+// T, N) are mapped four bytes at a time: one PRMT looks up the four ranks, another the letters
+// they belong to, and a byte that is not its letter gets -1.  12 ALU operations per 4 bytes
+// instead of the table's 32: 268 M bytes in 89 us, 0.89 of the copy bandwidth (table: 120 us).
 // ---------------------------------------------------------------------------------------------
+struct RankHash {
+    uint32_t ranks[2], letters[2];
+    int32_t shift;
+};
+
+__device__ __forceinline__ uint32_t hash4(const RankHash &h, uint32_t w, int &bad)
+{
+    const uint32_t sel = nibbles((w >> h.shift) & 0x07070707u);
+    const uint32_t m = nonzero_bytes(w ^ __byte_perm(h.letters[0], h.letters[1], sel));
+    bad = count_marks(m, bad);
+    return __byte_perm(h.ranks[0], h.ranks[1], sel) | __byte_perm(m, 0u, 0xba98);
+}
+
+__global__ void __launch_bounds__(256) k_rank_hash(const uint8_t *__restrict__ in, uint64_t n, int8_t *__restrict__ out,
+                                                   RankHash h, unsigned long long *__restrict__ invalid)
+{
+    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
+    const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    int bad = 0;
+    uint64_t done = 0;
+    if (vec) {
+        const uint64_t nv = n >> 4;
+        for (uint64_t v0 = tid; v0 < nv; v0 += kUnroll * nth) {
+            uint4 x[kUnroll];
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const uint64_t v = v0 + u * nth;
+                x[u] = v < nv ? __ldcs(reinterpret_cast<const uint4 *>(in) + v) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) {
+                const uint64_t v = v0 + u * nth;
+                if (v >= nv) break;
+                uint4 y;
+                y.x = hash4(h, x[u].x, bad);
+                y.y = hash4(h, x[u].y, bad);
+                y.z = hash4(h, x[u].z, bad);
+                y.w = hash4(h, x[u].w, bad);
+                __stcs(reinterpret_cast<uint4 *>(out) + v, y);
+            }
+        }
+        done = nv << 4;
+    }
+    for (uint64_t i = done + tid; i < n; i += nth) {    // the tail, or everything when unaligned
+        int one = 0;                                    // of the four copies of the byte, one counts
+        out[i] = (int8_t)hash4(h, in[i] * 0x01010101u, one);
+        bad += one / 4;
+    }
+    add_invalid(bad, invalid);
+}
+
+// Any other alphabet: the table is held 32 times in shared memory, word w of lane l at
+// [w * 32 + l], so the 32 lanes of a warp read 32 different banks whatever bytes they look up.
+struct RankTable {
+    int8_t rank[256];
+};
+
 __device__ __forceinline__ uint32_t rank4(const uint32_t *tab, int lane, uint32_t w)
 {
     uint32_t o = 0;
@@ -37,14 +126,14 @@ __device__ __forceinline__ uint32_t rank4(const uint32_t *tab, int lane, uint32_
 }
 
 __global__ void __launch_bounds__(256) k_rank_map(const uint8_t *__restrict__ in, uint64_t n,
-                                                  int8_t *__restrict__ out, const int8_t *__restrict__ table,
+                                                  int8_t *__restrict__ out, const __grid_constant__ RankTable table,
                                                   unsigned long long *__restrict__ invalid)
 {
     __shared__ uint32_t tab[64 * 32];
     for (int i = threadIdx.x; i < 64 * 32; i += blockDim.x) {
         const int w = i >> 5;
-        tab[i] = (uint32_t)(uint8_t)table[4 * w] | ((uint32_t)(uint8_t)table[4 * w + 1] << 8) |
-                 ((uint32_t)(uint8_t)table[4 * w + 2] << 16) | ((uint32_t)(uint8_t)table[4 * w + 3] << 24);
+        tab[i] = (uint32_t)(uint8_t)table.rank[4 * w] | ((uint32_t)(uint8_t)table.rank[4 * w + 1] << 8) |
+                 ((uint32_t)(uint8_t)table.rank[4 * w + 2] << 16) | ((uint32_t)(uint8_t)table.rank[4 * w + 3] << 24);
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -85,7 +174,7 @@ __global__ void __launch_bounds__(256) k_rank_map(const uint8_t *__restrict__ in
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
-    if (lane == 0 && bad) atomicAdd(invalid, (unsigned long long)bad);
+    if (lane == 0 && bad && invalid) atomicAdd(invalid, (unsigned long long)bad);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -93,17 +182,20 @@ __global__ void __launch_bounds__(256) k_rank_map(const uint8_t *__restrict__ in
 // four bytes of a word are coded at once with no lookup; a byte is a DNA letter when b | 0x20 is
 // one of a c g t.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t pack4(uint32_t w, unsigned &bad)
+__device__ __forceinline__ uint32_t pack4(uint32_t w, int &bad)
 {
     const uint32_t x = ((w >> 1) ^ (w >> 2)) & 0x03030303u;          // codes at bits 0, 8, 16, 24
     // the lower-case letter each code stands for (one PRMT); a byte is valid when b | 0x20 is it
-    const uint32_t sel = (x & 3u) | ((x >> 4) & 0x30u) | ((x >> 8) & 0x300u) | ((x >> 12) & 0x3000u);
-    const uint32_t diff = (w | 0x20202020u) ^ __byte_perm(0x74676361u, 0u, sel);
-    // bit 7 of a byte of z is set exactly when that byte of diff is zero (no carries between bytes)
-    const uint32_t z = ~(((diff & 0x7f7f7f7fu) + 0x7f7f7f7fu) | diff | 0x7f7f7f7fu);
-    bad += 4u - __popc(z);
-    const uint32_t y = x | (x >> 6);                                   // codes at bits 0-3, 16-19
-    return (y & 0xfu) | ((y >> 12) & 0xf0u);
+    bad = count_marks(nonzero_bytes((w | 0x20202020u) ^ __byte_perm(0x74676361u, 0u, nibbles(x))), bad);
+    return (uint32_t)__dp4a((int)x, 0x40100401, 0);                  // code k at bits 2k, 2k + 1
+}
+
+// Sixteen codes: the four bytes of codes joined by multiply-adds.  With the nibbles, the codes and
+// the count as dot products a word of 16 bases takes 32 ALU operations (80 before): 268 M bases in
+// 63 us, 0.79 of the copy bandwidth (84 us).
+__device__ __forceinline__ uint32_t pack16(uint4 v, int &bad)
+{
+    return ((pack4(v.w, bad) * 256u + pack4(v.z, bad)) * 256u + pack4(v.y, bad)) * 256u + pack4(v.x, bad);
 }
 
 __global__ void __launch_bounds__(256) k_pack_2bit(const uint8_t *__restrict__ in, uint64_t n,
@@ -114,7 +206,7 @@ __global__ void __launch_bounds__(256) k_pack_2bit(const uint8_t *__restrict__ i
     const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t nfull = n >> 4, nwords = (n + 15) >> 4;
     const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-    unsigned bad = 0;
+    int bad = 0;
     uint64_t first_slow = 0;
     if (vec) {
         for (uint64_t v0 = tid; v0 < nfull; v0 += kUnroll * nth) {
@@ -128,8 +220,7 @@ __global__ void __launch_bounds__(256) k_pack_2bit(const uint8_t *__restrict__ i
             for (int u = 0; u < kUnroll; ++u) {
                 const uint64_t v = v0 + u * nth;
                 if (v >= nfull) break;
-                words[v] = pack4(x[u].x, bad) | (pack4(x[u].y, bad) << 8) | (pack4(x[u].z, bad) << 16) |
-                           (pack4(x[u].w, bad) << 24);
+                __stcs(words + v, pack16(x[u], bad));
             }
         }
         first_slow = nfull;
@@ -151,13 +242,9 @@ __global__ void __launch_bounds__(256) k_pack_2bit(const uint8_t *__restrict__ i
                 w[k] = a;
             }
         }
-        const uint32_t out = pack4(w[0], bad) | (pack4(w[1], bad) << 8) | (pack4(w[2], bad) << 16) |
-                             (pack4(w[3], bad) << 24);
-        words[v] = out;
+        words[v] = pack16(make_uint4(w[0], w[1], w[2], w[3]), bad);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
-    if ((threadIdx.x & 31) == 0 && bad) atomicAdd(invalid, (unsigned long long)bad);
+    add_invalid(bad, invalid);
 }
 
 __device__ __forceinline__ uint32_t unpack4(uint32_t x)
@@ -213,10 +300,35 @@ static int stream_grid(int sm_count, uint64_t units)
     return (int)std::max<uint64_t>(1, std::min(want, cap));
 }
 
+// table: 256 ranks in host memory (they go with the launch's parameters).
 void rank_map_launch(const uint8_t *in, uint64_t n, int8_t *out, const int8_t *table, unsigned long long *invalid,
                      int sm_count, cudaStream_t st)
 {
-    k_rank_map<<<stream_grid(sm_count, (n + 15) / 16), 256, 0, st>>>(in, n, out, table, invalid);
+    const int grid = stream_grid(sm_count, (n + 15) / 16);
+    for (int shift = 0; shift <= 5; ++shift) {
+        uint8_t ranks[8], letters[8];
+        bool used[8] = {}, distinct = true;
+        // a slot without a symbol holds a byte of another slot, which no byte of this slot equals
+        for (int k = 0; k < 8; ++k) { ranks[k] = 0; letters[k] = (uint8_t)((k ^ 1) << shift); }
+        for (int b = 0; b < 256 && distinct; ++b) {
+            if (table[b] < 0) continue;
+            const int k = (b >> shift) & 7;
+            distinct = !used[k];
+            used[k] = true;
+            ranks[k] = (uint8_t)table[b];
+            letters[k] = (uint8_t)b;
+        }
+        if (!distinct) continue;
+        RankHash h;
+        std::memcpy(h.ranks, ranks, 8);
+        std::memcpy(h.letters, letters, 8);
+        h.shift = shift;
+        k_rank_hash<<<grid, 256, 0, st>>>(in, n, out, h, invalid);
+        return;
+    }
+    RankTable t;
+    std::memcpy(t.rank, table, 256);
+    k_rank_map<<<grid, 256, 0, st>>>(in, n, out, t, invalid);
 }
 
 void pack_2bit_launch(const uint8_t *in, uint64_t n, uint32_t *words, unsigned long long *invalid, int sm_count,
