@@ -119,6 +119,7 @@ struct pa_ctx {
     DevBuf io_ctr, in_words1, in_words2;
     // traceback: direction words of one chunk, their per-pair offsets, alignments and ops
     DevBuf tb_dir, tb_dir_off, tb_aln, tb_ops;
+    DevBuf tb_order, tb_cand, tb_words;   // tagged kernels: order and tickets, candidates, queue words
 };
 
 namespace {
@@ -432,16 +433,24 @@ void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const D
     c->last_launches++;
 }
 
-// Buffers of the long-pair kernel for a batch; the boundary cells start zeroed, so that no cell
-// carries a tag that a launch did not write.
-pa_status ensure_long(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
+// The boundary cells of row passes (16 bytes per streamed column) and the launch counter of their
+// tags; new cells are zeroed, so that none carries a tag that a launch did not write.
+pa_status ensure_cells(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
 {
     pa_status s;
-    const void *words = c->long_words.p, *cells = c->long_cells16.p;
+    const size_t words = c->long_words.cap, cells = c->long_cells16.cap;
     if ((s = ensure(c, c->long_words, 2 * sizeof(LongWords) + 8))) return s;
-    if (c->long_words.p != words) PA_CUDA(c, cudaMemsetAsync(c->long_words.p, 0, c->long_words.cap, c->stream));
+    if (c->long_words.cap != words) PA_CUDA(c, cudaMemsetAsync(c->long_words.p, 0, c->long_words.cap, c->stream));
     if ((s = ensure(c, c->long_cells16, (b1 + n_pairs) * 16))) return s;
-    if (c->long_cells16.p != cells) PA_CUDA(c, cudaMemsetAsync(c->long_cells16.p, 0, c->long_cells16.cap, c->stream));
+    if (c->long_cells16.cap != cells) PA_CUDA(c, cudaMemsetAsync(c->long_cells16.p, 0, c->long_cells16.cap, c->stream));
+    return PA_OK;
+}
+
+// Buffers of the long-pair kernel for a batch.
+pa_status ensure_long(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
+{
+    pa_status s = ensure_cells(c, n_pairs, b1);
+    if (s) return s;
     for (int k = 0; k < 2; ++k) {
         const uint64_t units = k == 0 ? (n_pairs + 1) / 2 : n_pairs;
         if ((s = ensure(c, c->long_start[k], (units + 1) * 4))) return s;
@@ -1386,7 +1395,8 @@ pa_status pa_destroy(pa_ctx *c)
                       &c->long_done[0], &c->long_done[1], &c->long_fail[0], &c->long_fail[1], &c->long_rec[0],
                       &c->long_rec[1], &c->mat_rank, &c->mat_scores,
                       &c->io_ctr, &c->in_words1, &c->in_words2,
-                      &c->tb_dir, &c->tb_dir_off, &c->tb_aln, &c->tb_ops};
+                      &c->tb_dir, &c->tb_dir_off, &c->tb_aln, &c->tb_ops,
+                      &c->tb_order, &c->tb_cand, &c->tb_words};
     for (DevBuf *b : bufs)
         if (b->p) cudaFree(b->p);
     for (DevBuf &b : c->band_list)
@@ -1701,6 +1711,8 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
     const bool use_matrix = C.rank_map != nullptr;
     std::vector<uint64_t> words(n_pairs);
     uint64_t cells = 0;
+    // values times 16 hold the directions in their low bits: scores below 2^26
+    bool tagged = !P.local || use_matrix || P.mismatch <= 0;
     for (uint64_t k = 0; k < n_pairs; ++k) {
         if (off1[k + 1] < off1[k] || off2[k + 1] < off2[k])
             return fail(ctx, PA_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing");
@@ -1708,8 +1720,9 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
         if (m >= (1ll << 30) || n >= (1ll << 30)) return fail(ctx, PA_ERR_TOO_LARGE, "sequence longer than 2^30");
         const int64_t a = std::abs((int64_t)P.match), b = std::abs((int64_t)P.mismatch);
         const int64_t o = -(int64_t)P.gap_open, e = -(int64_t)P.gap_ext;
-        if ((a + b) * std::min(m, n) + (o + e) * (m + n + 2) + 2 * o >= (1ll << 30))
-            return fail(ctx, PA_ERR_OVERFLOW, "scores of some pairs could exceed int32");
+        const int64_t most = (a + b) * std::min(m, n) + (o + e) * (m + n + 2) + 2 * o;
+        if (most >= (1ll << 30)) return fail(ctx, PA_ERR_OVERFLOW, "scores of some pairs could exceed int32");
+        tagged &= most < (1ll << 26);
         words[k] = (m && n) ? (uint64_t)((n + kTracebackPassRows - 1) / kTracebackPassRows) * (m + 31) * 32 : 0;
         if (words[k] > kTbBudgetWords) return fail(ctx, PA_ERR_TOO_LARGE, "a pair needs more than 4 GiB of directions");
         cells += (uint64_t)(m * n);
@@ -1728,7 +1741,8 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
     if ((s = ensure(ctx, ctx->in_seq1, b1)) || (s = ensure(ctx, ctx->in_seq2, b2)) ||
         (s = ensure(ctx, ctx->in_off1, (n_pairs + 1) * 8)) || (s = ensure(ctx, ctx->in_off2, (n_pairs + 1) * 8)) ||
         (s = ensure(ctx, ctx->in_out, n_pairs * sizeof(pa_result))) ||
-        (s = ensure(ctx, ctx->boundary, (b1 + n_pairs) * sizeof(Cell))) ||
+        (s = tagged ? ensure_cells(ctx, n_pairs, b1) : ensure(ctx, ctx->boundary, (b1 + n_pairs) * sizeof(Cell))) ||
+        (s = ensure(ctx, ctx->tb_order, (2 * n_pairs + 1) * 4)) ||
         (s = ensure(ctx, ctx->tb_aln, n_pairs * sizeof(pa_alignment))) || (s = ensure(ctx, ctx->tb_ops, b1 + b2)) ||
         (s = ensure(ctx, ctx->tb_dir_off, n_pairs * 8)))
         return s;
@@ -1758,6 +1772,29 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
         L.matrix = (const int32_t *)ctx->mat_scores.p;
         L.dim = ctx->mat_dim;
     }
+    // tagged kernels: the chunk's pairs by size, largest first (buckets of a quarter octave of
+    // their cells), and the tickets of their passes
+    uint32_t *tb_words = nullptr;                        // error, two queue heads
+    std::vector<uint32_t> order(tagged ? 2 * n_pairs + 1 : 0);
+    if (tagged) {
+        if ((s = ensure(ctx, ctx->tb_words, 32))) return s;
+        tb_words = (uint32_t *)ctx->tb_words.p;
+        PA_CUDA(ctx, cudaMemsetAsync(tb_words, 0, 32, st));
+        L.queue = tb_words + 1;
+        L.error = tb_words;
+        L.my_epoch = (unsigned long long *)(tb_words + 4);
+        L.epoch = long_epoch(ctx);
+        L.cells = (ulonglong2 *)ctx->long_cells16.p;
+        L.spin_limit = ctx->wait_limit;
+        L.tables = std::abs((int64_t)P.match) <= 63 && std::abs((int64_t)P.mismatch) <= 63;
+        L.order = (const uint32_t *)ctx->tb_order.p;
+    }
+    auto size_bucket = [&](uint64_t k) -> int {
+        const uint64_t x = (off1[k + 1] - off1[k]) * (off2[k + 1] - off2[k]);
+        if (x < 8) return (int)x;
+        const int e = 63 - __builtin_clzll(x);
+        return 4 * e + (int)((x >> (e - 2)) & 3);
+    };
     const int grid = traceback_grid(ctx->sm_count);
     uint64_t launches = 0;
     for (uint64_t first = 0; first < n_pairs;) {
@@ -1770,21 +1807,42 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
         if ((s = ensure(ctx, ctx->tb_dir, std::max<uint64_t>(total, 1) * 4))) return s;
         // the previous chunk's kernel may still read the offsets: copy them in stream order
         PA_CUDA(ctx, cudaMemcpyAsync(ctx->tb_dir_off.p, dir_off.data(), (end - first) * 8, cudaMemcpyHostToDevice, st));
-        PA_CUDA(ctx, cudaStreamSynchronize(st));        // dir_off is reused by the next chunk
+        if (tagged) {
+            const uint32_t cnt = (uint32_t)(end - first);
+            uint32_t at[257] = {}, *start = order.data() + cnt, tasks = 0;
+            for (uint64_t k = first; k < end; ++k) ++at[255 - size_bucket(k) + 1];
+            for (int x = 0; x < 256; ++x) at[x + 1] += at[x];
+            for (uint64_t k = first; k < end; ++k) order[at[255 - size_bucket(k)]++] = (uint32_t)(k - first);
+            for (uint32_t u = 0; u < cnt; ++u) {
+                const uint64_t k = first + order[u], n = off2[k + 1] - off2[k];
+                start[u] = tasks;
+                if (off1[k + 1] > off1[k]) tasks += (uint32_t)((n + 2 * kTracebackPassRows - 1) / (2 * kTracebackPassRows));
+            }
+            start[cnt] = tasks;
+            if ((s = ensure(ctx, ctx->tb_cand, std::max<uint64_t>(tasks, 1) * sizeof(int4)))) return s;
+            PA_CUDA(ctx, cudaMemcpyAsync(ctx->tb_order.p, order.data(), (2ull * cnt + 1) * 4, cudaMemcpyHostToDevice, st));
+            L.start = L.order + cnt;
+            L.cand = (int4 *)ctx->tb_cand.p;
+        }
+        PA_CUDA(ctx, cudaStreamSynchronize(st));        // the host arrays are reused by the next chunk
         L.first = (uint32_t)first;
         L.count = (uint32_t)(end - first);
         L.dir_off = (const uint64_t *)ctx->tb_dir_off.p;
         L.dir = (uint32_t *)ctx->tb_dir.p;
-        traceback_launch(grid, st, L, P);
-        ++launches;
+        if (tagged) traceback_tag_launch(ctx->sm_count, st, L, P);
+        else traceback_launch(grid, st, L, P);
+        launches += tagged ? 3 : 1;
         first = end;
     }
+    uint32_t wait_error = 0;
+    if (tagged) PA_CUDA(ctx, cudaMemcpyAsync(&wait_error, tb_words, 4, cudaMemcpyDeviceToHost, st));
     PA_CUDA(ctx, cudaGetLastError());
     PA_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
     PA_CUDA(ctx, cudaMemcpyAsync(out, ctx->in_out.p, n_pairs * sizeof(pa_result), cudaMemcpyDeviceToHost, st));
     PA_CUDA(ctx, cudaMemcpyAsync(alignments, ctx->tb_aln.p, n_pairs * sizeof(pa_alignment), cudaMemcpyDeviceToHost, st));
     if (b1 + b2) PA_CUDA(ctx, cudaMemcpyAsync(ops, ctx->tb_ops.p, b1 + b2, cudaMemcpyDeviceToHost, st));
     PA_CUDA(ctx, cudaStreamSynchronize(st));
+    if (wait_error) return fail(ctx, PA_ERR_TIMEOUT, "a wait between the passes of a pair ran out");
     if (stats) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);

@@ -96,8 +96,21 @@ struct TbLaunch {
     const int8_t *rank;             // substitution matrix (or null: match / mismatch)
     const int32_t *matrix;
     int32_t dim;
+    // tagged kernels: the chunk's pairs largest first, their first tickets (count + 1 words), a
+    // candidate per ticket, the queue heads (2 words), boundary cells (cell 0 of pair k at
+    // (off1[k] - off1[0]) + k), the launch counter and this launch's number
+    const uint32_t *order, *start;
+    int4 *cand;
+    uint32_t *queue;
+    ulonglong2 *cells;
+    unsigned long long *epoch, *my_epoch;
+    uint32_t *error;
+    uint32_t spin_limit;
+    int32_t tables;                 // 2 * match + 1 and 2 * mismatch + 1 fit a signed byte
 };
 int traceback_grid(int sm_count);
 void traceback_launch(int grid, cudaStream_t stream, const TbLaunch &L, const DpParams &P);
+// The tagged kernels (scores below 2^26): all passes of the chunk in one queue, then the walks.
+void traceback_tag_launch(int sm_count, cudaStream_t stream, const TbLaunch &L, const DpParams &P);
 
 }  // namespace pa

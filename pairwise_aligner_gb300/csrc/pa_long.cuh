@@ -47,6 +47,9 @@ struct LongUnit {
     int32_t fail;                  // a wait of this pass ran out
 };
 
+// A cell's tag: the launch (a counter of the context), then the pass.
+constexpr int kTagPassBits = 24;
+
 __device__ __forceinline__ ulonglong2 load_cell128(const ulonglong2 *p)
 {
     ulonglong2 v;
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
             u.passes = (u.nh + 32 * u.rpt - 1) / (32 * u.rpt);
             const uint32_t owner = u.m[1] > u.m[0] ? u.id[1] : u.id[0];
             u.row = Q.cells + (L.off1[owner] + owner);        // cells 0..m(owner) = 0..ms
-            u.tag = (epoch << 13) | (uint32_t)p;              // at most 2^20 / 128 = 8,192 passes
+            u.tag = (epoch << kTagPassBits) | (uint32_t)p;
             if (BAND)
                 for (int k = 0; k < 3; ++k) u.win[k] = long_window<NL>(L, u, min(max(p + k - 1, 0), u.passes - 1));
             su = u;

@@ -16,11 +16,16 @@
 // direction words of a step (ra rows x 4 bits each) are contiguous: word (p * (m + 31) + s) * 32
 // + t.  The walk back reads cell (i, j) at p = (j-1) / 256, t = ((j-1) % 256) / ra_p,
 // s = i + t - 1, nibble ((j-1) % 256) % ra_p.
+//
+// This kernel (k_traceback) computes a pair's passes and its walk on one warp.  It takes the calls
+// whose scores need more than 26 bits, and local byte comparison with a positive mismatch; all
+// others run on the tagged kernels of pa_traceback_tag.cuh.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "pa_launch.h"
+#include "pa_traceback_tag.cuh"
 
 namespace pa {
 
@@ -317,6 +322,30 @@ void traceback_launch(int grid, cudaStream_t st, const TbLaunch &L, const DpPara
         if (mat) k_traceback<false, true><<<grid, 128, 0, st>>>(L, P);
         else k_traceback<false, false><<<grid, 128, 0, st>>>(L, P);
     }
+}
+
+template <bool LOCAL, int SC>
+static void tag_dp(int grid, cudaStream_t st, const TbLaunch &L, const DpParams &P)
+{
+    k_tb_dp<LOCAL, SC><<<grid, kTagThreads, 0, st>>>(L, P);
+}
+
+void traceback_tag_launch(int sm_count, cudaStream_t st, const TbLaunch &L, const DpParams &P)
+{
+    const int grid = 4 * sm_count;
+    k_tb_start<<<1, 1, 0, st>>>(L);
+    const int sc = L.matrix ? SC_PROFILE : L.tables ? SC_TABLE : SC_BYTES;
+    if (P.local) {
+        if (sc == SC_TABLE) tag_dp<true, SC_TABLE>(grid, st, L, P);
+        else if (sc == SC_BYTES) tag_dp<true, SC_BYTES>(grid, st, L, P);
+        else tag_dp<true, SC_PROFILE>(grid, st, L, P);
+    } else {
+        if (sc == SC_TABLE) tag_dp<false, SC_TABLE>(grid, st, L, P);
+        else if (sc == SC_BYTES) tag_dp<false, SC_BYTES>(grid, st, L, P);
+        else tag_dp<false, SC_PROFILE>(grid, st, L, P);
+    }
+    if (P.local) k_tb_walk<true><<<8 * sm_count, kTagThreads, 0, st>>>(L, P);
+    else k_tb_walk<false><<<8 * sm_count, kTagThreads, 0, st>>>(L, P);
 }
 
 }  // namespace pa
