@@ -32,6 +32,14 @@ __device__ __forceinline__ uint32_t nonzero_bytes(uint32_t x)
     return (((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x) & 0x80808080u;
 }
 
+// 0xff in every marked byte of m: PRMT with sign replication (which __byte_perm masks out).
+__device__ __forceinline__ uint32_t fill_marks(uint32_t m)
+{
+    uint32_t d;
+    asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(d) : "r"(m));
+    return d;
+}
+
 // Count of marked bytes of m (0x80 or 0 each), as -128 per byte, added to acc.
 __device__ __forceinline__ int count_marks(uint32_t m, int acc) { return __dp4a((int)m, 0x01010101, acc); }
 
@@ -65,7 +73,7 @@ __device__ __forceinline__ uint32_t hash4(const RankHash &h, uint32_t w, int &ba
     const uint32_t sel = nibbles((w >> h.shift) & 0x07070707u);
     const uint32_t m = nonzero_bytes(w ^ __byte_perm(h.letters[0], h.letters[1], sel));
     bad = count_marks(m, bad);
-    return __byte_perm(h.ranks[0], h.ranks[1], sel) | __byte_perm(m, 0u, 0xba98);
+    return __byte_perm(h.ranks[0], h.ranks[1], sel) | fill_marks(m);
 }
 
 __global__ void __launch_bounds__(256) k_rank_hash(const uint8_t *__restrict__ in, uint64_t n, int8_t *__restrict__ out,
