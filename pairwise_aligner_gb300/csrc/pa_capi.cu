@@ -39,6 +39,9 @@ constexpr int kDefaultG = 8;       // threads per group
 // counters of a finished call (stage_stats).  Each is read only after a wait on the stream
 // that wrote it, and written only after the previous call's work on that stream finished.
 constexpr size_t kPinnedBytes = 1024;
+// Behind them, staging of small host calls: their inputs go over in one copy and their results
+// come back through page-locked words (a copy from or to pageable memory costs 5-10 us each).
+constexpr size_t kStageIn = 192 << 10, kStageOut = 64 << 10;
 constexpr int kShortVariant = 9;   // variants 9, 10: dp_short, 16 / 32 rows per thread
 constexpr int kVariants = kShortVariant + kShortFormCount;   // 0..8: dp_kernel (pa_kern_v*.cu)
 constexpr int kDefaultShortVariant = kShortVariant;          // with the rule below: 16 or 32 rows per thread
@@ -76,17 +79,18 @@ struct pa_ctx {
     cudaEvent_t ev_dp0 = nullptr, ev_dp1 = nullptr;   // bracket the DP kernels of the last call
     cudaStream_t side = nullptr;                      // s16x2 long pairs (highest priority)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaStream_t side2 = nullptr;                     // s32 and byte-compare pairs
-    cudaEvent_t ev_join2 = nullptr;
+    cudaStream_t side2 = nullptr;                     // s32 pairs
+    cudaStream_t side3 = nullptr;                     // byte-compare pairs
+    cudaEvent_t ev_join2 = nullptr, ev_join3 = nullptr;
     uint8_t *pinned = nullptr;                        // page-locked host words for band mode's reads
     pa_options opt{};
     std::string err;
     // device work buffers (grow only)
-    DevBuf keys, order, hist, starts, cursor, sums, ranges, counts, qtab, boundary, rerun, counters, pstats;
+    DevBuf keys, order, hist, starts, cursor, sums, ranges, counts, qtab, boundary, rerun, counters;
     DevBuf slots;                 // short-pair kernel: 16-byte column slots, (seq1_bytes + n_pairs)
     // long pairs (dp_long): queue words and launch counter, boundary cells, and per queue (s16x2,
-    // s32) the units' first tickets, finished passes, failed waits and records
-    DevBuf long_words, long_cells16, long_tasks, long_start[2], long_done[2], long_fail[2], long_rec[2];
+    // s32, redo in s32) the units' first tickets, finished passes, failed waits and records
+    DevBuf long_words, long_cells16, long_tasks, long_start[3], long_done[3], long_fail[3], long_rec[3];
     bool use_long = false;        // this call's batch may hold long pairs
     DevBuf ring, rerun_long;      // CTA mode: boundary rows per block; s16 long pairs to redo in s32
     int32_t ring_m = 0;           // longest sequence1 the ring rows hold (0: no CTA mode yet)
@@ -97,7 +101,7 @@ struct pa_ctx {
     int32_t team_max_n = 12288;       // byte-compare long pairs of at most this many rows run on teams
     uint32_t wait_limit = kSpinLimit; // polls of a CTA-mode progress wait before it gives up
     int64_t want_ring_m = 0;          // the next call's longest CTA-mode sequence1 (host: exact)
-    DevBuf in_seq1, in_off1, in_seq2, in_off2, in_out;   // staging for the host-buffer entry points
+    DevBuf in_seq1, in_off1, in_seq2, in_off2, in_out, in_small;   // staging for the host-buffer entry points
     int G[3] = {kDefaultG, kDefaultG, kDefaultG};
     int variant[3] = {0, 0, 0};
     pa_tuning tuning{};           // per method (0 local, 1 global) and s16 table; applied per call
@@ -134,6 +138,9 @@ Cell *cluster_ring(pa_ctx *c)
 {
     return (Cell *)c->ring.p + (size_t)c->ring_grid * 8 * ((size_t)c->ring_m + 2);
 }
+
+// The call's statistics, behind its 32 counter words.
+PrepStats *pstats(pa_ctx *c) { return (PrepStats *)((char *)c->counters.p + 128); }
 
 pa_status fail(pa_ctx *c, pa_status s, const std::string &msg)
 {
@@ -439,7 +446,7 @@ pa_status ensure_cells(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
 {
     pa_status s;
     const size_t words = c->long_words.cap, cells = c->long_cells16.cap;
-    if ((s = ensure(c, c->long_words, 2 * sizeof(LongWords) + 8))) return s;
+    if ((s = ensure(c, c->long_words, 3 * sizeof(LongWords) + 8))) return s;
     if (c->long_words.cap != words) PA_CUDA(c, cudaMemsetAsync(c->long_words.p, 0, c->long_words.cap, c->stream));
     if ((s = ensure(c, c->long_cells16, (b1 + n_pairs) * 16))) return s;
     if (c->long_cells16.cap != cells) PA_CUDA(c, cudaMemsetAsync(c->long_cells16.p, 0, c->long_cells16.cap, c->stream));
@@ -451,7 +458,7 @@ pa_status ensure_long(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
 {
     pa_status s = ensure_cells(c, n_pairs, b1);
     if (s) return s;
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < 3; ++k) {
         const uint64_t units = k == 0 ? (n_pairs + 1) / 2 : n_pairs;
         if ((s = ensure(c, c->long_start[k], (units + 1) * 4))) return s;
         if ((s = ensure(c, c->long_done[k], units * 4))) return s;
@@ -478,7 +485,7 @@ int long_grid(pa_ctx *c, bool lanes16, int mode) { return dp_long_occupancy(lane
 
 // The pass queues of one or two lists (s16x2 units, s32 units); a null list gets no block.
 // The word that counts long-pair launches.
-unsigned long long *long_epoch(pa_ctx *c) { return (unsigned long long *)((LongWords *)c->long_words.p + 2); }
+unsigned long long *long_epoch(pa_ctx *c) { return (unsigned long long *)((LongWords *)c->long_words.p + 3); }
 
 void plan_long(pa_ctx *c, cudaStream_t st, const uint64_t *o1, const uint64_t *o2, int mode, const LongPlan *p16, const LongPlan *p32)
 {
@@ -495,16 +502,23 @@ pa_status enqueue_prep(pa_ctx *c, const DpParams &P, const ClassCfg &C, const ui
                        uint64_t n_pairs)
 {
     cudaStream_t st = c->stream;
-    PA_CUDA(c, cudaMemsetAsync(c->hist.p, 0, sizeof(uint32_t) * kBuckets, st));
-    PA_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 128, st));
-    PA_CUDA(c, cudaMemsetAsync(c->pstats.p, 0, sizeof(PrepStats), st));
+    const bool small = n_pairs <= kSortSmall;
+    if (!small) PA_CUDA(c, cudaMemsetAsync(c->hist.p, 0, sizeof(uint32_t) * kBuckets, st));
+    PA_CUDA(c, cudaMemsetAsync(c->counters.p, 0, 128 + sizeof(PrepStats), st));   // and the statistics behind them
     // one resident wave (16 blocks of 4 warps per SM), each warp a stride of pairs: every block
     // adds its statistics to the same few global counters once, so fewer blocks contend less
     int cls_blocks = (int)std::min<uint64_t>((n_pairs * 32 + 127) / 128, (uint64_t)c->sm_count * 16);
     if (cls_blocks < 1) cls_blocks = 1;
     k_classify<<<cls_blocks, 128, 0, st>>>(s1, o1, b1, s2, o2, b2, n_pairs, P, C, (uint32_t *)c->keys.p,
-                                              (uint32_t *)c->hist.p, (uint32_t *)c->qtab.p, out,
-                                              (PrepStats *)c->pstats.p);
+                                              small ? nullptr : (uint32_t *)c->hist.p, (uint32_t *)c->qtab.p, out,
+                                              pstats(c));
+    if (small) {
+        k_sort_small<<<1, 1024, 0, st>>>((const uint32_t *)c->keys.p, (uint32_t)n_pairs, (uint32_t *)c->order.p,
+                                         (uint32_t *)c->ranges.p, (uint32_t *)c->counts.p, pstats(c), out);
+        c->last_launches += 2;
+        PA_CUDA(c, cudaGetLastError());
+        return PA_OK;
+    }
     k_scan_blocks<<<kBuckets / 1024, 1024, 0, st>>>((uint32_t *)c->hist.p, (uint32_t *)c->starts.p,
                                                     (uint32_t *)c->sums.p);
     k_scan_sums<<<1, kBuckets / 1024, 0, st>>>((uint32_t *)c->sums.p, kBuckets / 1024);
@@ -513,7 +527,7 @@ pa_status enqueue_prep(pa_ctx *c, const DpParams &P, const ClassCfg &C, const ui
     const int sc_blocks = (int)std::max<uint64_t>(1, (n_pairs + kBlock - 1) / kBlock);
     k_scatter<<<sc_blocks, kBlock, 0, st>>>((uint32_t *)c->keys.p, n_pairs, (uint32_t *)c->cursor.p,
                                             (uint32_t *)c->order.p, (uint32_t *)c->ranges.p,
-                                            (uint32_t *)c->counts.p, (const PrepStats *)c->pstats.p, out);
+                                            (uint32_t *)c->counts.p, pstats(c), out);
     c->last_launches += 6;
     PA_CUDA(c, cudaGetLastError());
     return PA_OK;
@@ -559,11 +573,18 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
     // inside a capture the record must become a graph node to fire on every replay
     const unsigned ev_flags = capturing == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     PA_CUDA(c, cudaEventRecordWithFlags(c->ev_dp0, st, ev_flags));
-    // Three branches run side by side after the bucket sort; each kernel finds its list empty or
-    // not on the device.  The long pairs' passes go to the side stream of the highest priority,
-    // so that they take the SMs first and the short pairs fill what their last passes leave.
+    // Four branches run side by side after the bucket sort; each kernel finds its list empty or not
+    // on the device, and a call with few pairs waits for the longest branch, not for every launch
+    // (1,024 reads: 33 us of empty launches beside the DP).  The s16x2 long pairs go to the side
+    // stream of the highest priority and are planned before the short pairs start, so that they
+    // take the SMs first and the short pairs fill what their last passes leave.
     const bool use_long = C.pass_queue != 0;
     LongPlan plan[2];
+    DpLaunch LL = L;
+    LL.error = counters + 8;
+    LL.rerun_list = (uint32_t *)c->rerun_long.p;
+    LL.rerun_count = counters + 6;
+    LL.G = 32;
     if (use_long) {
         for (int k = 0; k < 2; ++k)
             plan[k] = LongPlan{(const uint32_t *)c->order.p, ranges + (k == 0 ? K_S16L : K_S32L),
@@ -572,11 +593,7 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
     }
     PA_CUDA(c, cudaEventRecord(c->ev_fork, st));
     PA_CUDA(c, cudaStreamWaitEvent(c->side2, c->ev_fork, 0));
-    DpLaunch LL = L;
-    LL.error = counters + 8;
-    LL.rerun_list = (uint32_t *)c->rerun_long.p;
-    LL.rerun_count = counters + 6;
-    LL.G = 32;
+    PA_CUDA(c, cudaStreamWaitEvent(c->side3, c->ev_fork, 0));
     if (use_long) {
         PA_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
         for (int k = 0; k < 2; ++k) {
@@ -584,66 +601,67 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
             dp_long_launch(k == 0, mode, long_grid(c, k == 0, mode), k == 0 ? c->side : c->side2, LL, plan[k].Q, P);
             c->last_launches++;
         }
+        if (mode != M_LOCAL) {
+            // s16 results of long pairs that failed the exactness check, recomputed in s32
+            LongPlan redo{(const uint32_t *)c->rerun_long.p, counters + 5, counters + 6, 1, long_queue(c, 2)};
+            plan_long(c, c->side, o1, o2, mode, nullptr, &redo);
+            DpLaunch LR = LL;
+            LR.order = redo.order;
+            LR.begin_ptr = redo.begin; LR.count_ptr = redo.count; LR.unit_counter = counters + 12;
+            LR.rerun = 1;
+            dp_long_launch(false, mode, long_grid(c, false, mode), c->side, LR, redo.Q, P);
+            c->last_launches++;
+        }
         PA_CUDA(c, cudaEventRecord(c->ev_join, c->side));
     }
-    // s16x2 class
+    // s16x2 class, and its results that failed the exactness check, recomputed in s32
     L.begin_ptr = ranges + K_S16; L.count_ptr = counts + K_S16; L.unit_counter = counters + 0; L.G = c->G[K_S16];
     launch_class(c, K_S16, mode, true, false, L, P, st);
+    if (mode != M_LOCAL) {
+        DpLaunch LR = L;
+        LR.order = (const uint32_t *)c->rerun.p;
+        LR.begin_ptr = counters + 5;         // always zero
+        LR.count_ptr = counters + 4;
+        LR.unit_counter = counters + 3;
+        LR.rerun = 1;
+        LR.G = c->G[K_S32];
+        launch_class(c, K_S32, mode, false, false, LR, P, st);
+    }
     // s32 class
     L.begin_ptr = ranges + K_S32; L.count_ptr = counts + K_S32; L.unit_counter = counters + 1; L.G = c->G[K_S32];
     launch_class(c, K_S32, mode, false, false, L, P, c->side2);
     // byte-compare class, its long pairs on clusters, whole blocks (which take the largest pairs
     // that the router left them first) and teams of 4 warps
     L.begin_ptr = ranges + K_GEN; L.count_ptr = counts + K_GEN; L.unit_counter = counters + 2; L.G = c->G[K_GEN];
-    launch_class(c, K_GEN, mode, false, true, L, P, c->side2);
+    launch_class(c, K_GEN, mode, false, true, L, P, c->side3);
     if (use_long && c->ring.p) {
         const int cl_grid = dp_cluster_grid(mode, c->ring_grid);
-        k_route_huge<<<1, 1, 0, c->side2>>>(counts, (uint32_t)(cl_grid / kClusterBlocks), counters + 16);
+        k_route_huge<<<1, 1, 0, c->side3>>>(counts, (uint32_t)(cl_grid / kClusterBlocks), counters + 16);
         LL.ring_stride = (uint64_t)c->ring_m + 2;
         LL.ring = cluster_ring(c);
         LL.begin_ptr = ranges + K_GENH; LL.count_ptr = counters + 16; LL.unit_counter = counters + 13;
-        PA_CUDA(c, dp_cluster_launch(mode, cl_grid, c->side2, LL, P));
+        PA_CUDA(c, dp_cluster_launch(mode, cl_grid, c->side3, LL, P));
         LL.ring = (Cell *)c->ring.p;
         LL.begin_ptr = ranges + K_GENL; LL.count_ptr = counts + K_GENL; LL.unit_counter = counters + 11;
         LL.lead_order = (const uint32_t *)c->order.p;
         LL.lead_begin_ptr = ranges + K_GENH;
         LL.lead_count_ptr = counters + 17;
-        dp_cta_launch(mode, c->ring_grid, c->side2, LL, P);
+        dp_cta_launch(mode, c->ring_grid, c->side3, LL, P);
         LL.lead_order = nullptr;
         LL.lead_begin_ptr = LL.lead_count_ptr = nullptr;
         c->last_launches += 3;
         if (C.team_max_n > 0) {
             LL.ring = team_ring(c);
             LL.begin_ptr = ranges + K_GENM; LL.count_ptr = counts + K_GENM; LL.unit_counter = counters + 14;
-            dp_team_launch(mode, c->ring_grid, c->side2, LL, P);
+            dp_team_launch(mode, c->ring_grid, c->side3, LL, P);
             c->last_launches++;
         }
     }
     PA_CUDA(c, cudaEventRecord(c->ev_join2, c->side2));
+    PA_CUDA(c, cudaEventRecord(c->ev_join3, c->side3));
     PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join2, 0));
-    if (use_long) {
-        PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));   // the long pairs' results and redo list
-        if (mode != M_LOCAL) {
-            // s16 results of long pairs that failed the exactness check, recomputed in s32
-            LongPlan redo{(const uint32_t *)c->rerun_long.p, counters + 5, counters + 6, 1, long_queue(c, 1)};
-            plan_long(c, st, o1, o2, mode, nullptr, &redo);
-            LL.order = redo.order;
-            LL.begin_ptr = redo.begin; LL.count_ptr = redo.count; LL.unit_counter = counters + 12;
-            LL.rerun = 1;
-            dp_long_launch(false, mode, long_grid(c, false, mode), st, LL, redo.Q, P);
-            c->last_launches++;
-        }
-    }
-    // s16 global results that failed the exactness check, recomputed in s32
-    if (mode != M_LOCAL) {
-        L.order = (const uint32_t *)c->rerun.p;
-        L.begin_ptr = counters + 5;          // always zero
-        L.count_ptr = counters + 4;
-        L.unit_counter = counters + 3;
-        L.rerun = 1;
-        L.G = c->G[K_S32];
-        launch_class(c, K_S32, mode, false, false, L, P, st);
-    }
+    PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join3, 0));
+    if (use_long) PA_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));
     PA_CUDA(c, cudaEventRecordWithFlags(c->ev_dp1, st, ev_flags));
     PA_CUDA(c, cudaGetLastError());
     (void)cfg;
@@ -686,8 +704,7 @@ pa_status prepare_buffers(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
     if ((s = ensure(c, c->sums, sizeof(uint32_t) * 1024))) return s;
     if ((s = ensure(c, c->ranges, 64))) return s;
     if ((s = ensure(c, c->counts, 64))) return s;
-    if ((s = ensure(c, c->counters, 128))) return s;
-    if ((s = ensure(c, c->pstats, sizeof(PrepStats)))) return s;
+    if ((s = ensure(c, c->counters, 128 + sizeof(PrepStats)))) return s;
     if ((s = ensure(c, c->qtab, (b1 + np) * 4))) return s;
     if ((s = ensure(c, c->boundary, (b1 + np) * sizeof(Cell)))) return s;
     if ((s = ensure(c, c->slots, (b1 + np) * sizeof(Slot)))) return s;
@@ -869,7 +886,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     {
         // the classifier checked the offsets; a batch with inconsistent ones is not aligned (and
         // the band features, which read the sequences, must not run on it)
-        PA_CUDA(c, cudaMemcpyAsync(h_bad, &((PrepStats *)c->pstats.p)->bad_offsets, 8, cudaMemcpyDeviceToHost, st));
+        PA_CUDA(c, cudaMemcpyAsync(h_bad, &pstats(c)->bad_offsets, 8, cudaMemcpyDeviceToHost, st));
         PA_CUDA(c, cudaMemcpyAsync(h_ranges, c->ranges.p, 64, cudaMemcpyDeviceToHost, st));
         PA_CUDA(c, cudaMemcpyAsync(h_counts, c->counts.p, 4 * kClasses, cudaMemcpyDeviceToHost, st));
         PA_CUDA(c, cudaEventRecord(c->ev_join, st));
@@ -1141,7 +1158,7 @@ constexpr size_t kPinStats = 512;      // PrepStats, then 16 counter words
 void stage_stats(pa_ctx *c, cudaStream_t st)
 {
     static_assert(kPinStats + sizeof(PrepStats) + 64 <= kPinnedBytes, "page-locked words");
-    cudaMemcpyAsync(c->pinned + kPinStats, c->pstats.p, sizeof(PrepStats), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(c->pinned + kPinStats, pstats(c), sizeof(PrepStats), cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(c->pinned + kPinStats + sizeof(PrepStats), c->counters.p, 64, cudaMemcpyDeviceToHost, st);
 }
 
@@ -1154,7 +1171,7 @@ pa_status read_stats(pa_ctx *c, pa_stats *stats, bool staged)
         std::memcpy(&ps, c->pinned + kPinStats, sizeof(ps));
         std::memcpy(ctr, c->pinned + kPinStats + sizeof(PrepStats), sizeof(ctr));
     } else {
-        PA_CUDA(c, cudaMemcpy(&ps, c->pstats.p, sizeof(ps), cudaMemcpyDeviceToHost));
+        PA_CUDA(c, cudaMemcpy(&ps, pstats(c), sizeof(ps), cudaMemcpyDeviceToHost));
         PA_CUDA(c, cudaMemcpy(ctr, c->counters.p, sizeof(ctr), cudaMemcpyDeviceToHost));
     }
     if (stats) {
@@ -1349,10 +1366,12 @@ pa_status pa_create(pa_ctx **out, int device_ordinal, const pa_options *options)
         cudaDeviceGetStreamPriorityRange(nullptr, &high) != cudaSuccess ||
         cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, high) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->side3, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaHostAlloc((void **)&c->pinned, kPinnedBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaHostAlloc((void **)&c->pinned, kPinnedBytes + kStageIn + kStageOut, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         pa_destroy(c);
         return PA_ERR_CUDA;
@@ -1387,13 +1406,13 @@ pa_status pa_destroy(pa_ctx *c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     drop_graphs(c);
     DevBuf *bufs[] = {&c->keys, &c->order, &c->hist, &c->starts, &c->cursor, &c->sums, &c->ranges,
-                      &c->counts, &c->qtab, &c->boundary, &c->slots, &c->rerun, &c->counters, &c->pstats,
-                      &c->in_seq1, &c->in_off1, &c->in_seq2, &c->in_off2, &c->in_out,
+                      &c->counts, &c->qtab, &c->boundary, &c->slots, &c->rerun, &c->counters,
+                      &c->in_seq1, &c->in_off1, &c->in_seq2, &c->in_off2, &c->in_out, &c->in_small,
                       &c->band_spec, &c->band_win, &c->band_code, &c->band_bsum, &c->band_ctr, &c->band_in,
                       &c->mlp_feat, &c->mlp_x, &c->mlp_h1, &c->mlp_h2, &c->mlp_out,
                       &c->ring, &c->rerun_long, &c->long_words, &c->long_cells16, &c->long_tasks, &c->long_start[0], &c->long_start[1],
-                      &c->long_done[0], &c->long_done[1], &c->long_fail[0], &c->long_fail[1], &c->long_rec[0],
-                      &c->long_rec[1], &c->mat_rank, &c->mat_scores,
+                      &c->long_start[2], &c->long_done[0], &c->long_done[1], &c->long_done[2], &c->long_fail[0],
+                      &c->long_fail[1], &c->long_fail[2], &c->long_rec[0], &c->long_rec[1], &c->long_rec[2], &c->mat_rank, &c->mat_scores,
                       &c->io_ctr, &c->in_words1, &c->in_words2,
                       &c->tb_dir, &c->tb_dir_off, &c->tb_aln, &c->tb_ops,
                       &c->tb_order, &c->tb_cand, &c->tb_words};
@@ -1413,7 +1432,9 @@ pa_status pa_destroy(pa_ctx *c)
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->side2) cudaStreamDestroy(c->side2);
+    if (c->side3) cudaStreamDestroy(c->side3);
     if (c->ev_join2) cudaEventDestroy(c->ev_join2);
+    if (c->ev_join3) cudaEventDestroy(c->ev_join3);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -1621,6 +1642,44 @@ static pa_status align_host(pa_ctx *ctx, const pa_config *config, const uint8_t 
     const uint64_t base1 = off1[0], base2 = off2[0];
     const uint64_t b1 = off1[n_pairs] - base1, b2 = off2[n_pairs] - base2;
     pa_status s;
+    const size_t off_bytes = (size_t)(n_pairs + 1) * 8;
+    if (!packed && !(config && config->band_mode) && n_pairs * sizeof(pa_result) <= kStageOut && b1 <= kStageIn &&
+        b2 <= kStageIn && 2 * off_bytes + b1 + 16 + b2 <= kStageIn) {
+        // a small call: offsets (rebased to 0) and sequences side by side in one copy
+        uint8_t *h = ctx->pinned + kPinnedBytes;
+        uint64_t *r1 = (uint64_t *)h, *r2 = (uint64_t *)(h + off_bytes);
+        const size_t at1 = 2 * off_bytes, at2 = at1 + ((b1 + 15) & ~(uint64_t)15);
+        int64_t long_m = 0;
+        for (uint64_t k = 0; k <= n_pairs; ++k) {
+            r1[k] = off1[k] - base1;
+            r2[k] = off2[k] - base2;
+            if (k == 0) continue;
+            if (off1[k] < off1[k - 1] || off2[k] < off2[k - 1])
+                return fail(ctx, PA_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing");
+            const int64_t m = (int64_t)(r1[k] - r1[k - 1]), n = (int64_t)(r2[k] - r2[k - 1]);
+            if (m * n >= ctx->long_cells) long_m = std::max(long_m, m);
+        }
+        std::memcpy(h + at1, seq1 + base1, b1);
+        std::memcpy(h + at2, seq2 + base2, b2);
+        ctx->want_ring_m = long_m;
+        ctx->use_long = long_m > 0;
+        if ((s = ensure(ctx, ctx->in_small, kStageIn)) || (s = ensure(ctx, ctx->in_out, n_pairs * sizeof(pa_result))))
+            return s;
+        cudaStream_t st = ctx->stream;
+        uint8_t *d = (uint8_t *)ctx->in_small.p, *h_out = h + kStageIn;
+        PA_CUDA(ctx, cudaMemcpyAsync(d, h, at2 + b2, cudaMemcpyHostToDevice, st));
+        s = run_device(ctx, config, d + at1, (const uint64_t *)d, b1, d + at2, (const uint64_t *)(d + off_bytes), b2,
+                       n_pairs, (pa_result *)ctx->in_out.p, stats, false);
+        if (s) {
+            cudaStreamSynchronize(st);                // the staging words are free again
+            return s;
+        }
+        PA_CUDA(ctx, cudaMemcpyAsync(h_out, ctx->in_out.p, n_pairs * sizeof(pa_result), cudaMemcpyDeviceToHost, st));
+        stage_stats(ctx, st);
+        PA_CUDA(ctx, cudaStreamSynchronize(st));
+        std::memcpy(out, h_out, n_pairs * sizeof(pa_result));
+        return read_stats(ctx, stats, true);
+    }
     if ((s = ensure(ctx, ctx->in_seq1, b1))) return s;
     if ((s = ensure(ctx, ctx->in_seq2, b2))) return s;
     if ((s = ensure(ctx, ctx->in_off1, (n_pairs + 1) * 8))) return s;

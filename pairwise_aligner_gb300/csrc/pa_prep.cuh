@@ -186,7 +186,7 @@ __global__ void k_classify(const uint8_t *__restrict__ seq1, const uint64_t *__r
                 my_cells += (unsigned long long)(m * n);
             }
             keys[p] = key;
-            atomicAdd(&hist[key], 1u);
+            if (hist) atomicAdd(&hist[key], 1u);
             atomicAdd(&sh[1 + klass], 1ull);
         }
     }
@@ -285,6 +285,55 @@ __global__ void k_scatter(const uint32_t *__restrict__ keys, uint64_t n_pairs, u
     if ((key >> kClassShift) == K_NONE) return;
     const uint32_t pos = atomicAdd(&cursor[key], 1u);
     order[pos] = (uint32_t)p;
+}
+
+// A batch of at most kSortSmall pairs: the bucket sort's result by one block, a bitonic sort of
+// (key, pair) words in shared memory, instead of clearing, scanning and reading back 2^20 buckets
+// (1,024 pairs: 7 us and four launches less; the order within a bucket is by pair).  Steps whose
+// partners are at most 32 apart stay within a warp's 64 words.
+constexpr uint32_t kSortSmall = 4096;
+static_assert(kKeyBits == 20, "a key and a pair number share 32 bits");
+
+__global__ void __launch_bounds__(1024) k_sort_small(const uint32_t *__restrict__ keys, uint32_t n,
+                                                     uint32_t *__restrict__ order, uint32_t *__restrict__ ranges,
+                                                     uint32_t *__restrict__ counts, const PrepStats *__restrict__ st,
+                                                     pa_result *__restrict__ out)
+{
+    __shared__ uint32_t w[kSortSmall];
+    uint32_t size = 64;
+    while (size < n) size <<= 1;
+    const bool bad = st->bad_offsets != 0;
+    for (uint32_t x = threadIdx.x; x < size; x += 1024) w[x] = x < n ? (keys[x] << 12) | x : 0xffffffffu;
+    __syncthreads();
+    for (uint32_t k = 2; k <= size; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t x = threadIdx.x; x < size / 2; x += 1024) {
+                const uint32_t a = 2 * x - (x & (j - 1)), b = a + j;
+                const uint32_t u = w[a], v = w[b];
+                if ((u > v) == ((a & k) == 0)) { w[a] = v; w[b] = u; }
+            }
+            if (j > 32 || (j == 1 && k >= 64)) __syncthreads();
+            else __syncwarp();
+        }
+    __syncthreads();
+    for (uint32_t x = threadIdx.x; x < n; x += 1024) {
+        order[x] = w[x] & 4095u;
+        if (bad) out[x] = error_result(PA_RESULT_ERROR);
+    }
+    // class begins: the first word of class c or above
+    __shared__ uint32_t begin[16];
+    if (threadIdx.x < 16) {
+        uint32_t lo = 0, hi = n;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) / 2;
+            if ((w[mid] >> (12 + kClassShift)) < threadIdx.x) lo = mid + 1;
+            else hi = mid;
+        }
+        begin[threadIdx.x] = lo;
+        ranges[threadIdx.x] = lo;
+    }
+    __syncthreads();
+    if (threadIdx.x < kClasses) counts[threadIdx.x] = bad ? 0u : begin[threadIdx.x + 1] - begin[threadIdx.x];
 }
 
 // The pass queues of one or two long-pair launches (dp_long) that run side by side: start[u] for
