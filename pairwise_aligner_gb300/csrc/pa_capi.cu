@@ -35,8 +35,8 @@ constexpr int64_t kDefaultRingM = 65536;   // device entry points: CTA mode up t
 constexpr int kDefaultG = 8;       // threads per group
 // Page-locked host words of a context: [0, 8) band mode's bad-offset count, [16, 80) class
 // ranges, [80, 144) class counts, [160, 224) the two band steps' totals, [224, 236) the long
-// full-DP routing counts, [256, 280) full-DP list sizes (host to device), [512, 736) the
-// counters of a finished call (stage_stats).  Each is read only after a wait on the stream
+// full-DP routing counts, [256, 280) full-DP list sizes (host to device), from 512 the
+// counters and statistics of a finished call (stage_stats).  Each is read only after a wait on the stream
 // that wrote it, and written only after the previous call's work on that stream finished.
 constexpr size_t kPinnedBytes = 1024;
 // Behind them, staging of small host calls: their inputs go over in one copy and their results
@@ -589,13 +589,17 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
         for (int k = 0; k < 2; ++k)
             plan[k] = LongPlan{(const uint32_t *)c->order.p, ranges + (k == 0 ? K_S16L : K_S32L),
                                counts + (k == 0 ? K_S16L : K_S32L), k == 0 ? 2 : 1, long_queue(c, k)};
-        plan_long(c, st, o1, o2, mode, &plan[0], &plan[1]);
     }
+    // with few pairs the short ones do not wait for the plan (their kernel leaves SMs free anyway)
+    const bool plan_first = n_pairs > kSortSmall;
+    if (use_long && plan_first) plan_long(c, st, o1, o2, mode, &plan[0], &plan[1]);
     PA_CUDA(c, cudaEventRecord(c->ev_fork, st));
-    PA_CUDA(c, cudaStreamWaitEvent(c->side2, c->ev_fork, 0));
     PA_CUDA(c, cudaStreamWaitEvent(c->side3, c->ev_fork, 0));
     if (use_long) {
         PA_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
+        if (!plan_first) plan_long(c, c->side, o1, o2, mode, &plan[0], &plan[1]);
+        PA_CUDA(c, cudaEventRecord(c->ev_join, c->side));
+        PA_CUDA(c, cudaStreamWaitEvent(c->side2, c->ev_join, 0));
         for (int k = 0; k < 2; ++k) {
             LL.begin_ptr = plan[k].begin; LL.count_ptr = plan[k].count; LL.unit_counter = counters + 9 + k;
             dp_long_launch(k == 0, mode, long_grid(c, k == 0, mode), k == 0 ? c->side : c->side2, LL, plan[k].Q, P);
@@ -613,6 +617,8 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
             c->last_launches++;
         }
         PA_CUDA(c, cudaEventRecord(c->ev_join, c->side));
+    } else {
+        PA_CUDA(c, cudaStreamWaitEvent(c->side2, c->ev_fork, 0));
     }
     // s16x2 class, and its results that failed the exactness check, recomputed in s32
     L.begin_ptr = ranges + K_S16; L.count_ptr = counts + K_S16; L.unit_counter = counters + 0; L.G = c->G[K_S16];
@@ -1154,12 +1160,11 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
 
 // Queue the copies of the call's counters into page-locked host words (read_stats with
 // staged = true reads them after the caller's wait on `st`).
-constexpr size_t kPinStats = 512;      // PrepStats, then 16 counter words
+constexpr size_t kPinStats = 512;      // the 32 counter words, then PrepStats, as on the device
 void stage_stats(pa_ctx *c, cudaStream_t st)
 {
-    static_assert(kPinStats + sizeof(PrepStats) + 64 <= kPinnedBytes, "page-locked words");
-    cudaMemcpyAsync(c->pinned + kPinStats, pstats(c), sizeof(PrepStats), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(c->pinned + kPinStats + sizeof(PrepStats), c->counters.p, 64, cudaMemcpyDeviceToHost, st);
+    static_assert(kPinStats + 128 + sizeof(PrepStats) <= kPinnedBytes, "page-locked words");
+    cudaMemcpyAsync(c->pinned + kPinStats, c->counters.p, 128 + sizeof(PrepStats), cudaMemcpyDeviceToHost, st);
 }
 
 // Counters of the finished call (after a sync): class sizes, reruns, error bits.
@@ -1168,8 +1173,8 @@ pa_status read_stats(pa_ctx *c, pa_stats *stats, bool staged)
     PrepStats ps;
     uint32_t ctr[16];
     if (staged) {
-        std::memcpy(&ps, c->pinned + kPinStats, sizeof(ps));
-        std::memcpy(ctr, c->pinned + kPinStats + sizeof(PrepStats), sizeof(ctr));
+        std::memcpy(&ps, c->pinned + kPinStats + 128, sizeof(ps));
+        std::memcpy(ctr, c->pinned + kPinStats, sizeof(ctr));
     } else {
         PA_CUDA(c, cudaMemcpy(&ps, pstats(c), sizeof(ps), cudaMemcpyDeviceToHost));
         PA_CUDA(c, cudaMemcpy(ctr, c->counters.p, sizeof(ctr), cudaMemcpyDeviceToHost));
@@ -1182,8 +1187,8 @@ pa_status read_stats(pa_ctx *c, pa_stats *stats, bool staged)
         cudaGetLastError();
         const uint64_t rr = (uint64_t)ctr[4] + ctr[6];
         stats->cells = ps.cells;
-        stats->pairs_s16 = ps.n_class[K_S16] + ps.n_class[K_S16L] + ps.n_class[K_S16H] + ps.n_class[K_S16M] - rr;
-        stats->pairs_s32 = ps.n_class[K_S32] + ps.n_class[K_S32L] + ps.n_class[K_S32H] + ps.n_class[K_S32M] + rr;
+        stats->pairs_s16 = ps.n_class[K_S16] + ps.n_class[K_S16L] - rr;
+        stats->pairs_s32 = ps.n_class[K_S32] + ps.n_class[K_S32L] + rr;
         stats->pairs_general = ps.n_class[K_GEN] + ps.n_class[K_GENL] + ps.n_class[K_GENH] + ps.n_class[K_GENM];
         stats->pairs_trivial = ps.n_class[K_NONE];
         stats->pairs_rerun = rr;

@@ -20,8 +20,8 @@
 // last thread spills its bottom row per column to the pass-boundary scratch
 // (8 bytes per column), where thread 0 of the next pass reads it.
 //
-// Instruction budget (sm_103: PRMT, LOP3 and the 3-operand DPX forms take two
-// ALU issue slots, the 2-operand __vmaxs2 one, integer adds go to another pipe);
+// Instruction budget (sm_103: PRMT, LOP3 and the two- and three-operand max forms all run on the
+// ALU pipe at one warp-instruction per two cycles, constant subtractions as IMAD on the FMA pipe);
 // per register (two cells of s16x2 lanes):
 //     s  = PRMT(table_a, table_b, selector)            score of both lanes
 //     t  = VIADDMAX(diag, s, hgap)                      max(diag + s, hgap)
@@ -693,6 +693,7 @@ __device__ __forceinline__ void pass_body(const DpLaunch &L, const DpParams &P, 
     const uint32_t NEGV = NL == 2 ? w.CLAMP : (uint32_t)kNeg32;
     int2 bprev = make_int2(1, w.ms), bcur = bprev, bnext = bprev;
     const bool more = p + 1 < w.passes;
+    static_assert(MODE != M_BAND || SYNC == 0, "long pairs in band mode run on the pass queue");
     if (MODE == M_BAND) {
         bcur = band_window<NL>(L, w, p);
         if (p > 0) bprev = band_window<NL>(L, w, p - 1);
@@ -703,13 +704,7 @@ __device__ __forceinline__ void pass_body(const DpLaunch &L, const DpParams &P, 
         w.iend = bcur.y;
         const int32_t c0 = bcur.x - 1;
         w.diag0 = NEGV;
-        if (t == 0 && p > 0 && c0 >= bprev.x && c0 <= bprev.y) {
-            if (SYNC && w.seen < w.base_in + c0) {
-                w.seen = wait_progress<SYNC>(w.prog_in, w.base_in + c0, L.error, L.spin_limit);
-                if (w.seen == INT32_MAX) w.wait_failed = true;
-            }
-            w.diag0 = load_cell<SYNC>(w.bin + c0).h;
-        }
+        if (t == 0 && p > 0 && c0 >= bprev.x && c0 <= bprev.y) w.diag0 = load_cell<SYNC>(w.bin + c0).h;
     }
     switch (rpt / kChunk) {
     case 1: run_pass<V, R, 4, MODE, GEN, VAR, SYNC>(L, P, w, p, t, G, gmask, snap); break;
