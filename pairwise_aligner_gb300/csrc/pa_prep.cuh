@@ -83,8 +83,8 @@ __device__ void trivial_result(const DpParams &P, int32_t m, int32_t n, pa_resul
 // lie inside the buffer (`bytes` long) are loaded at once and tested four bytes at a time: the
 // letter that each byte's code stands for, by one PRMT (its selector a dot product), against the
 // byte; the buffer's ragged ends are read byte by byte.  The classification waits on memory, one pair
-after the other; with this and the next pair's offsets in flight 262,144 pairs of 64-512 bp take
-135 us, against 161 us with four byte loads per lane.
+// after the other; with this and the next pair's offsets in flight 262,144 pairs of 64-512 bp take
+// 135 us, against 161 us with four byte loads per lane.
 __device__ __forceinline__ bool all_dna(const uint8_t *seq, uint64_t bytes, uint64_t from, int64_t n, int lane)
 {
     const uintptr_t first = reinterpret_cast<uintptr_t>(seq + from), last = first + (uint64_t)n;
