@@ -24,10 +24,11 @@
 //
 // Bound: the integer ALU pipe, as in the short-pair kernel, while the queue is full; the column
 // steps of the longest passes at its end.  Measured per call (GB300) against blocks, 4-warp teams
-// and clusters of 4 blocks per pair: 4,001 global long reads of 500-20,000 bp 75.7 -> 15.0 ms
-// (4.9 T cells/s of DP), 32,768 pairs of a mixed stream 678 -> 105 ms (5.2 T), 500 local contig
-// pairs, part s32, 72.8 -> 12.4 ms.  Reading the boundary one column ahead instead of in staged
-// blocks of 16: 19.1, 131 and 14.8 ms.
+// and clusters of 4 blocks per pair: 4,001 global long reads of 500-20,000 bp 75.7 -> 14.4 ms
+// (5.1 T cells/s), 32,768 pairs of a mixed stream 678 -> 94-108 ms by draw (5.3 T), 500 local
+// contig pairs, part s32, 72.8 -> 10.8 ms.  Reading the boundary one column ahead instead of in
+// staged blocks of 16 took 1.2-1.3 times as long.  Blocks of one or two warps instead of eight:
+// long reads 14.1 -> 15.8 / 15.5 ms.
 #pragma once
 #include "pa_launch.h"
 #include "pa_short.cuh"
