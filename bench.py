@@ -60,9 +60,9 @@ WORKLOAD = "config2_local_262144_pairs_64-512bp_+1/-4/-6/-1"
 BAND_MODEL = os.path.join(REPO, "pairwise_aligner_gb300", "data", "band_model.npz")
 # DRAM bytes per cell of the short-pair local DP kernel (dp_short, 8 lanes per group, 32 rows
 # per thread), from one ncu capture of its launch on all 262,144 pairs of this workload:
-# dram__bytes.sum.per_second (207.49 GB/s) x gpu__time_duration.sum (4.95712 ms) over the
-# launch's 2.1770e10 cells.  Most of it is the write-back of the 16-byte column slots.
-DRAM_BYTES_PER_CELL = 207.492454e9 * 4.957120e-3 / 21769527988
+# dram__bytes.sum (997.6 MB in 4.41 ms) over the launch's 2.1770e10 cells.  Most of it is the
+# write-back of the 16-byte column slots.
+DRAM_BYTES_PER_CELL = 997621504 / 21769527988
 
 
 def env_rank():
