@@ -58,7 +58,7 @@ struct StripConst {
 template <class V, int NT = kBlock>
 struct StripShared {
     int32_t (*c)[3][NT];           // [lane][field][thread]
-    int32_t (*bi)[NT];             // [lane][thread]
+    int32_t (*bi)[NT];             // [lane][thread]; free last rows: the column, then the value
     __device__ __forceinline__ int32_t &s(int l) { return c[l][0][threadIdx.x]; }
     __device__ __forceinline__ int32_t &i(int l) { return c[l][1][threadIdx.x]; }
     __device__ __forceinline__ int32_t &j(int l) { return c[l][2][threadIdx.x]; }
@@ -195,6 +195,52 @@ __device__ __forceinline__ void strip_ends(const DpParams &P, const U &u, const 
     }
 }
 
+// Free end of sequence2's last row, after every column of a thread that holds such a row (strip
+// indices r0, r1 of the lanes): on a strict improvement the column and the stored value go to
+// shared memory.  `seen` is the best so far as a stored value of the current column (H - shift *
+// column, so one add-max moves it on), kept one below the clamp: a clamped value then counts
+// exactly as its comparison in true scores would.  Comparing the candidates in shared memory on
+// every column took 30 % of the kernel's instructions: 65,537 reads of 100-250 bp in windows 1,334
+// -> 1,098 us (comparing only on an improvement: 1,514, as a read's first columns all improve).
+template <class V, int MODE, int RA, int NT, class U>
+__device__ __forceinline__ void strip_end_track(const U &u, const uint32_t *H, uint32_t &seen, uint32_t shift_neg,
+                                                int32_t i, int32_t r0, int32_t r1, uint4 *snap, StripShared<V, NT> &sh)
+{
+    constexpr int NL = V::LANES;
+#pragma unroll
+    for (int v = 0; v < RA / 4; ++v) snap[v * NT] = make_uint4(H[4 * v], H[4 * v + 1], H[4 * v + 2], H[4 * v + 3]);
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(snap);
+    uint32_t x = row[(r0 >> 2) * (4 * NT) + (r0 & 3)], moved;
+    if (NL == 2) {
+        x = prmt(x, row[(r1 >> 2) * (4 * NT) + (r1 & 3)], 0x7610);
+        moved = __viaddmax_s16x2(seen, shift_neg, V::splat(StripConst<V, MODE>::clampt - 1));
+    } else {
+        moved = (uint32_t)__viaddmax_s32((int)seen, (int)shift_neg, kNeg32 - 1);
+    }
+    seen = V::max2(moved, x);
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+        if (V::improved(seen ^ moved, l) && i <= u.m[l]) {
+            sh.bi[l][threadIdx.x] = i;
+            sh.bi[NL + l][threadIdx.x] = (int32_t)x;
+        }
+    }
+}
+
+// ... and after the pass: its candidates.
+template <class V, int MODE, int NT, class U>
+__device__ __forceinline__ void strip_end_offer(const DpParams &P, const U &u, const int32_t *own,
+                                                StripShared<V, NT> &sh)
+{
+#pragma unroll
+    for (int l = 0; l < V::LANES; ++l) {
+        const int32_t i = sh.bi[l][threadIdx.x];
+        if (own[l] >= 0 && i > 0)
+            sh.offer(l, V::get((uint32_t)sh.bi[V::LANES + l][threadIdx.x], l) + P.shift * i - StripConst<V, MODE>::Kt,
+                     i, u.n[l]);
+    }
+}
+
 // Results of a finished unit from its candidates (one thread): the free-end borders, the s16
 // exactness check (a result at the floor goes to the s32 redo list), the failed waits.
 template <class V, int MODE>
@@ -326,6 +372,16 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
         mmin = min(mmin, u.m[l]);
     }
 
+    // the end rule of the last row (strip_end_track)
+    const bool row_end = MODE == M_GLOBAL_FREE && P.last_column_free && any_own;
+    uint32_t seen = NL == 2 ? V::splat(KC::clampt - 1) : (uint32_t)(kNeg32 - 1);
+    const uint32_t shift_neg = V::splat(-P.shift);
+    const int32_t r0 = max(own[0], 0), r1 = max(own[NL - 1], 0);
+    if (row_end) {
+#pragma unroll
+        for (int l = 0; l < NL; ++l) sh.bi[l][threadIdx.x] = 0;
+    }
+
     // step s of the pass: thread t computes column i = s - t + 1 when 1 <= i <= ms
     auto step = [&](int32_t s, bool active) {
         const int32_t i = s - t + 1;
@@ -361,8 +417,11 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
             if (writer) *reinterpret_cast<uint2 *>(&slot[i].h) = make_uint2(sH, sE);
             if (MODE == M_LOCAL)
                 strip_track<V, R, RA>(H, best, i, snap, sh);
-            else if ((MODE == M_GLOBAL_FREE && P.last_column_free && any_own) || i >= mmin)
-                strip_ends<V, MODE, RA>(P, u, H, i, j0, any_own, snap, sh, [&](int l) { return own[l]; });
+            else {
+                if (row_end) strip_end_track<V, MODE, RA, NT>(u, H, seen, shift_neg, i, r0, r1, snap, sh);
+                if (i >= mmin)
+                    strip_ends<V, MODE, RA>(P, u, H, i, j0, any_own, snap, sh, [&](int l) { return own[l]; });
+            }
         }
     };
     // The groups of a warp keep step with one another: loops of their own would let them drift apart
@@ -377,6 +436,7 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
     }
     for (; s < ms_max + G - 1; ++s) step(s, (uint32_t)(s - t) < (uint32_t)ms);
     if (MODE == M_LOCAL) strip_track_end<V, R, RA>(best, j0, snap, sh);
+    if (row_end) strip_end_offer<V, MODE, NT>(P, u, own, sh);
 }
 
 // With fewer work items than warps, only the first warps of every block take any: otherwise the
@@ -504,7 +564,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) dp_short(DpLaunch L, DpParams P)
     __shared__ uint4 snap_store[(MODE == M_LOCAL ? NL : 1) * (R / 4) * NT];
     __shared__ ShortUnit s_unit[NT / G];
     __shared__ int32_t s_cand[NL][3][NT];
-    __shared__ int32_t s_bi[MODE == M_LOCAL ? NL : 1][NT];
+    __shared__ int32_t s_bi[MODE == M_LOCAL ? NL : MODE == M_GLOBAL_FREE ? 2 * NL : 1][NT];
     __shared__ uint32_t s_mat[SC == SC_PROFILE ? 33 : 1][8];
     extern __shared__ uint4 s_prof[];
     uint4 *snap = snap_store + threadIdx.x;
