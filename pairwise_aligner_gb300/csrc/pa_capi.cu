@@ -737,7 +737,7 @@ int tune_shape_class(uint64_t n_pairs, uint64_t b1, uint64_t b2)
 // column step) that still gives every resident warp about three work units, so that the largest
 // pairs do not outlast the rest, and that holds a pair of mean length in two passes.  A warp unit
 // holds 32 / G groups of `lanes` pairs, a pass G * rows rows.  Measured (GB300, us per call on 8 /
-// 16 / 32 lanes): 65,537 reads of 175 rows 1,353 / 1,502 / 2,005; 16,384 pairs of 64-1,000 rows
+// 16 / 32 lanes): 65,537 reads of 175 rows 1,119 / 1,156 / 1,514; 16,384 pairs of 64-1,000 rows
 // 1,653 / 935 / 580; 60,000 local pairs of 288 rows 1,316 / 1,244 / 1,464; 32,768 proteins of 335
 // rows (16 per thread) 2,342 / 1,548 / 1,588.  Groups of 4 lanes pay for pairs of at most 128
 // rows, one pass of them: 262,144 local pairs of 288 rows 8,195, on 8 lanes 4,696.
