@@ -50,6 +50,7 @@ struct StripConst {
     static constexpr bool S16 = V::LANES == 2;
     static constexpr int32_t Kt = !S16 ? 0 : MODE == M_LOCAL ? 2048 : 32767 - 512;
     static constexpr int32_t clampt = S16 ? 2048 : MODE == M_LOCAL ? 0 : INT32_MIN;
+    static constexpr int32_t below = (S16 ? clampt : kNeg32) - 1;     // less than any stored value
     static constexpr int32_t floor_true = !S16 ? INT32_MIN : MODE == M_LOCAL ? 0 : 2048 - Kt;
 };
 
@@ -213,9 +214,9 @@ __device__ __forceinline__ void strip_end_track(const U &u, const uint32_t *H, u
     uint32_t x = row[(r0 >> 2) * (4 * NT) + (r0 & 3)], moved;
     if (NL == 2) {
         x = prmt(x, row[(r1 >> 2) * (4 * NT) + (r1 & 3)], 0x7610);
-        moved = __viaddmax_s16x2(seen, shift_neg, V::splat(StripConst<V, MODE>::clampt - 1));
+        moved = __viaddmax_s16x2(seen, shift_neg, V::splat(StripConst<V, MODE>::below));
     } else {
-        moved = (uint32_t)__viaddmax_s32((int)seen, (int)shift_neg, kNeg32 - 1);
+        moved = (uint32_t)__viaddmax_s32((int)seen, (int)shift_neg, StripConst<V, MODE>::below);
     }
     seen = V::max2(moved, x);
 #pragma unroll
@@ -374,7 +375,7 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
 
     // the end rule of the last row (strip_end_track)
     const bool row_end = MODE == M_GLOBAL_FREE && P.last_column_free && any_own;
-    uint32_t seen = NL == 2 ? V::splat(KC::clampt - 1) : (uint32_t)(kNeg32 - 1);
+    uint32_t seen = V::splat(KC::below);
     const uint32_t shift_neg = V::splat(-P.shift);
     const int32_t r0 = max(own[0], 0), r1 = max(own[NL - 1], 0);
     if (row_end) {
