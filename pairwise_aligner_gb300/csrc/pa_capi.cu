@@ -273,6 +273,9 @@ int dp_short_occupancy_free(int form);
 void dp_short_launch_local(int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
 void dp_short_launch_global(int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
 void dp_short_launch_free(int form, int grid, cudaStream_t st, const DpLaunch &L, const DpParams &P);
+cudaError_t dp_short32_allow_local();
+cudaError_t dp_short32_allow_global();
+cudaError_t dp_short32_allow_free();
 int dp_short32_occupancy_local(int scoring, int dim);
 int dp_short32_occupancy_global(int scoring, int dim);
 int dp_short32_occupancy_free(int scoring, int dim);
@@ -303,8 +306,8 @@ void dp_long_launch(bool lanes16, int mode, int grid, cudaStream_t st, const DpL
 
 static int mode_slot(int mode) { return mode == M_LOCAL ? 0 : mode == M_GLOBAL ? 1 : 2; }
 
-// Resident blocks per SM, looked up once (outside any capture: warm_occupancy and, for the
-// profiles of a matrix, pa_set_substitution_matrix).
+// Resident blocks per SM, looked up once per process (outside any capture: warm_occupancy and, for
+// the profiles of a matrix, pa_set_substitution_matrix).
 int dp_short_occupancy(int form, int mode)
 {
     static int cache[3][kShortFormCount];
@@ -1559,6 +1562,10 @@ pa_status pa_set_substitution_matrix(pa_ctx *ctx, const uint8_t *symbols, uint32
         lo = std::min(lo, scores[k]);
     }
     if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, PA_ERR_CUDA, "cudaSetDevice");
+    // the profile kernels' shared memory, on this context's device whatever another one has asked for
+    PA_CUDA(ctx, dp_short32_allow_local());
+    PA_CUDA(ctx, dp_short32_allow_global());
+    PA_CUDA(ctx, dp_short32_allow_free());
     PA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));      // no call in flight reads the old matrix
     PA_CUDA(ctx, cudaStreamSynchronize(ctx->side));
     pa_status s;

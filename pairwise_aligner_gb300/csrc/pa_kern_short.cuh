@@ -19,8 +19,6 @@ int occ_short(int smem)
                         : k == 1 ? (const void *)dp_short<V, SC, MODE, 16, R, NT>
                         : k == 2 ? (const void *)dp_short<V, SC, MODE, 8, R, NT>
                                  : (const void *)dp_short<V, SC, MODE, 4, R, NT>;
-        // the limit for any matrix, so that a small one does not lower it for a larger one
-        if (smem > 0) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * NT * 16);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, f, NT, smem);
         per_sm = v < per_sm ? v : per_sm;
     }
@@ -52,6 +50,22 @@ void go_short16(int form, int grid, cudaStream_t st, const DpLaunch &L, const Dp
 {
     if (form == 1) go_short<L16, SC_TABLE, MODE, 32, kBlock>(grid, 0, st, L, P);
     else go_short<L16, SC_TABLE, MODE, 16, kBlock>(grid, 0, st, L, P);
+}
+
+// Lets the profile kernels use the shared memory of the largest matrix (32 symbols) on the current
+// device.  The attribute belongs to the device, so every context asks for its own.
+template <int MODE>
+cudaError_t allow_profiles()
+{
+    constexpr int NT = kProfileThreads, bytes = 32 * NT * 16;
+    const void *f[4] = {(const void *)dp_short<L32, SC_PROFILE, MODE, 32, 16, NT>,
+                        (const void *)dp_short<L32, SC_PROFILE, MODE, 16, 16, NT>,
+                        (const void *)dp_short<L32, SC_PROFILE, MODE, 8, 16, NT>,
+                        (const void *)dp_short<L32, SC_PROFILE, MODE, 4, 16, NT>};
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 4 && e == cudaSuccess; ++k)
+        e = cudaFuncSetAttribute(f[k], cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e;
 }
 
 template <int MODE>

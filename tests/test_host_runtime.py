@@ -1,0 +1,85 @@
+"""The library's host logic on a make-believe CUDA runtime (cpp/host_runtime.cpp): two devices, no
+kernel runs, every launch, allocation and occupancy query is on record."""
+from __future__ import annotations
+
+import ctypes
+import os
+import re
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import REPO
+
+
+class HostRuntime:
+    def __init__(self, path):
+        from pairwise_aligner_gb300 import _lib
+        self._lib = _lib
+        self.lib = _lib.load(path)
+        for name, res in (("events", ctypes.c_char_p), ("most", ctypes.c_size_t), ("reset", None), ("limit", None)):
+            fn = getattr(self.lib, "host_runtime_" + name)
+            fn.restype = res
+            setattr(self, "_" + name, fn)
+        self._limit.argtypes = [ctypes.c_size_t]
+
+    def context(self, device=0, **opt):
+        o = self._lib.PaOptions()
+        o.kernel_variant = -1
+        for k, v in opt.items():
+            setattr(o, k, v)
+        p = ctypes.c_void_p()
+        assert self.lib.pa_create(ctypes.byref(p), device, ctypes.byref(o)) == 0
+        return p
+
+    def matrix(self, ctx, dim, top=9):
+        symbols = np.arange(65, 65 + dim, dtype=np.uint8)
+        scores = np.where(np.eye(dim), top, -3).astype(np.int32)
+        return self.lib.pa_set_substitution_matrix(ctx, symbols.ctypes.data, dim, scores.ctypes.data)
+
+    def align_device(self, ctx, n, b1, b2, local=True, matrix=False, match=1, mismatch=-4, free=False, width=0):
+        """One device call; nothing reads the (made-up) buffers."""
+        f = int(local or free)
+        cfg = self._lib.PaConfig(int(local) | (self._lib.PA_SCORE_MATRIX if matrix else 0), match, mismatch, -6, -1,
+                                 f, f, f, f, width, 0)
+        at = [ctypes.c_void_p(0x10000 * k) for k in range(1, 6)]
+        return self.lib.pa_align_batch_device(ctx, ctypes.byref(cfg), at[0], at[1], b1, at[2], at[3], b2, n, at[4], None,
+                                              None)
+
+    def events(self):
+        text = self._events().decode()
+        self._reset()
+        return text.splitlines()
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    from pairwise_aligner_gb300 import build
+    objs = build.objects()
+    d = tmp_path_factory.mktemp("host_runtime")
+    lib, group = str(d / "libpa_host.so"), d / "group.cu"
+    group.write_text(f'#include "{build.CSRC}/pa_common.cuh"\n'
+                     'extern "C" int dp_launch_group(const void *p) { return ((const pa::DpLaunch *)p)->G; }\n')
+    nvcc = build.nvcc()
+    subprocess.check_call([nvcc, *build.ARCH, "-std=c++17", "-Xcompiler", "-fPIC", "-diag-suppress", "177", "-shared",
+                           "-cudart", "none", "-Xlinker", "-Bsymbolic", "-o", lib, str(group),
+                           os.path.join(REPO, "tests", "cpp", "host_runtime.cpp"), *objs])
+    return HostRuntime(lib)
+
+
+def test_matrix_kernels_may_use_their_shared_memory_on_every_device(host):
+    """The right to more than 48 KB of shared memory belongs to a device: a context on the second one
+    needs its own, also when the first has asked for the same kernels already."""
+    host.events()
+    for device in (0, 1):
+        ctx = host.context(device)
+        for dim in (20, 32):                            # 40 and 64 KB of profiles
+            assert host.matrix(ctx, dim) == 0
+            for local, free in ((True, False), (False, False), (False, True)):
+                assert host.align_device(ctx, 20000, 20000 * 300, 20000 * 300, local, True, free=free) == 0
+        ev = host.events()
+        assert not [e for e in ev if e.startswith("refused")], ev
+        profile = [e for e in ev if "dp_short" in e and "Li2E" in e]
+        assert profile and all(f"device {device}" in e for e in profile)
+        host.lib.pa_destroy(ctx)
