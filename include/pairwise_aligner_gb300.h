@@ -257,7 +257,9 @@ pa_status pa_get_graph_count(const pa_ctx *ctx, uint32_t *out);
 /* Polls a wait between the passes of a long pair makes after its first look before it gives up
  * (default 2^24, with a short sleep between polls).  A wait that gives up marks its
  * pair PA_RESULT_ERROR and the call returns PA_ERR_TIMEOUT; 0 gives up at the first
- * look (tests use it to exercise that path).  No counterpart in the reference. */
+ * look (tests use it to exercise that path).  A traceback whose waits give up is computed
+ * again without waits, one warp per pair, and returns its results.  No counterpart in the
+ * reference. */
 pa_status pa_set_wait_limit(pa_ctx *ctx, uint32_t polls);
 
 /* Of the long pairs scored by byte comparison or a substitution matrix, those whose sequence2

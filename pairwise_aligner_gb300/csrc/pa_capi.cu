@@ -1868,52 +1868,63 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
     };
     const int grid = traceback_grid(ctx->sm_count);
     uint64_t launches = 0;
-    for (uint64_t first = 0; first < n_pairs;) {
-        uint64_t total = 0, end = first;
-        while (end < n_pairs && total + words[end] <= kTbBudgetWords) {
-            dir_off[end - first] = total;
-            total += words[end];
-            ++end;
-        }
-        if ((s = ensure(ctx, ctx->tb_dir, std::max<uint64_t>(total, 1) * 4))) return s;
-        // the previous chunk's kernel may still read the offsets: copy them in stream order
-        PA_CUDA(ctx, cudaMemcpyAsync(ctx->tb_dir_off.p, dir_off.data(), (end - first) * 8, cudaMemcpyHostToDevice, st));
-        if (tagged) {
-            const uint32_t cnt = (uint32_t)(end - first);
-            uint32_t at[257] = {}, *start = order.data() + cnt, tasks = 0;
-            for (uint64_t k = first; k < end; ++k) ++at[255 - size_bucket(k) + 1];
-            for (int x = 0; x < 256; ++x) at[x + 1] += at[x];
-            for (uint64_t k = first; k < end; ++k) order[at[255 - size_bucket(k)]++] = (uint32_t)(k - first);
-            for (uint32_t u = 0; u < cnt; ++u) {
-                const uint64_t k = first + order[u], n = off2[k + 1] - off2[k];
-                start[u] = tasks;
-                if (off1[k + 1] > off1[k]) tasks += (uint32_t)((n + 2 * kTracebackPassRows - 1) / (2 * kTracebackPassRows));
+    auto run = [&](bool tagged) -> pa_status {
+        for (uint64_t first = 0; first < n_pairs;) {
+            uint64_t total = 0, end = first;
+            while (end < n_pairs && total + words[end] <= kTbBudgetWords) {
+                dir_off[end - first] = total;
+                total += words[end];
+                ++end;
             }
-            start[cnt] = tasks;
-            if ((s = ensure(ctx, ctx->tb_cand, std::max<uint64_t>(tasks, 1) * sizeof(int4)))) return s;
-            PA_CUDA(ctx, cudaMemcpyAsync(ctx->tb_order.p, order.data(), (2ull * cnt + 1) * 4, cudaMemcpyHostToDevice, st));
-            L.start = L.order + cnt;
-            L.cand = (int4 *)ctx->tb_cand.p;
+            if ((s = ensure(ctx, ctx->tb_dir, std::max<uint64_t>(total, 1) * 4))) return s;
+            // the previous chunk's kernel may still read the offsets: copy them in stream order
+            PA_CUDA(ctx, cudaMemcpyAsync(ctx->tb_dir_off.p, dir_off.data(), (end - first) * 8, cudaMemcpyHostToDevice, st));
+            if (tagged) {
+                const uint32_t cnt = (uint32_t)(end - first);
+                uint32_t at[257] = {}, *start = order.data() + cnt, tasks = 0;
+                for (uint64_t k = first; k < end; ++k) ++at[255 - size_bucket(k) + 1];
+                for (int x = 0; x < 256; ++x) at[x + 1] += at[x];
+                for (uint64_t k = first; k < end; ++k) order[at[255 - size_bucket(k)]++] = (uint32_t)(k - first);
+                for (uint32_t u = 0; u < cnt; ++u) {
+                    const uint64_t k = first + order[u], n = off2[k + 1] - off2[k];
+                    start[u] = tasks;
+                    if (off1[k + 1] > off1[k]) tasks += (uint32_t)((n + 2 * kTracebackPassRows - 1) / (2 * kTracebackPassRows));
+                }
+                start[cnt] = tasks;
+                if ((s = ensure(ctx, ctx->tb_cand, std::max<uint64_t>(tasks, 1) * sizeof(int4)))) return s;
+                PA_CUDA(ctx, cudaMemcpyAsync(ctx->tb_order.p, order.data(), (2ull * cnt + 1) * 4, cudaMemcpyHostToDevice, st));
+                L.start = L.order + cnt;
+                L.cand = (int4 *)ctx->tb_cand.p;
+            }
+            PA_CUDA(ctx, cudaStreamSynchronize(st));        // the host arrays are reused by the next chunk
+            L.first = (uint32_t)first;
+            L.count = (uint32_t)(end - first);
+            L.dir_off = (const uint64_t *)ctx->tb_dir_off.p;
+            L.dir = (uint32_t *)ctx->tb_dir.p;
+            if (tagged) traceback_tag_launch(ctx->sm_count, st, L, P);
+            else traceback_launch(grid, st, L, P);
+            launches += tagged ? 3 : 1;
+            first = end;
         }
-        PA_CUDA(ctx, cudaStreamSynchronize(st));        // the host arrays are reused by the next chunk
-        L.first = (uint32_t)first;
-        L.count = (uint32_t)(end - first);
-        L.dir_off = (const uint64_t *)ctx->tb_dir_off.p;
-        L.dir = (uint32_t *)ctx->tb_dir.p;
-        if (tagged) traceback_tag_launch(ctx->sm_count, st, L, P);
-        else traceback_launch(grid, st, L, P);
-        launches += tagged ? 3 : 1;
-        first = end;
-    }
+        PA_CUDA(ctx, cudaGetLastError());
+        PA_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
+        PA_CUDA(ctx, cudaMemcpyAsync(out, ctx->in_out.p, n_pairs * sizeof(pa_result), cudaMemcpyDeviceToHost, st));
+        PA_CUDA(ctx, cudaMemcpyAsync(alignments, ctx->tb_aln.p, n_pairs * sizeof(pa_alignment), cudaMemcpyDeviceToHost, st));
+        if (b1 + b2) PA_CUDA(ctx, cudaMemcpyAsync(ops, ctx->tb_ops.p, b1 + b2, cudaMemcpyDeviceToHost, st));
+        return PA_OK;
+    };
+    if ((s = run(tagged))) return s;
     uint32_t wait_error = 0;
     if (tagged) PA_CUDA(ctx, cudaMemcpyAsync(&wait_error, tb_words, 4, cudaMemcpyDeviceToHost, st));
-    PA_CUDA(ctx, cudaGetLastError());
-    PA_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
-    PA_CUDA(ctx, cudaMemcpyAsync(out, ctx->in_out.p, n_pairs * sizeof(pa_result), cudaMemcpyDeviceToHost, st));
-    PA_CUDA(ctx, cudaMemcpyAsync(alignments, ctx->tb_aln.p, n_pairs * sizeof(pa_alignment), cudaMemcpyDeviceToHost, st));
-    if (b1 + b2) PA_CUDA(ctx, cudaMemcpyAsync(ops, ctx->tb_ops.p, b1 + b2, cudaMemcpyDeviceToHost, st));
     PA_CUDA(ctx, cudaStreamSynchronize(st));
-    if (wait_error) return fail(ctx, PA_ERR_TIMEOUT, "a wait between the passes of a pair ran out");
+    if (wait_error) {
+        // a wait between the passes of a pair ran out, and nothing was walked: once more on one warp
+        // per pair, which waits for nothing
+        if ((s = ensure(ctx, ctx->boundary, (b1 + n_pairs) * sizeof(Cell)))) return s;
+        L.bnd = (Cell *)ctx->boundary.p;
+        if ((s = run(false))) return s;
+        PA_CUDA(ctx, cudaStreamSynchronize(st));
+    }
     if (stats) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);

@@ -19,7 +19,8 @@
 //
 // This kernel (k_traceback) computes a pair's passes and its walk on one warp.  It takes the calls
 // whose scores need more than 26 bits, and local byte comparison with a positive mismatch; all
-// others run on the tagged kernels of pa_traceback_tag.cuh.
+// others run on the tagged kernels of pa_traceback_tag.cuh, and on this one again if a wait between
+// their passes runs out.
 #include <cuda_runtime.h>
 
 #include <algorithm>

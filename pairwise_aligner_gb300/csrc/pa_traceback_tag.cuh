@@ -15,7 +15,7 @@
 // The passes (512 rows, 16 per lane; the last one ra = ceil(rows left / 128) * 4 per lane) of all
 // pairs of a chunk stand in one queue, largest pair first, and hand their bottom rows on through
 // tagged cells as in pa_long.cuh; a pass leaves its end-cell candidate, and k_tb_walk walks the
-// paths when all passes are done.  Words of pass p of a pair start at p * (m + 31) * 64; a step
+// paths when all passes are done.  If a wait ran out it walks none, and the caller runs k_traceback.  Words of pass p of a pair start at p * (m + 31) * 64; a step
 // holds a word per lane (ra <= 8) or two; row k of a lane's first word is its nibble k (of a
 // shorter strip: k + 8 - ra), rows 8.. are in the second (nibble k - 8 + 16 - ra).
 //
@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(kTagThreads) k_tb_walk(TbLaunch L, DpParams P)
     const int lane = threadIdx.x & 31;
     const int fcf = P.first_column_free, frf = P.first_row_free;
     const bool lcf = P.last_column_free, lrf = P.last_row_free;
+    if (__ldcg(L.error)) return;                  // directions are missing: the call computes them again
     for (;;) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(L.queue + 1, 1u);
