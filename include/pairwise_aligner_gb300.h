@@ -329,10 +329,9 @@ pa_status pa_align_batch_banded(pa_ctx *ctx, const pa_config *config,
  * L1 prefetch, 4 as 3 with a two-op vertical-gap chain, 5 / 6 as 3 / 4 with one prefetch
  * per 8 columns, 7 / 8 as 3 / 4 without the score-table prefetch), 9 / 10 the short-pair
  * kernel with 16 / 32 rows of sequence2 per thread (s32 lanes: 16; matrix scores beyond a
- * signed byte take the general kernel's default).  variant_s32 at its default (0 local, 4
- * global) selects the short-pair kernel too; group_threads: lanes per pair group (1..32,
- * power of two; 0: the built-in rule, which picks it from the batch size).  Index 0 =
- * local, 1 = global.
+ * signed byte take form 0 (local) or 4 (global) of the general kernel), the default of
+ * variant_s16 and variant_s32; group_threads: lanes per pair group (1..32, power of two;
+ * 0: the built-in rule, which picks it from the batch size).  Index 0 = local, 1 = global.
  * The s16x2 class also has a table of tuned entries, one per method, batch-size class
  * and pair-size class: size class s = 0..3 when n_pairs < 2^(12 + 2s), else 4; pair-size
  * class h = 0..2 when the mean m*n per pair < 2^(14 + 2h), else 3.  An entry with

@@ -760,10 +760,7 @@ void apply_tuning(pa_ctx *c, const pa_config *cfg, uint64_t n_pairs, uint64_t b1
     const pa_tune_entry &e = c->tuning.s16[mi][tune_size_class(n_pairs)][tune_shape_class(n_pairs, b1, b2)];
     if (!c->fixed_variant) {
         c->variant[K_S16] = e.group_threads ? e.variant : c->tuning.variant_s16[mi];
-        // the other classes: the short-pair kernel, unless a form of dp_kernel other than the
-        // default (0 local, 4 global) was set
-        const int v32 = c->tuning.variant_s32[mi];
-        c->variant[K_S32] = c->variant[K_GEN] = v32 == (mi == 0 ? 0 : 4) ? kDefaultShortVariant : v32;
+        c->variant[K_S32] = c->variant[K_GEN] = c->tuning.variant_s32[mi];
     }
     if (!c->fixed_G) {
         int g16 = e.group_threads ? e.group_threads : c->tuning.group_threads_s16[mi];
@@ -1384,12 +1381,9 @@ pa_status pa_create(pa_ctx **out, int device_ordinal, const pa_options *options)
         pa_destroy(c);
         return PA_ERR_CUDA;
     }
-    // defaults measured on GB300 (262,144 pairs of 64..512 bp): local s16x2 is fastest with
-    // variant 7, global with variant 4; 8 lanes per group
+    // the short-pair kernel for every class; group sizes 0: the built-in rule
     c->tuning = pa_tuning{};
-    c->tuning.variant_s16[0] = c->tuning.variant_s16[1] = kDefaultShortVariant;
-    c->tuning.variant_s32[0] = 0;
-    c->tuning.variant_s32[1] = 4;                 // group sizes 0: the built-in rule
+    for (int m = 0; m < 2; ++m) c->tuning.variant_s16[m] = c->tuning.variant_s32[m] = kDefaultShortVariant;
     if (c->opt.group_threads) {
         int g = c->opt.group_threads;
         if (g < 1 || g > 32 || (g & (g - 1))) { pa_destroy(c); return PA_ERR_INVALID_ARGUMENT; }

@@ -83,3 +83,23 @@ def test_matrix_kernels_may_use_their_shared_memory_on_every_device(host):
         profile = [e for e in ev if "dp_short" in e and "Li2E" in e]
         assert profile and all(f"device {device}" in e for e in profile)
         host.lib.pa_destroy(ctx)
+
+
+@pytest.mark.parametrize("local", [True, False])
+def test_every_s32_variant_names_its_kernel(host, local):
+    """pa_tuning::variant_s32 selects the inner loop of the s32 and byte-compare classes: 0..8 a form of
+    the general kernel, whatever the default is; the default itself is the short-pair kernel."""
+    mi, t = int(not local), host._lib.PaTuning()
+    ctx = host.context(use_graphs=-1)
+    assert host.lib.pa_get_tuning(ctx, ctypes.byref(t)) == 0
+    for v in (None, 0, 4, 7, 9):
+        if v is not None:
+            t.variant_s32[mi] = v
+            assert host.lib.pa_set_tuning(ctx, ctypes.byref(t)) == 0
+        host.events()
+        assert host.align_device(ctx, 5000, 5000 * 200, 5000 * 200, local) == 0
+        s32 = [e for e in host.events() if re.search(r"dp_(short|kernel)I.*3L32", e)]
+        assert len(s32) >= 2
+        kind = "dp_kernel" if v is not None and v < 9 else "dp_short"
+        assert all(kind in e for e in s32), (v, s32)
+    host.lib.pa_destroy(ctx)
