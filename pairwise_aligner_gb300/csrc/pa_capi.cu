@@ -223,19 +223,24 @@ pa_status check_config(pa_ctx *c, const pa_config *cfg, DpParams &P, ClassCfg &C
     C.s16_params = (int64_t)cfg->gap_open + cfg->gap_extension >= -1000 && cfg->gap_extension >= -1000;
     C.force32 = cfg->width_hint == 32;
     C.local = local;
+    C.long_cells = c->long_cells;
+    C.huge_cells = c->huge_cells;
+    C.huge_min_n = c->huge_min_n;
+    C.team_max_n = c->team_max_n;
+    C.qtab_s16 = C.qtab_s32 = 1;
+    return PA_OK;
+}
+
+// What the classifier takes from the call's group sizes and ring.
+void set_classes(const pa_ctx *c, ClassCfg &C)
+{
     for (int k = 0; k < kClasses; ++k) {
         const bool cta = k >= (int)kLongOffset;
         C.gcnt[k] = cta ? 32 : c->G[k < 3 ? k : 0];
         C.rpt[k] = kR;
         C.rows[k] = C.gcnt[k] * kR;
     }
-    C.long_cells = c->long_cells;
-    C.huge_cells = c->huge_cells;
-    C.huge_min_n = c->huge_min_n;
-    C.team_max_n = c->team_max_n;
     C.long_max_m = c->use_long && c->ring.p ? c->ring_m : 0;
-    C.qtab_s16 = C.qtab_s32 = 1;
-    return PA_OK;
 }
 
 }  // namespace
@@ -406,6 +411,11 @@ void warm_occupancy()
     }
 }
 
+int dp_mode(const DpParams &P)
+{
+    return P.local ? M_LOCAL : ((P.last_column_free || P.last_row_free) ? M_GLOBAL_FREE : M_GLOBAL);
+}
+
 // Whether the short-pair kernel takes a class under these scores: the plain modes, except scores
 // of a matrix that do not fit a signed byte, and local byte comparison with a positive mismatch
 // (its padding rows would score); the default form of dp_kernel takes those.
@@ -548,7 +558,7 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
     uint32_t *counters = (uint32_t *)c->counters.p;
     pa_status ps = enqueue_prep(c, P, C, s1, o1, b1, s2, o2, b2, out, n_pairs);
     if (ps) return ps;
-    const int mode = P.local ? M_LOCAL : ((P.last_column_free || P.last_row_free) ? M_GLOBAL_FREE : M_GLOBAL);
+    const int mode = dp_mode(P);
     DpLaunch L;
     std::memset(&L, 0, sizeof(L));
     L.seq1 = s1; L.off1 = o1; L.seq2 = s2; L.off2 = o2;
@@ -736,8 +746,8 @@ int tune_shape_class(uint64_t n_pairs, uint64_t b1, uint64_t b2)
     return PA_TUNE_SHAPES - 1;
 }
 
-// The built-in group size: the smallest group (fewest fill and drain steps per pass, most rows per
-// column step) that still gives every resident warp about three work units, so that the largest
+// The built-in group size of the short-pair kernel: the smallest group (fewest fill and drain steps
+// per pass, most rows per column step) that still gives every resident warp about three work units, so that the largest
 // pairs do not outlast the rest, and that holds a pair of mean length in two passes.  A warp unit
 // holds 32 / G groups of `lanes` pairs, a pass G * rows rows.  Measured (GB300, us per call on 8 /
 // 16 / 32 lanes): 65,537 reads of 175 rows 1,119 / 1,156 / 1,514; 16,384 pairs of 64-1,000 rows
@@ -753,9 +763,22 @@ int rule_group_threads(const pa_ctx *c, uint64_t n_pairs, uint64_t b2, int lanes
     return 32;
 }
 
-void apply_tuning(pa_ctx *c, const pa_config *cfg, uint64_t n_pairs, uint64_t b1, uint64_t b2)
+// ... and of the general kernel, which runs explicit variants 0..8, matrix scores beyond a signed byte
+// and short pairs with caller-given bands: about eight units per resident warp, whatever the lengths.
+// With the short-pair kernel's rule 60,000 free-end pairs of 64-512 rows took 6,906 us on variant 4
+// (4,291 with this one), 60,000 with given bands 4,813 (2,590), 20,000 under a matrix of large scores
+// 6,104 (4,668).
+int rule_group_threads_general(const pa_ctx *c, uint64_t n_pairs, int lanes)
 {
-    if (!cfg) return;
+    const double warps = (double)c->sm_count * (2 * kBlock / 32);
+    for (int g = 4; g < 32; g *= 2)
+        if ((double)n_pairs * g / (32.0 * lanes) >= 8.0 * warps) return g;
+    return 32;
+}
+
+void apply_tuning(pa_ctx *c, const pa_config *cfg, const DpParams &P, uint64_t n_pairs, uint64_t b1, uint64_t b2,
+                  bool given_bands)
+{
     const int mi = (cfg->method & ~PA_SCORE_MATRIX) == PA_METHOD_LOCAL ? 0 : 1;
     const pa_tune_entry &e = c->tuning.s16[mi][tune_size_class(n_pairs)][tune_shape_class(n_pairs, b1, b2)];
     if (!c->fixed_variant) {
@@ -765,8 +788,15 @@ void apply_tuning(pa_ctx *c, const pa_config *cfg, uint64_t n_pairs, uint64_t b1
     if (!c->fixed_G) {
         int g16 = e.group_threads ? e.group_threads : c->tuning.group_threads_s16[mi];
         int g32 = c->tuning.group_threads_s32[mi];
-        c->G[K_S16] = g16 ? g16 : rule_group_threads(c, n_pairs, b2, 2, 32);
-        c->G[K_S32] = c->G[K_GEN] = g32 ? g32 : rule_group_threads(c, n_pairs, b2, 1, kR);
+        // dp_kernel runs the banded DP of the DNA classes, and what launch_class does not give dp_short
+        auto rule = [&](Klass k, bool short_kernel, int lanes, int rows) {
+            return short_kernel && c->variant[k] >= kShortVariant ? rule_group_threads(c, n_pairs, b2, lanes, rows)
+                                                                  : rule_group_threads_general(c, n_pairs, lanes);
+        };
+        const bool gen_short = short_fits(dp_mode(P), true, (cfg->method & PA_SCORE_MATRIX) != 0, P);
+        c->G[K_S16] = g16 ? g16 : rule(K_S16, !given_bands, 2, 32);
+        c->G[K_S32] = g32 ? g32 : rule(K_S32, !given_bands, 1, kR);
+        c->G[K_GEN] = g32 ? g32 : rule(K_GEN, gen_short, 1, kR);
         // untuned short-pair kernel: 32 rows per thread
         if (!e.group_threads && !g16 && !c->fixed_variant && c->tuning.variant_s16[mi] >= kShortVariant)
             c->variant[K_S16] = kShortVariant + 1;
@@ -816,12 +846,13 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
                    const uint8_t *s2, const uint64_t *o2, uint64_t b2, uint64_t n_pairs, pa_result *out,
                    const int32_t *h_bands, pa_stats *stats, bool sync_at_end)
 {
-    apply_tuning(c, cfg, n_pairs, b1, b2);
-    pa_status s = n_pairs ? ensure_ring(c, c->want_ring_m) : PA_OK;
-    if (s) return s;
     DpParams P;
     ClassCfg C;
-    if ((s = check_config(c, cfg, P, C))) return s;
+    pa_status s = check_config(c, cfg, P, C);
+    if (s) return s;
+    apply_tuning(c, cfg, P, n_pairs, b1, b2, h_bands != nullptr);
+    if (n_pairs && (s = ensure_ring(c, c->want_ring_m))) return s;
+    set_classes(c, C);
     C.team_max_n = 0;                                 // band mode has its own team choice
     if (P.local || P.first_column_free || P.first_row_free || P.last_column_free || P.last_row_free)
         return fail(c, PA_ERR_UNSUPPORTED, "band mode needs global alignment with penalised end gaps");
@@ -1208,13 +1239,13 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
 {
     if (cfg && cfg->band_mode)
         return run_band(c, cfg, s1, o1, b1, s2, o2, b2, n_pairs, out, nullptr, stats, sync_for_stats || stats);
-    apply_tuning(c, cfg, n_pairs, b1, b2);
-    pa_status s = n_pairs ? ensure_ring(c, c->want_ring_m) : PA_OK;
-    if (s) return s;
     DpParams P;
     ClassCfg C;
-    s = check_config(c, cfg, P, C);
+    pa_status s = check_config(c, cfg, P, C);
     if (s) return s;
+    apply_tuning(c, cfg, P, n_pairs, b1, b2, false);
+    if (n_pairs && (s = ensure_ring(c, c->want_ring_m))) return s;
+    set_classes(c, C);
     // the short-pair kernel (launch_class) builds its own column tables: a class needs none when
     // neither it nor, for global s16x2 pairs, their s32 redo runs on dp_kernel
     auto on_short = [&](Klass k) { return c->variant[k] >= kShortVariant && dp_short_supports(c->G[k]); };

@@ -103,3 +103,25 @@ def test_every_s32_variant_names_its_kernel(host, local):
         kind = "dp_kernel" if v is not None and v < 9 else "dp_short"
         assert all(kind in e for e in s32), (v, s32)
     host.lib.pa_destroy(ctx)
+
+
+def test_group_size_of_the_general_kernel(host):
+    """Its rule is its own: about eight units per resident warp (2,432 of them here), lane by lane; the
+    short-pair kernel takes smaller groups for the same batches."""
+    def groups(ctx, n, **kw):
+        host.events()
+        assert host.align_device(ctx, n, n * 288, n * 288, **kw) == 0
+        got = {}
+        for e in host.events():
+            k = re.search(r"dp_(short|kernel)I.*(L16|L32)", e)
+            if k:
+                got.setdefault((k[1], k[2]), set()).add(int(e.split(" G ")[1]))
+        return got
+    general = host.context(use_graphs=-1, kernel_variant=4)
+    assert groups(general, 60000, local=False, free=True) == {("kernel", "L16"): {32}, ("kernel", "L32"): {16}}
+    matrix = host.context(use_graphs=-1)
+    assert host.matrix(matrix, 20, top=400) == 0
+    assert groups(matrix, 20000, matrix=True)[("kernel", "L32")] == {32}
+    assert groups(matrix, 60000)[("short", "L16")] == {8}
+    host.lib.pa_destroy(general)
+    host.lib.pa_destroy(matrix)
