@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -88,9 +89,10 @@ struct pa_ctx {
     // device work buffers (grow only)
     DevBuf keys, order, hist, starts, cursor, sums, ranges, counts, qtab, boundary, rerun, counters;
     DevBuf slots;                 // short-pair kernel: 16-byte column slots, (seq1_bytes + n_pairs)
-    // long pairs (dp_long): queue words and launch counter, boundary cells, and per queue (s16x2,
-    // s32, redo in s32) the units' first tickets, finished passes, failed waits and records
-    DevBuf long_words, long_cells16, long_tasks, long_start[3], long_done[3], long_fail[3], long_rec[3];
+    // long pairs (dp_long): queue words and launch counter, and per queue (s16x2, s32, redo in s32)
+    // the units' first tickets, finished passes, failed waits and records; their boundary cells are
+    // the pairs' slots
+    DevBuf long_words, long_tasks, long_start[3], long_done[3], long_fail[3], long_rec[3];
     bool use_long = false;        // this call's batch may hold long pairs
     DevBuf ring, rerun_long;      // CTA mode: boundary rows per block; s16 long pairs to redo in s32
     int32_t ring_m = 0;           // longest sequence1 the ring rows hold (0: no CTA mode yet)
@@ -453,26 +455,33 @@ void launch_class(pa_ctx *c, int slot, int mode, bool lanes16, bool gen, const D
     c->last_launches++;
 }
 
-// The boundary cells of row passes (16 bytes per streamed column) and the launch counter of their
-// tags; new cells are zeroed, so that none carries a tag that a launch did not write.
-pa_status ensure_cells(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
+// The words of the pass queues and the launch counter of their tags.
+pa_status ensure_queue_words(pa_ctx *c)
 {
-    pa_status s;
-    const size_t words = c->long_words.cap, cells = c->long_cells16.cap;
-    if ((s = ensure(c, c->long_words, 3 * sizeof(LongWords) + 8))) return s;
-    if (c->long_words.cap != words) PA_CUDA(c, cudaMemsetAsync(c->long_words.p, 0, c->long_words.cap, c->stream));
-    if ((s = ensure(c, c->long_cells16, (b1 + n_pairs) * 16))) return s;
-    if (c->long_cells16.cap != cells) PA_CUDA(c, cudaMemsetAsync(c->long_cells16.p, 0, c->long_cells16.cap, c->stream));
+    if (c->long_words.p) return PA_OK;
+    pa_status s = ensure(c, c->long_words, 3 * sizeof(LongWords) + 8);
+    if (s) return s;
+    PA_CUDA(c, cudaMemsetAsync(c->long_words.p, 0, c->long_words.cap, c->stream));
     return PA_OK;
 }
 
-// Buffers of the long-pair kernel for a batch.
-pa_status ensure_long(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
+// At most so many pairs of a batch are long: their m sum to at most b1 and their n to b2, so if L of
+// them have m * n >= long_cells, L * sqrt(long_cells) <= sqrt(b1 * b2).
+uint64_t most_long(const pa_ctx *c, uint64_t n_pairs, uint64_t b1, uint64_t b2)
 {
-    pa_status s = ensure_cells(c, n_pairs, b1);
+    const double most = std::sqrt((double)b1 * (double)b2 / (double)c->long_cells) + 2.0;
+    return most < (double)n_pairs ? (uint64_t)most : n_pairs;
+}
+
+// Buffers of the long-pair kernel for a batch of at most `pairs` long pairs.  The boundary cells are
+// the pairs' column slots: a pair is short or long, never both, and k_classify clears the slots of
+// the long ones.
+pa_status ensure_long(pa_ctx *c, uint64_t pairs)
+{
+    pa_status s = ensure_queue_words(c);
     if (s) return s;
     for (int k = 0; k < 3; ++k) {
-        const uint64_t units = k == 0 ? (n_pairs + 1) / 2 : n_pairs;
+        const uint64_t units = k == 0 ? (pairs + 1) / 2 : pairs;
         if ((s = ensure(c, c->long_start[k], (units + 1) * 4))) return s;
         if ((s = ensure(c, c->long_done[k], units * 4))) return s;
         if ((s = ensure(c, c->long_fail[k], units * 4))) return s;
@@ -490,7 +499,7 @@ LongQueue long_queue(pa_ctx *c, int k)
     q.done = (uint32_t *)c->long_done[k].p;
     q.fail = (uint32_t *)c->long_fail[k].p;
     q.rec = (LongRecord *)c->long_rec[k].p;
-    q.cells = (ulonglong2 *)c->long_cells16.p;
+    q.cells = (ulonglong2 *)c->slots.p;
     return q;
 }
 
@@ -523,8 +532,8 @@ pa_status enqueue_prep(pa_ctx *c, const DpParams &P, const ClassCfg &C, const ui
     int cls_blocks = (int)std::min<uint64_t>((n_pairs * 32 + 127) / 128, (uint64_t)c->sm_count * 16);
     if (cls_blocks < 1) cls_blocks = 1;
     k_classify<<<cls_blocks, 128, 0, st>>>(s1, o1, b1, s2, o2, b2, n_pairs, P, C, (uint32_t *)c->keys.p,
-                                              small ? nullptr : (uint32_t *)c->hist.p, (uint32_t *)c->qtab.p, out,
-                                              pstats(c));
+                                              small ? nullptr : (uint32_t *)c->hist.p, (uint32_t *)c->qtab.p,
+                                              (uint4 *)c->slots.p, out, pstats(c));
     if (small) {
         k_sort_small<<<1, 1024, 0, st>>>((const uint32_t *)c->keys.p, (uint32_t)n_pairs, (uint32_t *)c->order.p,
                                          (uint32_t *)c->ranges.p, (uint32_t *)c->counts.p, pstats(c), out);
@@ -863,8 +872,9 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     if (!s1 || !o1 || !s2 || !o2 || !out) return fail(c, PA_ERR_INVALID_ARGUMENT, "null buffer");
     if (n_pairs >= (1ull << 31)) return fail(c, PA_ERR_TOO_LARGE, "n_pairs must be < 2^31");
     if ((s = prepare_buffers(c, n_pairs, b1))) return s;
-    if (c->use_long && ((s = ensure_long(c, n_pairs, b1)) ||
-                        (s = ensure(c, c->long_tasks, (b2 / (32 * kR) + n_pairs + 1) * sizeof(uint2)))))
+    const uint64_t longs = most_long(c, n_pairs, b1, b2);
+    if (c->use_long && ((s = ensure_long(c, longs)) ||
+                        (s = ensure(c, c->long_tasks, (b2 / (32 * kR) + longs + 1) * sizeof(uint2)))))
         return s;
     C.pass_queue = c->use_long;
     const uint64_t np = n_pairs;
@@ -1258,7 +1268,7 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
     if (!s1 || !o1 || !s2 || !o2 || !out) return fail(c, PA_ERR_INVALID_ARGUMENT, "null buffer");
     if (n_pairs >= (1ull << 31)) return fail(c, PA_ERR_TOO_LARGE, "n_pairs must be < 2^31");
     if ((s = prepare_buffers(c, n_pairs, b1))) return s;
-    if (c->use_long && (s = ensure_long(c, n_pairs, b1))) return s;
+    if (c->use_long && (s = ensure_long(c, most_long(c, n_pairs, b1, b2)))) return s;
     C.pass_queue = c->use_long;
     c->last_launches = 0;
     const bool use_graph = c->opt.use_graphs >= 0;
@@ -1443,7 +1453,7 @@ pa_status pa_destroy(pa_ctx *c)
                       &c->in_seq1, &c->in_off1, &c->in_seq2, &c->in_off2, &c->in_out, &c->in_small,
                       &c->band_spec, &c->band_win, &c->band_code, &c->band_bsum, &c->band_ctr, &c->band_in,
                       &c->mlp_feat, &c->mlp_x, &c->mlp_h1, &c->mlp_h2, &c->mlp_out,
-                      &c->ring, &c->rerun_long, &c->long_words, &c->long_cells16, &c->long_tasks, &c->long_start[0], &c->long_start[1],
+                      &c->ring, &c->rerun_long, &c->long_words, &c->long_tasks, &c->long_start[0], &c->long_start[1],
                       &c->long_start[2], &c->long_done[0], &c->long_done[1], &c->long_done[2], &c->long_fail[0],
                       &c->long_fail[1], &c->long_fail[2], &c->long_rec[0], &c->long_rec[1], &c->long_rec[2], &c->mat_rank, &c->mat_scores,
                       &c->io_ctr, &c->in_words1, &c->in_words2,
@@ -1837,15 +1847,26 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
     if ((s = ensure(ctx, ctx->in_seq1, b1)) || (s = ensure(ctx, ctx->in_seq2, b2)) ||
         (s = ensure(ctx, ctx->in_off1, (n_pairs + 1) * 8)) || (s = ensure(ctx, ctx->in_off2, (n_pairs + 1) * 8)) ||
         (s = ensure(ctx, ctx->in_out, n_pairs * sizeof(pa_result))) ||
-        (s = tagged ? ensure_cells(ctx, n_pairs, b1) : ensure(ctx, ctx->boundary, (b1 + n_pairs) * sizeof(Cell))) ||
+        (s = ensure_queue_words(ctx)) ||
         (s = ensure(ctx, ctx->tb_order, (2 * n_pairs + 1) * 4)) ||
         (s = ensure(ctx, ctx->tb_aln, n_pairs * sizeof(pa_alignment))) || (s = ensure(ctx, ctx->tb_ops, b1 + b2)) ||
         (s = ensure(ctx, ctx->tb_dir_off, n_pairs * 8)))
         return s;
+    uint64_t chunk = 0, most = 1;                      // direction words of the largest chunk
+    for (uint64_t k = 0; k < n_pairs; ++k) {
+        chunk = chunk + words[k] <= kTbBudgetWords ? chunk + words[k] : words[k];
+        most = std::max(most, chunk);
+    }
+    if ((s = ensure(ctx, ctx->tb_dir, most * 4))) return s;
+    // the tagged kernels' boundary cells take twice the memory of k_traceback's: without room for them
+    // the call runs on that one
+    if (tagged && ensure(ctx, ctx->slots, (b1 + n_pairs) * sizeof(Slot))) tagged = false;
+    if (!tagged && (s = ensure(ctx, ctx->boundary, (b1 + n_pairs) * sizeof(Cell)))) return s;
     std::vector<uint64_t> r1(off1, off1 + n_pairs + 1), r2(off2, off2 + n_pairs + 1);
     for (auto &v : r1) v -= base1;
     for (auto &v : r2) v -= base2;
     cudaStream_t st = ctx->stream;
+    if (tagged) PA_CUDA(ctx, cudaMemsetAsync(ctx->slots.p, 0, (b1 + n_pairs) * sizeof(Slot), st));
     PA_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
     if (b1) PA_CUDA(ctx, cudaMemcpyAsync(ctx->in_seq1.p, seq1 + base1, b1, cudaMemcpyHostToDevice, st));
     if (b2) PA_CUDA(ctx, cudaMemcpyAsync(ctx->in_seq2.p, seq2 + base2, b2, cudaMemcpyHostToDevice, st));
@@ -1880,7 +1901,7 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
         L.error = tb_words;
         L.my_epoch = (unsigned long long *)(tb_words + 4);
         L.epoch = long_epoch(ctx);
-        L.cells = (ulonglong2 *)ctx->long_cells16.p;
+        L.cells = (ulonglong2 *)ctx->slots.p;
         L.spin_limit = ctx->wait_limit;
         L.tables = std::abs((int64_t)P.match) <= 63 && std::abs((int64_t)P.mismatch) <= 63;
         L.order = (const uint32_t *)ctx->tb_order.p;
@@ -1901,7 +1922,6 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
                 total += words[end];
                 ++end;
             }
-            if ((s = ensure(ctx, ctx->tb_dir, std::max<uint64_t>(total, 1) * 4))) return s;
             // the previous chunk's kernel may still read the offsets: copy them in stream order
             PA_CUDA(ctx, cudaMemcpyAsync(ctx->tb_dir_off.p, dir_off.data(), (end - first) * 8, cudaMemcpyHostToDevice, st));
             if (tagged) {

@@ -55,7 +55,7 @@ struct LongQueue {
     uint32_t *done;                // passes finished per unit
     uint32_t *fail;                // per unit: a wait ran out
     LongRecord *rec;
-    ulonglong2 *cells;             // (seq1_bytes + n_pairs) boundary cells, pair k's at off1[k] + k
+    ulonglong2 *cells;             // (seq1_bytes + n_pairs) boundary cells, pair k's at off1[k] + k (DpLaunch::slots)
 };
 
 // Long pairs with unitary DNA scores (pa_long.cuh): the row passes of all units in one queue.

@@ -13,7 +13,9 @@
 // The boundary row.  Pass p - 1 hands its bottom row to pass p through one 16-byte cell per
 // column, {H, vertical gap, tag}, written and read with single 128-bit relaxed accesses at
 // GPU scope.  The tag names the launch and the pass, so a reader that finds it has the whole
-// cell: no flag, no fence, no order between cells is needed.  The row is reused in place:
+// cell: no flag, no fence, no order between cells is needed.  The cells are the pair's column slots
+// of the short-pair kernel, cleared by k_classify (a memory of their own would add 16 bytes per base
+// of sequence1 to every call that may hold a long pair).  The row is reused in place:
 // pass p overwrites column i only after its own first thread read column i.  The reader
 // fetches blocks of kStage columns, one block ahead (lane t the block's column t), and hands
 // them to thread 0 through shared memory with the score tables; a cell that is not there yet

@@ -125,3 +125,40 @@ def test_group_size_of_the_general_kernel(host):
     assert groups(matrix, 60000)[("short", "L16")] == {8}
     host.lib.pa_destroy(general)
     host.lib.pa_destroy(matrix)
+
+
+def test_scratch_of_a_batch_without_room_for_long_pairs(host):
+    """What a device call of short pairs may take: per byte of sequence1 and pair 28 bytes (score tables,
+    boundary cells, slots), 16 per pair for the lists, the ring rows of 3.83 GB for long byte-compare
+    pairs and the buckets of the sort.  Long pairs share the slots."""
+    n, b = 1_000_000, 250_000_000
+    for call in (dict(local=True), dict(local=False), dict(local=True, width=32)):
+        host._reset()
+        ctx = host.context()
+        host._limit(28 * (b + n) + 16 * n + 3 * 304 * 8 * (65536 + 2) * 8 + 16 * 10**6 + 132 * b // 1024)
+        assert host.align_device(ctx, n, b, b, **call) == 0
+        host._limit(2**63)
+        host.lib.pa_destroy(ctx)
+
+
+def test_traceback_without_room_for_tagged_cells(host):
+    """The tagged kernels need 16 bytes per column, the kernel with one warp per pair 8: a call that fits
+    only with 8 runs on the latter."""
+    n, m, k = 4000, 2500, 30
+    s1, s2 = np.full(n * m, 65, np.uint8), np.full(n * k, 65, np.uint8)
+    o1, o2 = np.arange(n + 1, dtype=np.uint64) * m, np.arange(n + 1, dtype=np.uint64) * k
+    cfg = host._lib.PaConfig(0, 2, -3, -5, -1, 0, 0, 0, 0, 0, 0)
+    out, aln, ops = np.zeros(n * 16, np.uint8), np.zeros(n * 16, np.uint8), np.zeros(n * (m + k), np.uint8)
+    seen = []
+    for cell in (16, 8):
+        ctx = host.context()
+        host.events()
+        words = 4 * n * (m + 31) * 32                   # one pass of 256 rows
+        host._limit(words + n * (m * 2 + k * 2 + 80) + cell * n * (m + 1) + 2 * 10**6)
+        rc = host.lib.pa_traceback_batch(ctx, ctypes.byref(cfg), s1.ctypes.data, o1.ctypes.data, s2.ctypes.data,
+                                         o2.ctypes.data, n, out.ctypes.data, aln.ctypes.data, ops.ctypes.data, None)
+        host._limit(2**63)
+        assert rc == 0, cell
+        seen.append([re.search(r"k_t\w+", e)[0] for e in host.events() if "k_t" in e])
+        host.lib.pa_destroy(ctx)
+    assert all("k_tb" in x for x in seen[0]) and all("k_traceback" in x for x in seen[1]), seen
