@@ -168,19 +168,27 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
     };
     fetch(1);
     uint32_t best = V::splat(KC::Kt);
-    // global modes: whether a lane's last row is this thread's, and the first column a lane ends at
-    auto own_row = [&](int l) -> int32_t {        // its index in the strip, or -1
-        const int32_t r = (u.n[l] - 1) - j0;
-        return r >= 0 && r < RA && (u.n[l] - 1) / rows_full == p ? r : -1;
-    };
+    // global modes: a lane's last row as an index into the strip (-1: not this thread's), and the first
+    // column a lane ends at
+    int32_t own[NL];
     bool any_own = false;
     int32_t mmin = u.ms;
-    if (MODE != M_LOCAL) {
 #pragma unroll
-        for (int l = 0; l < NL; ++l) {
-            any_own |= own_row(l) >= 0;
-            mmin = min(mmin, u.m[l]);
-        }
+    for (int l = 0; l < NL; ++l) {
+        const int32_t r = (u.n[l] - 1) - j0;
+        own[l] = MODE != M_LOCAL && r >= 0 && r < RA && (u.n[l] - 1) / rows_full == p ? r : -1;
+        any_own |= own[l] >= 0;
+        mmin = min(mmin, u.m[l]);
+    }
+    // the end rule of the last row (strip_end_track; with a comparison in shared memory on every column
+    // a free-end pair of 200,000 x 100 took 132.6 ms, now 86.6)
+    const bool row_end = MODE == M_GLOBAL_FREE && P.last_column_free && any_own;
+    uint32_t seen = V::splat(KC::below);
+    const uint32_t shift_neg = V::splat(-P.shift);
+    const int32_t r0 = max(own[0], 0), r1 = max(own[NL - 1], 0);
+    if (row_end) {
+#pragma unroll
+        for (int l = 0; l < NL; ++l) sh.bi[l][threadIdx.x] = 0;
     }
 
     auto step = [&](int32_t s, bool active) {
@@ -210,8 +218,10 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
             if (writer) store_cell128(u.row + i, (uint64_t)sH | ((uint64_t)sE << 32), u.tag);
             if (MODE == M_LOCAL)
                 strip_track<V, R, RA>(H, best, i, snap, sh);
-            else if ((MODE == M_GLOBAL_FREE && P.last_column_free && any_own) || i >= mmin)
-                strip_ends<V, MODE, RA>(P, u, H, i, j0, any_own, snap, sh, own_row);
+            else {
+                if (row_end) strip_end_track<V, MODE, RA, kBlock>(u, H, seen, shift_neg, i, r0, r1, snap, sh);
+                if (i >= mmin) strip_ends<V, MODE, RA>(P, u, H, i, j0, any_own, snap, sh, [&](int l) { return own[l]; });
+            }
         }
     };
     // fill: thread t starts at step t; steady: every thread active; drain
@@ -227,6 +237,7 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
         step(s, i >= 1 && i <= ms);
     }
     if (MODE == M_LOCAL) strip_track_end<V, R, RA>(best, j0, snap, sh);
+    if (row_end) strip_end_offer<V, MODE, kBlock>(P, u, own, sh);
     if (BAND) {
         // upper bounds on the paths that leave the window (exit_bound): first through its right
         // edge, cells (iend + 1, j), by a horizontal gap from (iend, j) or diagonally from
@@ -422,7 +433,7 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
     __shared__ LongUnit s_unit[NW];
     __shared__ uint4 s_stage[NW][2 * kStage];
     __shared__ int32_t s_cand[NL][3][kBlock];
-    __shared__ int32_t s_bi[MODE == M_LOCAL ? NL : 1][kBlock];
+    __shared__ int32_t s_bi[MODE == M_LOCAL ? NL : MODE == M_GLOBAL_FREE ? 2 * NL : 1][kBlock];
     uint4 *snap = snap_store + threadIdx.x;
     StripShared<V> sh{s_cand, s_bi};
     const int t = threadIdx.x & 31;

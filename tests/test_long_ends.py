@@ -1,0 +1,46 @@
+"""End rules of the pass queue: last rows at every edge of strips and passes, on either lane of a unit,
+ties along the last row and column, values at the s16 clamp, in both lane types."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ACGT = np.frombuffer(b"ACGT", np.uint8)
+NS = [1, 3, 4, 5, 127, 128, 129, 130, 255, 257, 383, 385, 511, 513, 640, 767, 768, 769, 1025]
+FREE = ["first_column_free", "first_row_free", "last_column_free", "last_row_free"]
+
+
+@pytest.mark.parametrize("ends", ["last_column_free", "last_row_free", "first_column_free,last_column_free",
+                                  "first_row_free,last_row_free", "last_column_free,last_row_free",
+                                  "first_column_free,first_row_free,last_column_free,last_row_free"])
+@pytest.mark.parametrize("scores", [(2, -3, -5, -1), (1, 0, -1, 0), (3, -20, -40, -12)])
+@pytest.mark.parametrize("width", [0, 32])
+def test_end_rules_equal_oracle(built_lib, oracle, ends, scores, width):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import pairwise_aligner_gb300 as pa
+    rng = np.random.default_rng(11)
+    s1, s2 = [], []
+    for k, n in enumerate(NS * 3):
+        m = [int(rng.integers(1, 60)), n, int(rng.integers(300, 900))][k % 3]
+        b = ACGT[rng.integers(0, 4, n)]
+        a = np.resize(b, m) if k % 2 else ACGT[rng.integers(0, 4, m)]
+        a = np.where(rng.random(m) < 0.9, a, ACGT[rng.integers(0, 4, m)]).astype(np.uint8)
+        if k % 5 == 0:
+            a[:] = b[:] = ord("A")                       # ties everywhere
+        s1.append(bytes(a))
+        s2.append(bytes(b))
+    match, mismatch, go, ge = scores
+    free = {k: k in ends.split(",") for k in FREE}
+    c = dict(local=False, match=match, mismatch=mismatch, gap_open=go, gap_extension=ge, width_hint=width, **free)
+    q, qo = pa.pack(s1)
+    t, to = pa.pack(s2)
+    ctx = pa.Context(0)
+    ctx.set_cta_threshold(1)                             # every pair on the queue
+    res = pa.Aligner(c, context=ctx).compute_arrays(q, qo, t, to)
+    sc, e1, e2 = oracle.align_batch(oracle.make_cfg(match, mismatch, go, ge, **free), q, qo, t, to)
+    bad = np.flatnonzero((res["score"] != sc) | (res["end1"] != e1) | (res["end2"] != e2))
+    assert len(bad) == 0, (len(bad), [(len(s1[k]), len(s2[k])) for k in bad[:5]], res[bad[:5]],
+                           list(zip(sc[bad[:5]], e1[bad[:5]], e2[bad[:5]])))
+    ctx.close()
