@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(1024) k_long_plan(LongPlan a, LongPlan b, cons
         uint32_t total, v = 0;
         if (u < units) {
             const uint2 s = long_shape(p, off1, off2, count, units, u);
-            const uint32_t rows = 32u * (uint32_t)long_rows(budget, floor_rows, (int32_t)s.x);
+            const uint32_t rows = 32u * (uint32_t)long_rows(budget, floor_rows, (int32_t)s.x, (int32_t)s.y);
             v = (s.y + rows - 1) / rows;
         }
         const uint32_t ex = block_exclusive_scan(v, sh, total);

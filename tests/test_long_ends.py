@@ -44,3 +44,33 @@ def test_end_rules_equal_oracle(built_lib, oracle, ends, scores, width):
     assert len(bad) == 0, (len(bad), [(len(s1[k]), len(s2[k])) for k in bad[:5]], res[bad[:5]],
                            list(zip(sc[bad[:5]], e1[bad[:5]], e2[bad[:5]])))
     ctx.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 70000), (17, 30000), (100, 3000), (300, 6500), (700, 2900)])
+@pytest.mark.parametrize("kw", [dict(), dict(local=True), {k: True for k in FREE}], ids=["global", "local", "free"])
+@pytest.mark.parametrize("width", [0, 32])
+def test_few_tall_pairs_equal_oracle(built_lib, oracle, shape, kw, width):
+    """Few pairs of many more rows than columns: passes of up to 768 rows, whatever the batch's work."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import pairwise_aligner_gb300 as pa
+    rng = np.random.default_rng(12)
+    m, n = shape
+    s1, s2 = [], []
+    for k in range(3):
+        a, b = ACGT[rng.integers(0, 4, m)], ACGT[rng.integers(0, 4, n + k)]
+        b[n // 2:n // 2 + m] = a[:len(b[n // 2:n // 2 + m])]
+        s1.append(bytes(a))
+        s2.append(bytes(b))
+    local = bool(kw.get("local"))
+    free = {k: local or bool(kw.get(k)) for k in FREE}
+    q, qo = pa.pack(s1)
+    t, to = pa.pack(s2)
+    ctx = pa.Context(0)
+    ctx.set_cta_threshold(1)
+    c = dict(local=local, match=2, mismatch=-3, gap_open=-5, gap_extension=-1, width_hint=width, **free)
+    res = pa.Aligner(c, context=ctx).compute_arrays(q, qo, t, to)
+    sc, e1, e2 = oracle.align_batch(oracle.make_cfg(2, -3, -5, -1, local=local, **free), q, qo, t, to)
+    assert np.array_equal(res["score"], sc) and np.array_equal(res["end1"], e1) and np.array_equal(res["end2"], e2)
+    ctx.close()
