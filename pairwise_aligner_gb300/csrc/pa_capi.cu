@@ -465,6 +465,17 @@ pa_status ensure_queue_words(pa_ctx *c)
     return PA_OK;
 }
 
+// Column slots for `columns` bases of sequence1 and pairs; new ones are zeroed, so that none looks
+// like a cell of a row pass (kTagMark).
+pa_status ensure_slots(pa_ctx *c, uint64_t columns)
+{
+    const size_t cap = c->slots.cap;
+    pa_status s = ensure(c, c->slots, columns * sizeof(Slot));
+    if (s) return s;
+    if (c->slots.cap != cap) PA_CUDA(c, cudaMemsetAsync(c->slots.p, 0, c->slots.cap, c->stream));
+    return PA_OK;
+}
+
 // At most so many pairs of a batch are long: their m sum to at most b1 and their n to b2, so if L of
 // them have m * n >= long_cells, L * sqrt(long_cells) <= sqrt(b1 * b2).
 uint64_t most_long(const pa_ctx *c, uint64_t n_pairs, uint64_t b1, uint64_t b2)
@@ -474,8 +485,7 @@ uint64_t most_long(const pa_ctx *c, uint64_t n_pairs, uint64_t b1, uint64_t b2)
 }
 
 // Buffers of the long-pair kernel for a batch of at most `pairs` long pairs.  The boundary cells are
-// the pairs' column slots: a pair is short or long, never both, and k_classify clears the slots of
-// the long ones.
+// the pairs' column slots: a pair is short or long, never both.
 pa_status ensure_long(pa_ctx *c, uint64_t pairs)
 {
     pa_status s = ensure_queue_words(c);
@@ -532,8 +542,8 @@ pa_status enqueue_prep(pa_ctx *c, const DpParams &P, const ClassCfg &C, const ui
     int cls_blocks = (int)std::min<uint64_t>((n_pairs * 32 + 127) / 128, (uint64_t)c->sm_count * 16);
     if (cls_blocks < 1) cls_blocks = 1;
     k_classify<<<cls_blocks, 128, 0, st>>>(s1, o1, b1, s2, o2, b2, n_pairs, P, C, (uint32_t *)c->keys.p,
-                                              small ? nullptr : (uint32_t *)c->hist.p, (uint32_t *)c->qtab.p,
-                                              (uint4 *)c->slots.p, out, pstats(c));
+                                              small ? nullptr : (uint32_t *)c->hist.p, (uint32_t *)c->qtab.p, out,
+                                              pstats(c));
     if (small) {
         k_sort_small<<<1, 1024, 0, st>>>((const uint32_t *)c->keys.p, (uint32_t)n_pairs, (uint32_t *)c->order.p,
                                          (uint32_t *)c->ranges.p, (uint32_t *)c->counts.p, pstats(c), out);
@@ -735,7 +745,7 @@ pa_status prepare_buffers(pa_ctx *c, uint64_t n_pairs, uint64_t b1)
     if ((s = ensure(c, c->counters, 128 + sizeof(PrepStats)))) return s;
     if ((s = ensure(c, c->qtab, (b1 + np) * 4))) return s;
     if ((s = ensure(c, c->boundary, (b1 + np) * sizeof(Cell)))) return s;
-    if ((s = ensure(c, c->slots, (b1 + np) * sizeof(Slot)))) return s;
+    if ((s = ensure_slots(c, b1 + np))) return s;
     return PA_OK;
 }
 
@@ -1860,13 +1870,12 @@ pa_status pa_traceback_batch(pa_ctx *ctx, const pa_config *config, const uint8_t
     if ((s = ensure(ctx, ctx->tb_dir, most * 4))) return s;
     // the tagged kernels' boundary cells take twice the memory of k_traceback's: without room for them
     // the call runs on that one
-    if (tagged && ensure(ctx, ctx->slots, (b1 + n_pairs) * sizeof(Slot))) tagged = false;
+    if (tagged && ensure_slots(ctx, b1 + n_pairs)) tagged = false;
     if (!tagged && (s = ensure(ctx, ctx->boundary, (b1 + n_pairs) * sizeof(Cell)))) return s;
     std::vector<uint64_t> r1(off1, off1 + n_pairs + 1), r2(off2, off2 + n_pairs + 1);
     for (auto &v : r1) v -= base1;
     for (auto &v : r2) v -= base2;
     cudaStream_t st = ctx->stream;
-    if (tagged) PA_CUDA(ctx, cudaMemsetAsync(ctx->slots.p, 0, (b1 + n_pairs) * sizeof(Slot), st));
     PA_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
     if (b1) PA_CUDA(ctx, cudaMemcpyAsync(ctx->in_seq1.p, seq1 + base1, b1, cudaMemcpyHostToDevice, st));
     if (b2) PA_CUDA(ctx, cudaMemcpyAsync(ctx->in_seq2.p, seq2 + base2, b2, cudaMemcpyHostToDevice, st));

@@ -14,8 +14,9 @@
 // column, {H, vertical gap, tag}, written and read with single 128-bit relaxed accesses at
 // GPU scope.  The tag names the launch and the pass, so a reader that finds it has the whole
 // cell: no flag, no fence, no order between cells is needed.  The cells are the pair's column slots
-// of the short-pair kernel, cleared by k_classify (a memory of their own would add 16 bytes per base
-// of sequence1 to every call that may hold a long pair).  The row is reused in place:
+// of the short-pair kernel (a memory of their own would add 16 bytes per base of sequence1 to every
+// call that may hold a long pair); no slot's contents look like a tag (kTagMark).  The row is reused in
+// place:
 // pass p overwrites column i only after its own first thread read column i.  The reader
 // fetches blocks of kStage columns, one block ahead (lane t the block's column t), and hands
 // them to thread 0 through shared memory with the score tables; a cell that is not there yet
@@ -50,8 +51,16 @@ struct LongUnit {
     int32_t fail;                  // a wait of this pass ran out
 };
 
-// A cell's tag: the launch (a counter of the context), then the pass.
+// A cell's tag: the mark, the launch (a counter of the context, below 2^38), the pass.  Where a slot
+// keeps its vertical gap, a tag has its upper half, which the mark sets to a value that no gap has: bits
+// 31 and 30 are 1 0, but s32 gaps lie within 2^30 of zero (the classifier's overflow bound), and both
+// s16x2 halves are positive (clamped H is at least 2,048, opening a gap takes at most 1,000).
 constexpr int kTagPassBits = 24;
+constexpr uint64_t kTagMark = 1ull << 63;
+__device__ __forceinline__ uint64_t pass_tag(uint64_t epoch, int32_t pass)
+{
+    return kTagMark | (epoch << kTagPassBits) | (uint32_t)pass;
+}
 
 __device__ __forceinline__ ulonglong2 load_cell128(const ulonglong2 *p)
 {
@@ -468,7 +477,7 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
             u.passes = (u.nh + 32 * u.rpt - 1) / (32 * u.rpt);
             const uint32_t owner = u.m[1] > u.m[0] ? u.id[1] : u.id[0];
             u.row = Q.cells + (L.off1[owner] + owner);        // cells 0..m(owner) = 0..ms
-            u.tag = (epoch << kTagPassBits) | (uint32_t)p;
+            u.tag = pass_tag(epoch, p);
             if (BAND)
                 for (int k = 0; k < 3; ++k) u.win[k] = long_window<NL>(L, u, min(max(p + k - 1, 0), u.passes - 1));
             su = u;

@@ -114,16 +114,16 @@ __device__ __forceinline__ bool all_dna(const uint8_t *seq, uint64_t bytes, uint
 }
 
 // One warp per pair: check the pair's offsets against the byte buffers and sequence2's
-// alphabet, pick the class, write the bucket key, the score tables of sequence1, empty boundary
-// cells for long pairs and the results of pairs the DP does not compute: empty sequences (their border result),
+// alphabet, pick the class, write the bucket key, the score tables of sequence1 and the
+// results of pairs the DP does not compute: empty sequences (their border result),
 // inconsistent offsets, scores that could exceed int32 and, with a substitution matrix,
 // symbols outside it (INT32_MIN and a PA_RESULT_* flag).  Sequence bytes and scratch
 // indices are touched only for pairs whose offsets passed the check.
 __global__ void k_classify(const uint8_t *__restrict__ seq1, const uint64_t *__restrict__ off1, uint64_t seq1_bytes,
                            const uint8_t *__restrict__ seq2, const uint64_t *__restrict__ off2, uint64_t seq2_bytes,
                            uint64_t n_pairs, DpParams P, ClassCfg C, uint32_t *__restrict__ keys,
-                           uint32_t *__restrict__ hist, uint32_t *__restrict__ qtab, uint4 *__restrict__ slots,
-                           pa_result *__restrict__ out, PrepStats *__restrict__ st)
+                           uint32_t *__restrict__ hist, uint32_t *__restrict__ qtab, pa_result *__restrict__ out,
+                           PrepStats *__restrict__ st)
 {
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -200,9 +200,6 @@ __global__ void k_classify(const uint8_t *__restrict__ seq1, const uint64_t *__r
                     if (i + u <= m) qt[i + u] = (i + u < m) ? score_table(a[u], match4, mis4) : 0x80808080u;
             }
         }
-        // boundary cells of a long pair: whatever another call left in its slots could pass for a tag
-        if (klass == K_S16L || klass == K_S32L)
-            for (int64_t i = lane; i <= m; i += 32) slots[q0 + p + i] = make_uint4(0u, 0u, 0u, 0u);
         if (lane == 0) {
             uint32_t key;
             if (klass == K_NONE) {

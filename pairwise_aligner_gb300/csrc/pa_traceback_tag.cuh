@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kTagThreads, 4) k_tb_dp(TbLaunch L, DpParams P
             x.b_seq = L.seq2 + r0;
             x.D = L.dir + L.dir_off[q] + (uint64_t)p * (uint32_t)(x.m + 31) * 64u;
             x.row = L.cells + (q0 - L.off1[0]) + k;
-            x.tag = (epoch << kTagPassBits) | (uint32_t)p;
+            x.tag = pass_tag(epoch, p);
             x.fail = 0;
             w = x;
         }

@@ -74,3 +74,35 @@ def test_few_tall_pairs_equal_oracle(built_lib, oracle, shape, kw, width):
     sc, e1, e2 = oracle.align_batch(oracle.make_cfg(2, -3, -5, -1, local=local, **free), q, qo, t, to)
     assert np.array_equal(res["score"], sc) and np.array_equal(res["end1"], e1) and np.array_equal(res["end2"], e2)
     ctx.close()
+
+
+def test_long_pairs_after_short_ones_in_the_same_slots(built_lib, oracle):
+    """The passes' boundary cells are the slots that short pairs of earlier calls, tracebacks and other
+    long pairs have written: alternating calls of one context stay exact."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import pairwise_aligner_gb300 as pa
+    rng = np.random.default_rng(14)
+    ctx = pa.Context(0)
+
+    def batch(shapes):
+        s1 = [bytes(ACGT[rng.integers(0, 4, m)]) for m, _ in shapes]
+        return (*pa.pack(s1), *pa.pack([bytes(ACGT[rng.integers(0, 4, n)]) for _, n in shapes]))
+
+    for k, width in enumerate((0, 32, 0, 32)):
+        for local in (False, True):
+            f = dict.fromkeys(FREE, local)
+            c = dict(local=local, match=2, mismatch=-3, gap_open=-5, gap_extension=-1, width_hint=width, **f)
+            oc = oracle.make_cfg(2, -3, -5, -1, local=local, **f)
+            al = pa.Aligner(c, context=ctx)
+            for shapes in ([(int(m), 70) for m in rng.integers(1, 200, 400)], [(1200, 1300 + k), (2000, 900)] * 4):
+                b = batch(shapes)
+                res = al.compute_arrays(*b)
+                sc, e1, e2 = oracle.align_batch(oc, *b)
+                assert np.array_equal(res["score"], sc) and np.array_equal(res["end1"], e1)
+                assert np.array_equal(res["end2"], e2)
+            b = batch([(700, 1100)] * 6)
+            res = al.compute_traceback_arrays(*b)[0]
+            assert np.array_equal(res["score"], oracle.align_batch(oc, *b)[0])
+    ctx.close()
