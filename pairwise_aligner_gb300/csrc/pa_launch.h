@@ -47,14 +47,14 @@ __device__ inline int32_t long_rows(uint32_t budget, int32_t floor_rows, int32_t
 // The queue of a launch: unit u's passes are tickets start[u] .. start[u + 1] - 1.
 struct LongWords {
     uint32_t tasks;                // tickets
-    uint32_t budget;               // rows per thread x columns a pass may cover (long_rows)
-    int32_t floor_rows;
     uint32_t pad;
     uint64_t epoch;                // names the launch in the cell tags
 };
 struct LongRecord {                // a unit's best candidates between its passes
     int32_t s[2], i[2], j[2];
     int32_t ub[2];                 // band mode: the largest exit bound
+    int32_t rpt;                   // rows per thread of a full pass, from k_long_plan (not in band mode)
+    int32_t pad;
 };
 struct LongQueue {
     LongWords *words;

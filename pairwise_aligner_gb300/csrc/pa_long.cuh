@@ -451,8 +451,6 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
     const uint32_t units = (count + NL - 1) / NL;
     const uint32_t total = Q.words->tasks;
     if (!strip_warp_takes_part(total)) return;
-    const uint32_t budget = Q.words->budget;
-    const int32_t floor_rows = Q.words->floor_rows;
     const uint64_t epoch = Q.words->epoch;
     const uint32_t *order = L.order + *L.begin_ptr;
 
@@ -473,7 +471,7 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
         }
         if (t == 0) {
             LongUnit u = long_unit<NL>(L, order, (units - 1 - uu) * NL, count);   // largest units first
-            u.rpt = BAND ? L.band_rows / 32 : long_rows(budget, floor_rows, u.ms, u.nh);
+            u.rpt = BAND ? L.band_rows / 32 : __ldcg(&Q.rec[uu].rpt);
             u.passes = (u.nh + 32 * u.rpt - 1) / (32 * u.rpt);
             const uint32_t owner = u.m[1] > u.m[0] ? u.id[1] : u.id[0];
             u.row = Q.cells + (L.off1[owner] + owner);        // cells 0..m(owner) = 0..ms

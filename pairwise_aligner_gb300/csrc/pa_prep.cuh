@@ -367,9 +367,9 @@ __global__ void __launch_bounds__(1024) k_sort_small(const uint32_t *__restrict_
     if (threadIdx.x < kClasses) counts[threadIdx.x] = bad ? 0u : begin[threadIdx.x + 1] - begin[threadIdx.x];
 }
 
-// The pass queues of one or two long-pair launches (dp_long) that run side by side: start[u] for
-// the units of a list, largest first (the list is ascending), the budget of a pass, and the
-// launch's epoch.  Block b plans list b.
+// The pass queues of one or two long-pair launches (dp_long) that run side by side: start[u] and the
+// rows of a pass for the units of a list, largest first (the list is ascending), and the launch's
+// epoch.  Block b plans list b.
 struct LongPlan {
     const uint32_t *order, *begin, *count;
     int32_t lanes;                 // pairs per unit
@@ -421,8 +421,9 @@ __global__ void __launch_bounds__(1024) k_long_plan(LongPlan a, LongPlan b, cons
         uint32_t total, v = 0;
         if (u < units) {
             const uint2 s = long_shape(p, off1, off2, count, units, u);
-            const uint32_t rows = 32u * (uint32_t)long_rows(budget, floor_rows, (int32_t)s.x, (int32_t)s.y);
-            v = (s.y + rows - 1) / rows;
+            const int32_t rpt = long_rows(budget, floor_rows, (int32_t)s.x, (int32_t)s.y);
+            p.Q.rec[u].rpt = rpt;
+            v = (s.y + 32u * rpt - 1) / (32u * rpt);
         }
         const uint32_t ex = block_exclusive_scan(v, sh, total);
         if (u < units) {
@@ -435,8 +436,6 @@ __global__ void __launch_bounds__(1024) k_long_plan(LongPlan a, LongPlan b, cons
     if (threadIdx.x == 0) {
         p.Q.start[units] = carry;
         p.Q.words->tasks = carry;
-        p.Q.words->budget = budget;
-        p.Q.words->floor_rows = floor_rows;
         p.Q.words->epoch = (uint64_t)atomicAdd(epoch, 1ull) + 1ull;
     }
 }
