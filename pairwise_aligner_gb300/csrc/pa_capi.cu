@@ -34,6 +34,7 @@ namespace {
 constexpr int kR = 16;             // rows per thread per lane
 constexpr int64_t kDefaultRingM = 65536;   // device entry points: CTA mode up to this sequence1 length
 constexpr int kDefaultG = 8;       // threads per group
+constexpr int64_t kLongCells = 1ll << 20;
 // Page-locked host words of a context: [0, 8) band mode's bad-offset count, [16, 80) class
 // ranges, [80, 144) class counts, [160, 224) the two band steps' totals, [224, 236) the long
 // full-DP routing counts, [256, 280) full-DP list sizes (host to device), from 512 the
@@ -97,7 +98,7 @@ struct pa_ctx {
     DevBuf ring, rerun_long;      // CTA mode: boundary rows per block; s16 long pairs to redo in s32
     int32_t ring_m = 0;           // longest sequence1 the ring rows hold (0: no CTA mode yet)
     int ring_grid = 0;            // blocks of every CTA-mode launch
-    int64_t long_cells = 1ll << 20;   // pairs with at least this many cells are long
+    int64_t long_cells = kLongCells;  // pairs with at least this many cells are long
     int64_t huge_cells = 1ll << 28;   // byte-compare and banded: ... and this many (and n >= huge_min_n): clusters
     int32_t huge_min_n = 8192;
     int32_t team_max_n = 12288;       // byte-compare long pairs of at most this many rows run on teams
@@ -1253,6 +1254,22 @@ pa_status read_stats(pa_ctx *c, pa_stats *stats, bool staged)
     return PA_OK;
 }
 
+// Which pairs of more than long_cells cells stay with the short-pair kernel, on its 32-lane groups.
+// A pair of at most 128 rows is one pass in either kernel, and the short one's columns cost less unless
+// there are thousands of them: a global pair of 200,000 x 100 56.9 ms on the queue, 52.3 there; free ends
+// 86.6 and 59.6.  Pairs of few columns and many rows keep few warps busy each, and when the batch is full
+// of them the warps of the later passes only wait (a pass starts 47 columns behind the one above): 2,000
+// local pairs of 150 x 8,000 1,368 us on the queue, 804 there; of 300 x 8,000 1,856 and 1,339; but 1,100 of
+// 384 x 3,000 532 and 652, 1,000 of 600 x 8,000 1,633 and 2,363.  A caller who lowers the threshold wants
+// the queue.
+void one_warp_rules(const pa_ctx *c, ClassCfg &C, uint64_t n_pairs, uint64_t b1, uint64_t b2)
+{
+    if (c->long_cells < kLongCells) return;
+    if (n_pairs <= 1024) C.one_warp_rows = 128;
+    const double m = (double)b1 / (double)n_pairs, n = (double)b2 / (double)n_pairs;
+    if (n_pairs >= 1024 && m <= 384.0 && n >= 20.0 * m && m * n >= 0.5 * (double)kLongCells) C.one_warp_cols = 384;
+}
+
 pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uint64_t *o1, uint64_t b1,
                      const uint8_t *s2, const uint64_t *o2, uint64_t b2, uint64_t n_pairs, pa_result *out,
                      pa_stats *stats, bool sync_for_stats)
@@ -1269,6 +1286,7 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
     // the short-pair kernel (launch_class) builds its own column tables: a class needs none when
     // neither it nor, for global s16x2 pairs, their s32 redo runs on dp_kernel
     auto on_short = [&](Klass k) { return c->variant[k] >= kShortVariant && dp_short_supports(c->G[k]); };
+    if (n_pairs) one_warp_rules(c, C, n_pairs, b1, b2);
     if (on_short(K_S32)) C.qtab_s32 = 0;
     if (on_short(K_S16) && (P.local || on_short(K_S32))) C.qtab_s16 = 0;
     if (n_pairs == 0) {

@@ -23,6 +23,7 @@ struct ClassCfg {
     int32_t huge_min_n;
     int32_t team_max_n;      // CTA-mode pairs with n at most this run on teams of 4 warps (0: none)
     int32_t pass_queue;      // the call may hold long pairs (their kernels are launched)
+    int32_t one_warp_rows, one_warp_cols;   // pairs of a 32-lane class up to these stay short (0: none)
     int32_t qtab_s16, qtab_s32;   // write the score tables of K_S16, K_S32 (0: their kernels build their own)
     const int8_t *rank_map;  // substitution-matrix scoring: symbol -> rank (null: unitary scores)
 };
@@ -185,7 +186,9 @@ __global__ void k_classify(const uint8_t *__restrict__ seq1, const uint64_t *__r
         // the clamp floor (checked after the DP), so any length may try s16 first
         else if (!C.force32 && C.s16_params && (!C.local || (int64_t)P.smax * min(m, n) <= 30000)) klass = K_S16;
         else klass = K_S32;
-        if (klass != K_NONE && C.pass_queue && m * n >= C.long_cells && n <= (1 << 20) &&
+        // DNA pairs whose passes one warp runs as well as several (one_warp_rules)
+        const bool one_warp = klass < K_GEN && C.gcnt[klass] == 32 && (n <= C.one_warp_rows || m <= C.one_warp_cols);
+        if (klass != K_NONE && C.pass_queue && !one_warp && m * n >= C.long_cells && n <= (1 << 20) &&
             m <= (klass != K_GEN ? (1 << 20) : C.long_max_m))
             klass += klass != K_GEN                                 ? kLongOffset
                      : (m * n >= C.huge_cells && n >= C.huge_min_n) ? kHugeOffset

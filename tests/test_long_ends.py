@@ -106,3 +106,39 @@ def test_long_pairs_after_short_ones_in_the_same_slots(built_lib, oracle):
             res = al.compute_traceback_arrays(*b)[0]
             assert np.array_equal(res["score"], oracle.align_batch(oc, *b)[0])
     ctx.close()
+
+
+@pytest.mark.parametrize("shapes", [[(8300, n) for n in (126, 127, 128, 129, 130)] * 4,
+                                    [(m, 2800) for m in (382, 383, 384, 385, 386)] * 4 + [(64, 9000)] * 1020],
+                         ids=["flat", "narrow"])
+@pytest.mark.parametrize("kw", [dict(), dict(local=True), {k: True for k in FREE}], ids=["global", "local", "free"])
+@pytest.mark.parametrize("width", [0, 32])
+def test_pairs_on_both_sides_of_the_one_warp_rules(built_lib, oracle, shapes, kw, width):
+    """Pairs above the long threshold: up to 128 rows, or 384 columns in a batch full of narrow pairs, they
+    stay with the short-pair kernel."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import pairwise_aligner_gb300 as pa
+    rng = np.random.default_rng(13)
+    s1, s2 = [], []
+    for m, n in shapes:
+        a, b = ACGT[rng.integers(0, 4, m)], ACGT[rng.integers(0, 4, n)]
+        w = min(m, n)
+        at = int(rng.integers(0, max(m, n) - w + 1))
+        if n > m:
+            b[at:at + w] = a
+        else:
+            a[at:at + w] = b
+        s1.append(bytes(a))
+        s2.append(bytes(b))
+    local = bool(kw.get("local"))
+    free = {k: local or bool(kw.get(k)) for k in FREE}
+    q, qo = pa.pack(s1)
+    t, to = pa.pack(s2)
+    c = dict(local=local, match=2, mismatch=-3, gap_open=-5, gap_extension=-1, width_hint=width, **free)
+    al = pa.Aligner(c, context=pa.Context(0))
+    res = al.compute_arrays(q, qo, t, to)
+    sc, e1, e2 = oracle.align_batch(oracle.make_cfg(2, -3, -5, -1, local=local, **free), q, qo, t, to)
+    assert np.array_equal(res["score"], sc) and np.array_equal(res["end1"], e1) and np.array_equal(res["end2"], e2)
+    al.context.close()
