@@ -411,7 +411,9 @@ void warm_occupancy()
         for (int form = 0; form < kShortFormCount; ++form) dp_short_occupancy(form, mode);
         dp_short32_occupancy(SC_TABLE, mode, 0);
         dp_short32_occupancy(SC_BYTES, mode, 0);
+        for (bool lanes16 : {true, false}) dp_long_occupancy(lanes16, mode);
     }
+    for (bool lanes16 : {true, false}) dp_long_band_occupancy(lanes16);
 }
 
 int dp_mode(const DpParams &P)

@@ -5,6 +5,7 @@ from __future__ import annotations
 import ctypes
 import os
 import re
+import shutil
 import subprocess
 
 import numpy as np
@@ -16,6 +17,7 @@ from conftest import REPO
 class HostRuntime:
     def __init__(self, path):
         from pairwise_aligner_gb300 import _lib
+        self.path = path
         self._lib = _lib
         self.lib = _lib.load(path)
         for name, res in (("events", ctypes.c_char_p), ("most", ctypes.c_size_t), ("reset", None), ("limit", None)):
@@ -162,3 +164,17 @@ def test_traceback_without_room_for_tagged_cells(host):
         seen.append([re.search(r"k_t\w+", e)[0] for e in host.events() if "k_t" in e])
         host.lib.pa_destroy(ctx)
     assert all("k_tb" in x for x in seen[0]) and all("k_traceback" in x for x in seen[1]), seen
+
+
+def test_no_occupancy_query_inside_a_capture(host, tmp_path):
+    """What a launch needs to know of a kernel is asked when the context is made or the matrix set: the first
+    calls of a process only enqueue while they are captured."""
+    fresh = HostRuntime(shutil.copy(host.path, str(tmp_path / "fresh.so")))      # nothing asked yet
+    ctx = fresh.context()
+    assert fresh.matrix(ctx, 20) == 0
+    for local, free in ((True, False), (False, False), (False, True)):
+        for matrix in (False, True):
+            for n, m in ((5000, 200), (300, 3000)):
+                assert fresh.align_device(ctx, n, n * m, n * m, local, matrix, free=free) == 0
+    assert not [e for e in fresh.events() if "in a capture" in e]
+    fresh.lib.pa_destroy(ctx)
