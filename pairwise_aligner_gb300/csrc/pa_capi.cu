@@ -709,7 +709,9 @@ pa_status enqueue(pa_ctx *c, const pa_config *cfg, const DpParams &P, const Clas
     return PA_OK;
 }
 
-// Ring rows of CTA mode for sequence1 lengths up to `max_m` (grow only).
+// Ring rows of CTA mode for sequence1 lengths up to `max_m` (grow only).  A call without room for them
+// goes on without: long byte-compare pairs then run on the group kernels, and no other pair needs a ring
+// (61 GB for a sequence1 of 2^20).
 pa_status ensure_ring(pa_ctx *c, int64_t max_m)
 {
     if (max_m <= 0) return PA_OK;
@@ -873,7 +875,7 @@ pa_status run_band(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const uin
     pa_status s = check_config(c, cfg, P, C);
     if (s) return s;
     apply_tuning(c, cfg, P, n_pairs, b1, b2, h_bands != nullptr);
-    if (n_pairs && (s = ensure_ring(c, c->want_ring_m))) return s;
+    if (n_pairs && (s = ensure_ring(c, c->want_ring_m)) && s != PA_ERR_OUT_OF_MEMORY) return s;
     set_classes(c, C);
     C.team_max_n = 0;                                 // band mode has its own team choice
     if (P.local || P.first_column_free || P.first_row_free || P.last_column_free || P.last_row_free)
@@ -1283,7 +1285,7 @@ pa_status run_device(pa_ctx *c, const pa_config *cfg, const uint8_t *s1, const u
     pa_status s = check_config(c, cfg, P, C);
     if (s) return s;
     apply_tuning(c, cfg, P, n_pairs, b1, b2, false);
-    if (n_pairs && (s = ensure_ring(c, c->want_ring_m))) return s;
+    if (n_pairs && (s = ensure_ring(c, c->want_ring_m)) && s != PA_ERR_OUT_OF_MEMORY) return s;
     set_classes(c, C);
     // the short-pair kernel (launch_class) builds its own column tables: a class needs none when
     // neither it nor, for global s16x2 pairs, their s32 redo runs on dp_kernel

@@ -178,3 +178,24 @@ def test_no_occupancy_query_inside_a_capture(host, tmp_path):
                 assert fresh.align_device(ctx, n, n * m, n * m, local, matrix, free=free) == 0
     assert not [e for e in fresh.events() if "in a capture" in e]
     fresh.lib.pa_destroy(ctx)
+
+
+@pytest.mark.parametrize("band_mode", [0, 2])
+def test_a_long_pair_without_room_for_ring_rows(host, band_mode):
+    """Only long byte-compare pairs use the ring rows, 24 bytes per base of the longest sequence1 and resident
+    warp (61 GB at 2^20): a call that has no room for them runs all the same."""
+    m, n = 1 << 20, 2000
+    s1, s2 = np.full(m, 65, np.uint8), np.full(n, 65, np.uint8)
+    o1, o2 = np.array([0, m], np.uint64), np.array([0, n], np.uint64)
+    cfg, out = host._lib.PaConfig(0, 2, -3, -5, -1, 0, 0, 0, 0, 0, band_mode), np.zeros(16, np.uint8)
+    ctx = host.context()
+    host.events()
+    host._limit(2 * 10**9)
+    rc = host.lib.pa_align_batch(ctx, ctypes.byref(cfg), s1.ctypes.data, o1.ctypes.data, s2.ctypes.data, o2.ctypes.data,
+                                 1, out.ctypes.data, None)
+    host._limit(2**63)
+    assert rc == 0
+    ev = host.events()
+    assert band_mode or any("dp_longI" in e for e in ev)
+    assert not any("dp_kernel_c" in e or "dp_kernel_team" in e for e in ev)
+    host.lib.pa_destroy(ctx)
