@@ -4,8 +4,9 @@
 // synchronisation inside it (so it can be captured once into a CUDA graph and
 // replayed):
 //   1. k_classify    class, bucket key, score tables and empty-pair results
-//   2. k_scan_*      exclusive scan of the bucket histogram (2^18 buckets)
-//   3. k_scatter     bucket sort of the pair ids (order inside a bucket is free)
+//   2. k_scan_*      exclusive scan of the bucket histogram (2^20 buckets)
+//   3. k_scatter     bucket sort of the pair ids (order inside a bucket is free); up to 4,096 pairs
+//                    k_sort_small does both in one block
 //   4. persistent DP kernels per class (s16x2, s32, byte-compare), each pulling work from its own
 //      device queue, longest first: dp_short / dp_kernel for short pairs, dp_long for long ones
 //   5. s32 recomputation of s16 global results that failed their check
@@ -30,16 +31,15 @@ using namespace pa;
 
 namespace {
 
-
 constexpr int kR = 16;             // rows per thread per lane
 constexpr int64_t kDefaultRingM = 65536;   // device entry points: CTA mode up to this sequence1 length
-constexpr int kDefaultG = 8;       // threads per group
+constexpr int kDefaultG = 8;       // threads per group before a call's rule has set them
 constexpr int64_t kLongCells = 1ll << 20;
 // Page-locked host words of a context: [0, 8) band mode's bad-offset count, [16, 80) class
-// ranges, [80, 144) class counts, [160, 224) the two band steps' totals, [224, 236) the long
-// full-DP routing counts, [256, 280) full-DP list sizes (host to device), from 512 the
-// counters and statistics of a finished call (stage_stats).  Each is read only after a wait on the stream
-// that wrote it, and written only after the previous call's work on that stream finished.
+// ranges, [80, 144) class counts, [160, 168) a band step's counts, [256, 272) full-DP list sizes
+// (host to device), from 512 the counters and statistics of a finished call (stage_stats).  Each is
+// read only after a wait on the stream that wrote it, and written only after the previous call's
+// work on that stream finished.
 constexpr size_t kPinnedBytes = 1024;
 // Behind them, staging of small host calls: their inputs go over in one copy and their results
 // come back through page-locked words (a copy from or to pageable memory costs 5-10 us each).
@@ -99,10 +99,10 @@ struct pa_ctx {
     int32_t ring_m = 0;           // longest sequence1 the ring rows hold (0: no CTA mode yet)
     int ring_grid = 0;            // blocks of every CTA-mode launch
     int64_t long_cells = kLongCells;  // pairs with at least this many cells are long
-    int64_t huge_cells = 1ll << 28;   // byte-compare and banded: ... and this many (and n >= huge_min_n): clusters
+    int64_t huge_cells = 1ll << 28;   // byte-compare: ... and this many (and n >= huge_min_n): clusters
     int32_t huge_min_n = 8192;
     int32_t team_max_n = 12288;       // byte-compare long pairs of at most this many rows run on teams
-    uint32_t wait_limit = kSpinLimit; // polls of a CTA-mode progress wait before it gives up
+    uint32_t wait_limit = kSpinLimit; // polls of a wait between a long pair's passes before it gives up
     int64_t want_ring_m = 0;          // the next call's longest CTA-mode sequence1 (host: exact)
     DevBuf in_seq1, in_off1, in_seq2, in_off2, in_out, in_small;   // staging for the host-buffer entry points
     int G[3] = {kDefaultG, kDefaultG, kDefaultG};
@@ -240,8 +240,6 @@ void set_classes(const pa_ctx *c, ClassCfg &C)
     for (int k = 0; k < kClasses; ++k) {
         const bool cta = k >= (int)kLongOffset;
         C.gcnt[k] = cta ? 32 : c->G[k < 3 ? k : 0];
-        C.rpt[k] = kR;
-        C.rows[k] = C.gcnt[k] * kR;
     }
     C.long_max_m = c->use_long && c->ring.p ? c->ring_m : 0;
 }
@@ -518,10 +516,10 @@ LongQueue long_queue(pa_ctx *c, int k)
 
 int long_grid(pa_ctx *c, bool lanes16, int mode) { return dp_long_occupancy(lanes16, mode) * c->sm_count; }
 
-// The pass queues of one or two lists (s16x2 units, s32 units); a null list gets no block.
 // The word that counts long-pair launches.
 unsigned long long *long_epoch(pa_ctx *c) { return (unsigned long long *)((LongWords *)c->long_words.p + 3); }
 
+// The pass queues of one or two lists (s16x2 units, s32 units); a null list gets no block.
 void plan_long(pa_ctx *c, cudaStream_t st, const uint64_t *o1, const uint64_t *o2, int mode, const LongPlan *p16, const LongPlan *p32)
 {
     const LongPlan &a = p16 ? *p16 : *p32;
@@ -775,9 +773,10 @@ int tune_shape_class(uint64_t n_pairs, uint64_t b1, uint64_t b2)
 // pairs do not outlast the rest, and that holds a pair of mean length in two passes.  A warp unit
 // holds 32 / G groups of `lanes` pairs, a pass G * rows rows.  Measured (GB300, us per call on 8 /
 // 16 / 32 lanes): 65,537 reads of 175 rows 1,119 / 1,156 / 1,514; 16,384 pairs of 64-1,000 rows
-// 1,653 / 935 / 580; 60,000 local pairs of 288 rows 1,316 / 1,244 / 1,464; 32,768 proteins of 335
-// rows (16 per thread) 2,342 / 1,548 / 1,588.  Groups of 4 lanes pay for pairs of at most 128
-// rows, one pass of them: 262,144 local pairs of 288 rows 8,195, on 8 lanes 4,696.
+// 1,653 / 935 / 580; 60,000 local pairs of 288 rows 1,316 / 1,244 / 1,464 (the rule takes 8, 6 % behind
+// 16: the line that is right for the reads lies between); 32,768 proteins of 335 rows (16 per thread)
+// 2,342 / 1,548 / 1,588.  Groups of 4 lanes pay for pairs that are one pass of them, 128 rows (s32
+// lanes 64): 262,144 local pairs of 288 rows 8,195, on 8 lanes 4,696.
 int rule_group_threads(const pa_ctx *c, uint64_t n_pairs, uint64_t b2, int lanes, int rows)
 {
     const double warps = (double)c->sm_count * (2 * kBlock / 32);
@@ -787,11 +786,12 @@ int rule_group_threads(const pa_ctx *c, uint64_t n_pairs, uint64_t b2, int lanes
     return 32;
 }
 
-// ... and of the general kernel, which runs explicit variants 0..8, matrix scores beyond a signed byte
-// and short pairs with caller-given bands: about eight units per resident warp, whatever the lengths.
-// With the short-pair kernel's rule 60,000 free-end pairs of 64-512 rows took 6,906 us on variant 4
-// (4,291 with this one), 60,000 with given bands 4,813 (2,590), 20,000 under a matrix of large scores
-// 6,104 (4,668).
+// ... and of the general kernel in global modes, which runs explicit variants 0..8, matrix scores beyond a
+// signed byte and short pairs with caller-given bands: about eight units per resident warp, whatever the
+// lengths.  With the short-pair kernel's rule 60,000 free-end pairs of 64-512 rows took 6,906 us on
+// variant 4 (4,291 with this one), 60,000 with given bands 4,813 (2,590), 20,000 under a matrix of large
+// scores 6,104 (4,668).  In local mode the short-pair kernel's rule is the better one for it, too (60,000
+// pairs on variant 7 1,632 us, 1,918 with this one).
 int rule_group_threads_general(const pa_ctx *c, uint64_t n_pairs, int lanes)
 {
     const double warps = (double)c->sm_count * (2 * kBlock / 32);
@@ -814,8 +814,8 @@ void apply_tuning(pa_ctx *c, const pa_config *cfg, const DpParams &P, uint64_t n
         int g32 = c->tuning.group_threads_s32[mi];
         // dp_kernel runs the banded DP of the DNA classes, and what launch_class does not give dp_short
         auto rule = [&](Klass k, bool short_kernel, int lanes, int rows) {
-            return short_kernel && c->variant[k] >= kShortVariant ? rule_group_threads(c, n_pairs, b2, lanes, rows)
-                                                                  : rule_group_threads_general(c, n_pairs, lanes);
+            return P.local || (short_kernel && c->variant[k] >= kShortVariant)
+                       ? rule_group_threads(c, n_pairs, b2, lanes, rows) : rule_group_threads_general(c, n_pairs, lanes);
         };
         const bool gen_short = short_fits(dp_mode(P), true, (cfg->method & PA_SCORE_MATRIX) != 0, P);
         c->G[K_S16] = g16 ? g16 : rule(K_S16, !given_bands, 2, 32);
@@ -1252,7 +1252,7 @@ pa_status read_stats(pa_ctx *c, pa_stats *stats, bool staged)
     if (ps.bad_offsets)
         return fail(c, PA_ERR_INVALID_ARGUMENT,
                     "offsets decrease or run past seq1_bytes / seq2_bytes; no pair was aligned");
-    if (ctr[8]) return fail(c, PA_ERR_TIMEOUT, "a CTA-mode progress wait ran out");
+    if (ctr[8]) return fail(c, PA_ERR_TIMEOUT, "a wait between the passes of a long pair ran out");
     if (ps.overflow) return fail(c, PA_ERR_OVERFLOW, "scores of some pairs could exceed int32");
     if (ps.invalid) return fail(c, PA_ERR_INVALID_ARGUMENT, "a sequence holds a symbol outside the substitution matrix");
     return PA_OK;

@@ -14,14 +14,12 @@ struct ClassCfg {
     int32_t s16_params;      // gap scores small enough for s16 lanes
     int32_t force32;         // width hint 32
     int32_t local;
-    int32_t rows[kClasses];  // rows per pass (G*R) of each DP class
     int32_t gcnt[kClasses];  // G of each class (for the last-pass chunk count)
-    int32_t rpt[kClasses];   // R of each class
-    int64_t long_cells;      // pairs with m*n at least this (and m <= long_max_m) go to CTA mode
-    int64_t huge_cells;      // ... and with m*n at least this and n >= huge_min_n to cluster mode
+    int64_t long_cells;      // pairs with m*n at least this are long (byte comparison: and m <= long_max_m)
+    int64_t huge_cells;      // byte comparison: with m*n at least this and n >= huge_min_n to cluster mode
     int32_t long_max_m;      // the longest sequence1 the ring rows hold
     int32_t huge_min_n;
-    int32_t team_max_n;      // CTA-mode pairs with n at most this run on teams of 4 warps (0: none)
+    int32_t team_max_n;      // byte comparison: with n at most this on teams of 4 warps (0: none)
     int32_t pass_queue;      // the call may hold long pairs (their kernels are launched)
     int32_t one_warp_rows, one_warp_cols;   // pairs of a 32-lane class up to these stay short (0: none)
     int32_t qtab_s16, qtab_s32;   // write the score tables of K_S16, K_S32 (0: their kernels build their own)
@@ -307,7 +305,7 @@ __global__ void k_scatter(const uint32_t *__restrict__ keys, uint64_t n_pairs, u
     const uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const bool bad = st->bad_offsets != 0;
     if (p == 0) {
-        // class sizes from the class begins (classes 7 and 11.. hold no keys)
+        // class sizes from the class begins (7 to 9 and 11 to 13 are no classes and hold no keys)
         for (int c = 0; c < kClasses; ++c) counts[c] = bad ? 0u : ranges[c + 1] - ranges[c];
     }
     if (p >= n_pairs) return;

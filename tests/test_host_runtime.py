@@ -108,8 +108,8 @@ def test_every_s32_variant_names_its_kernel(host, local):
 
 
 def test_group_size_of_the_general_kernel(host):
-    """Its rule is its own: about eight units per resident warp (2,432 of them here), lane by lane; the
-    short-pair kernel takes smaller groups for the same batches."""
+    """Its rule in global modes is its own: about eight units per resident warp (2,432 of them here), lane by
+    lane; the short-pair kernel takes smaller groups for the same batches."""
     def groups(ctx, n, **kw):
         host.events()
         assert host.align_device(ctx, n, n * 288, n * 288, **kw) == 0
@@ -123,8 +123,9 @@ def test_group_size_of_the_general_kernel(host):
     assert groups(general, 60000, local=False, free=True) == {("kernel", "L16"): {32}, ("kernel", "L32"): {16}}
     matrix = host.context(use_graphs=-1)
     assert host.matrix(matrix, 20, top=400) == 0
-    assert groups(matrix, 20000, matrix=True)[("kernel", "L32")] == {32}
+    assert groups(matrix, 20000, matrix=True, local=False)[("kernel", "L32")] == {32}
     assert groups(matrix, 60000)[("short", "L16")] == {8}
+    assert groups(general, 60000, local=True)[("kernel", "L16")] == {8}          # its best in local mode
     host.lib.pa_destroy(general)
     host.lib.pa_destroy(matrix)
 
