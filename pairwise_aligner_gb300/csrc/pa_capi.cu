@@ -481,7 +481,8 @@ pa_status ensure_slots(pa_ctx *c, uint64_t columns)
 // them have m * n >= long_cells, L * sqrt(long_cells) <= sqrt(b1 * b2).
 uint64_t most_long(const pa_ctx *c, uint64_t n_pairs, uint64_t b1, uint64_t b2)
 {
-    const double most = std::sqrt((double)b1 * (double)b2 / (double)c->long_cells) + 2.0;
+    // some more, so that growing calls do not allocate each time
+    const double most = std::sqrt((double)b1 * (double)b2 / (double)c->long_cells) + 1024.0;
     return most < (double)n_pairs ? (uint64_t)most : n_pairs;
 }
 

@@ -111,7 +111,7 @@ constexpr int kStage = 16;
 // Pass p of the unit: rows p * rows_full + t * RA + 1 .. + RA (1-based) on thread t.
 template <class V, int MODE, int R, int RA>
 __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q, const DpParams &P, LongUnit &u, int p,
-                                          int32_t rows_full, int t, uint4 *snap, StripShared<V> sh, uint4 *stage,
+                                          int32_t rows_full, int t, uint4 *snap, uint4 *cut, StripShared<V> sh, uint4 *stage,
                                           int32_t *ub)
 {
     using KC = StripConst<V, MODE>;
@@ -200,6 +200,7 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
         for (int l = 0; l < NL; ++l) sh.bi[l][threadIdx.x] = 0;
     }
 
+    const int32_t cut_at = strip_cut_at<V, MODE>(P, u);
     auto step = [&](int32_t s, bool active) {
         const int32_t i = ibase + s - t + 1;
         if ((s & (kStage - 1)) == 0 && s < ms) {
@@ -229,7 +230,9 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
                 strip_track<V, R, RA>(H, best, i, snap, sh);
             else {
                 if (row_end) strip_end_track<V, MODE, RA, kBlock>(u, H, seen, shift_neg, i, r0, r1, snap, sh);
-                if (i >= mmin) strip_ends<V, MODE, RA>(P, u, H, i, j0, any_own, snap, sh, [&](int l) { return own[l]; });
+                else if (i >= mmin)
+                    strip_ends<V, MODE, RA>(P, u, H, i, any_own, snap, sh, [&](int l) { return own[l]; });
+                if (MODE == M_GLOBAL_FREE && NL == 2 && i == cut_at) strip_cut<RA, kBlock>(H, cut);
             }
         }
     };
@@ -247,6 +250,7 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
     }
     if (MODE == M_LOCAL) strip_track_end<V, R, RA>(best, j0, snap, sh);
     if (row_end) strip_end_offer<V, MODE, kBlock>(P, u, own, sh);
+    if (MODE == M_GLOBAL_FREE && P.last_row_free) strip_column_offer<V, MODE, RA, kBlock>(P, u, H, j0, cut, sh);
     if (BAND) {
         // upper bounds on the paths that leave the window (exit_bound): first through its right
         // edge, cells (iend + 1, j), by a horizontal gap from (iend, j) or diagonally from
@@ -439,11 +443,13 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
     constexpr int NW = kBlock / 32;
     constexpr bool BAND = MODE == M_BAND;
     __shared__ uint4 snap_store[(MODE == M_LOCAL ? NL : 1) * (R / 4) * kBlock];
+    __shared__ uint4 cut_store[MODE == M_GLOBAL_FREE && NL == 2 ? (R / 4) * kBlock : 1];
     __shared__ LongUnit s_unit[NW];
     __shared__ uint4 s_stage[NW][2 * kStage];
     __shared__ int32_t s_cand[NL][3][kBlock];
     __shared__ int32_t s_bi[MODE == M_LOCAL ? NL : MODE == M_GLOBAL_FREE ? 2 * NL : 1][kBlock];
     uint4 *snap = snap_store + threadIdx.x;
+    uint4 *cut = cut_store + (MODE == M_GLOBAL_FREE && NL == 2 ? threadIdx.x : 0);
     StripShared<V> sh{s_cand, s_bi};
     const int t = threadIdx.x & 31;
     LongUnit &su = s_unit[threadIdx.x >> 5];
@@ -494,12 +500,12 @@ __global__ void __launch_bounds__(kBlock, 2) dp_long(DpLaunch L, LongQueue Q, Dp
             const int32_t rows_full = 32 * su.rpt, rem = su.nh - p * rows_full;
             const int32_t rpt = rem >= rows_full ? su.rpt : ((rem + 32 * kChunk - 1) / (32 * kChunk)) * kChunk;
             switch (rpt / kChunk) {
-            case 1: long_pass<V, MODE, R, 4>(L, Q, P, su, p, rows_full, t, snap, sh, s_stage[threadIdx.x >> 5], ub); break;
-            case 2: long_pass<V, MODE, R, 8>(L, Q, P, su, p, rows_full, t, snap, sh, s_stage[threadIdx.x >> 5], ub); break;
-            case 3: long_pass<V, MODE, R, 12>(L, Q, P, su, p, rows_full, t, snap, sh, s_stage[threadIdx.x >> 5], ub); break;
-            case 4: long_pass<V, MODE, R, 16>(L, Q, P, su, p, rows_full, t, snap, sh, s_stage[threadIdx.x >> 5], ub); break;
-            case 5: long_pass<V, MODE, R, R >= 20 ? 20 : R>(L, Q, P, su, p, rows_full, t, snap, sh, s_stage[threadIdx.x >> 5], ub); break;
-            default: long_pass<V, MODE, R, R>(L, Q, P, su, p, rows_full, t, snap, sh, s_stage[threadIdx.x >> 5], ub); break;
+            case 1: long_pass<V, MODE, R, 4>(L, Q, P, su, p, rows_full, t, snap, cut, sh, s_stage[threadIdx.x >> 5], ub); break;
+            case 2: long_pass<V, MODE, R, 8>(L, Q, P, su, p, rows_full, t, snap, cut, sh, s_stage[threadIdx.x >> 5], ub); break;
+            case 3: long_pass<V, MODE, R, 12>(L, Q, P, su, p, rows_full, t, snap, cut, sh, s_stage[threadIdx.x >> 5], ub); break;
+            case 4: long_pass<V, MODE, R, 16>(L, Q, P, su, p, rows_full, t, snap, cut, sh, s_stage[threadIdx.x >> 5], ub); break;
+            case 5: long_pass<V, MODE, R, R >= 20 ? 20 : R>(L, Q, P, su, p, rows_full, t, snap, cut, sh, s_stage[threadIdx.x >> 5], ub); break;
+            default: long_pass<V, MODE, R, R>(L, Q, P, su, p, rows_full, t, snap, cut, sh, s_stage[threadIdx.x >> 5], ub); break;
             }
         }
         __syncwarp();

@@ -167,13 +167,13 @@ __device__ __forceinline__ void strip_track_end(uint32_t best, int32_t j0, const
     }
 }
 
-// Global modes, after column i: the candidates of the end rules.  own_row(l) is the strip index
-// of lane l's last row, or -1; the row's H is read back from shared memory, where the thread
-// puts its column first (a chain of selects over the rows cost 60 ALU operations a column, a
-// third of the free-end kernel's time; the stores go to the idle LSU pipe).
+// Global modes, after column i: the end cell of every lane whose last row this thread holds and whose
+// last column this is.  own_row(l) is the strip index of lane l's last row, or -1; the row's H is read
+// back from shared memory, where the thread puts its column first (a chain of selects over the rows
+// cost 60 ALU operations a column; the stores go to the idle LSU pipe).
 template <class V, int MODE, int RA, int NT, class U, class O>
-__device__ __forceinline__ void strip_ends(const DpParams &P, const U &u, const uint32_t *H, int32_t i, int32_t j0,
-                                           bool any_own, uint4 *snap, StripShared<V, NT> &sh, O own_row)
+__device__ __forceinline__ void strip_ends(const DpParams &P, const U &u, const uint32_t *H, int32_t i, bool any_own,
+                                           uint4 *snap, StripShared<V, NT> &sh, O own_row)
 {
     if (any_own) {
 #pragma unroll
@@ -184,22 +184,51 @@ __device__ __forceinline__ void strip_ends(const DpParams &P, const U &u, const 
     for (int l = 0; l < V::LANES; ++l) {
         if (l == 1 && !u.has_b) continue;
         const int32_t base = P.shift * i - StripConst<V, MODE>::Kt, ml = u.m[l], r = own_row(l);
-        if (r >= 0 && (i == ml || (MODE == M_GLOBAL_FREE && P.last_column_free && i < ml))) {
+        if (r >= 0 && i == ml) {
             const uint32_t *q = reinterpret_cast<const uint32_t *>(snap + (r >> 2) * NT);
             sh.offer(l, V::get(q[r & 3], l) + base, i, u.n[l]);
         }
-        if (MODE == M_GLOBAL_FREE && P.last_row_free && i == ml) {
-            // the column's first best row, offered once: an offer per row went to shared memory RA times
-            // (2,000 pairs of 150 x 8,000 with free ends: 4,639 us a call, now 2,174)
-            const int32_t rows = u.n[l] - j0;
-            int32_t top = INT32_MIN, at = -1;
+    }
+}
+
+// ... the column at which the shorter lane ends, if its end rule needs it and it is not the last (else 0:
+// no column), and its store.
+template <class V, int MODE, class U>
+__device__ __forceinline__ int32_t strip_cut_at(const DpParams &P, const U &u)
+{
+    if (V::LANES == 1 || MODE != M_GLOBAL_FREE || !P.last_row_free || !u.has_b || u.m[0] == u.m[1]) return 0;
+    return min(u.m[0], u.m[1]);
+}
+
+template <int RA, int NT>
+__device__ __forceinline__ void strip_cut(const uint32_t *H, uint4 *cut)
+{
 #pragma unroll
-            for (int k = 0; k < RA; ++k) {
-                const int32_t x = V::get(H[k], l);
-                if (k < rows && (x > top || at < 0)) { top = x; at = k; }
-            }
-            if (at >= 0) sh.offer(l, top + base, i, j0 + at + 1);
+    for (int v = 0; v < RA / 4; ++v) cut[v * NT] = make_uint4(H[4 * v], H[4 * v + 1], H[4 * v + 2], H[4 * v + 3]);
+}
+
+// Free end of sequence1's last column: its first best row, offered once after the pass.  The longer
+// lane's column is the last that the thread computed, so H still holds it; the shorter lane's was put
+// into `cut` (16-byte words NT apart) when it was computed.  An offer per row in the column's step took
+// 3,176 us for 60,000 pairs of 64-512 rows with all ends free, the scan in that step 1,710 (and 3-12 %
+// of calls without this end rule, whose loop carried it), 1,323 here.
+template <class V, int MODE, int RA, int NT, class U>
+__device__ __forceinline__ void strip_column_offer(const DpParams &P, const U &u, const uint32_t *H, int32_t j0,
+                                                   const uint4 *cut, StripShared<V, NT> &sh)
+{
+#pragma unroll
+    for (int l = 0; l < V::LANES; ++l) {
+        if (l == 1 && !u.has_b) continue;
+        const int32_t ml = u.m[l], rows = u.n[l] - j0;
+        const bool held = V::LANES == 1 || ml == u.ms;
+        int32_t top = INT32_MIN, at = -1;
+#pragma unroll
+        for (int k = 0; k < RA; ++k) {
+            const uint32_t h = held ? H[k] : reinterpret_cast<const uint32_t *>(cut + (k >> 2) * NT)[k & 3];
+            const int32_t x = V::get(h, l);
+            if (k < rows && (x > top || at < 0)) { top = x; at = k; }
         }
+        if (at >= 0) sh.offer(l, top + P.shift * ml - StripConst<V, MODE>::Kt, ml, j0 + at + 1);
     }
 }
 
@@ -330,8 +359,8 @@ __device__ __forceinline__ void build_profile(uint4 *prof, const uint32_t (*mat)
 // One pass p of the unit: rows p*G*R + t*RA + 1 .. + RA (1-based) on thread t.
 template <class V, int SC, int MODE, int G, int R, int RA, int NT>
 __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P, const ShortUnit &u, int p, int t,
-                                           int32_t ms_min, int32_t ms_max, uint4 *snap, StripShared<V, NT> sh, uint4 *prof,
-                                           const uint32_t (*mat)[8])
+                                           int32_t ms_min, int32_t ms_max, uint4 *snap, uint4 *cut,
+                                           StripShared<V, NT> sh, uint4 *prof, const uint32_t (*mat)[8])
 {
     using KC = StripConst<V, MODE>;
     constexpr int NL = V::LANES;
@@ -390,6 +419,7 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
         for (int l = 0; l < NL; ++l) sh.bi[l][threadIdx.x] = 0;
     }
 
+    const int32_t cut_at = strip_cut_at<V, MODE>(P, u);
     // step s of the pass: thread t computes column i = s - t + 1 when 1 <= i <= ms
     auto step = [&](int32_t s, bool active) {
         const int32_t i = s - t + 1;
@@ -427,8 +457,10 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
                 strip_track<V, R, RA>(H, best, i, snap, sh);
             else {
                 if (row_end) strip_end_track<V, MODE, RA, NT>(u, H, seen, shift_neg, i, r0, r1, snap, sh);
-                if (i >= mmin)
-                    strip_ends<V, MODE, RA>(P, u, H, i, j0, any_own, snap, sh, [&](int l) { return own[l]; });
+                if (i >= mmin) {
+                    strip_ends<V, MODE, RA>(P, u, H, i, any_own, snap, sh, [&](int l) { return own[l]; });
+                    if (MODE == M_GLOBAL_FREE && NL == 2 && i == cut_at) strip_cut<RA, NT>(H, cut);
+                }
             }
         }
     };
@@ -445,6 +477,7 @@ __device__ __forceinline__ void short_pass(const DpLaunch &L, const DpParams &P,
     for (; s < ms_max + G - 1; ++s) step(s, (uint32_t)(s - t) < (uint32_t)ms);
     if (MODE == M_LOCAL) strip_track_end<V, R, RA>(best, j0, snap, sh);
     if (row_end) strip_end_offer<V, MODE, NT>(P, u, own, sh);
+    if (MODE == M_GLOBAL_FREE && P.last_row_free && ms > 0) strip_column_offer<V, MODE, RA, NT>(P, u, H, j0, cut, sh);
 }
 
 // With fewer work items than warps, only the first warps of every block take any: otherwise the
@@ -459,8 +492,8 @@ __device__ __forceinline__ bool strip_warp_takes_part(uint32_t items)
 // position `end`, a group's first pair at first + g * lanes.
 template <class V, int SC, int MODE, int G, int R, int NT>
 __device__ __forceinline__ void short_unit(const DpLaunch &L, const DpParams &P, const uint32_t *order, uint32_t first,
-                                           uint32_t end, ShortUnit *s_unit, uint4 *snap, StripShared<V, NT> sh,
-                                           uint4 *prof, const uint32_t (*mat)[8])
+                                           uint32_t end, ShortUnit *s_unit, uint4 *snap, uint4 *cut,
+                                           StripShared<V, NT> sh, uint4 *prof, const uint32_t (*mat)[8])
 {
     constexpr int NL = V::LANES;
     const int lane = threadIdx.x & 31;
@@ -525,7 +558,7 @@ __device__ __forceinline__ void short_unit(const DpLaunch &L, const DpParams &P,
         const int32_t ms = p < u.passes ? u.ms : 0;
         const int32_t ms_min = __reduce_min_sync(0xffffffffu, ms), ms_max = __reduce_max_sync(0xffffffffu, ms);
 #define PA_SHORT_PASS(RA) \
-    short_pass<V, SC, MODE, G, R, (R >= RA ? RA : R), NT>(L, P, u, p, t, ms_min, ms_max, snap, sh, prof, mat)
+    short_pass<V, SC, MODE, G, R, (R >= RA ? RA : R), NT>(L, P, u, p, t, ms_min, ms_max, snap, cut, sh, prof, mat)
         switch (rpt / kChunk) {
         case 1: PA_SHORT_PASS(4); break;
         case 2: PA_SHORT_PASS(8); break;
@@ -570,12 +603,14 @@ __global__ void __launch_bounds__(NT, 512 / NT) dp_short(DpLaunch L, DpParams P)
     static_assert(R % kChunk == 0 && R <= 32, "R must be a multiple of the chunk");
     constexpr int NL = V::LANES;
     __shared__ uint4 snap_store[(MODE == M_LOCAL ? NL : 1) * (R / 4) * NT];
+    __shared__ uint4 cut_store[MODE == M_GLOBAL_FREE && NL == 2 ? (R / 4) * NT : 1];
     __shared__ ShortUnit s_unit[NT / G];
     __shared__ int32_t s_cand[NL][3][NT];
     __shared__ int32_t s_bi[MODE == M_LOCAL ? NL : MODE == M_GLOBAL_FREE ? 2 * NL : 1][NT];
     __shared__ uint32_t s_mat[SC == SC_PROFILE ? 33 : 1][8];
     extern __shared__ uint4 s_prof[];
     uint4 *snap = snap_store + threadIdx.x;
+    uint4 *cut = cut_store + (MODE == M_GLOBAL_FREE && NL == 2 ? threadIdx.x : 0);
     uint4 *prof = s_prof + threadIdx.x;
     StripShared<V, NT> sh{s_cand, s_bi};
     const uint32_t count = *L.count_ptr;
@@ -598,7 +633,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) dp_short(DpLaunch L, DpParams P)
         if ((threadIdx.x & 31) == 0) uu = atomicAdd(L.unit_counter, 1u);
         uu = __shfl_sync(0xffffffffu, uu, 0);
         if (uu >= n_units) break;
-        short_unit<V, SC, MODE, G, R, NT>(L, P, order, (n_units - 1 - uu) * ppw, count, s_unit, snap, sh, prof, s_mat);
+        short_unit<V, SC, MODE, G, R, NT>(L, P, order, (n_units - 1 - uu) * ppw, count, s_unit, snap, cut, sh, prof, s_mat);
         __syncwarp();
     }
 }
