@@ -182,13 +182,17 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
     int32_t own[NL];
     bool any_own = false;
     int32_t mmin = u.ms;
+    auto find_row = [&](int l) -> int32_t {
+        const int32_t r = (u.n[l] - 1) - j0;
+        return MODE != M_LOCAL && r >= 0 && r < RA && (u.n[l] - 1) / rows_full == p ? r : -1;
+    };
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
-        const int32_t r = (u.n[l] - 1) - j0;
-        own[l] = MODE != M_LOCAL && r >= 0 && r < RA && (u.n[l] - 1) / rows_full == p ? r : -1;
+        own[l] = find_row(l);
         any_own |= own[l] >= 0;
         mmin = min(mmin, u.m[l]);
     }
+    auto own_row = [&](int l) { return BAND ? find_row(l) : own[l]; };   // band mode has no registers to keep it
     // the end rule of the last row (strip_end_track; with a comparison in shared memory on every column
     // a free-end pair of 200,000 x 100 took 132.6 ms, now 86.6)
     const bool row_end = MODE == M_GLOBAL_FREE && P.last_column_free && any_own;
@@ -231,7 +235,7 @@ __device__ __forceinline__ void long_pass(const DpLaunch &L, const LongQueue &Q,
             else {
                 if (row_end) strip_end_track<V, MODE, RA, kBlock>(u, H, seen, shift_neg, i, r0, r1, snap, sh);
                 else if (i >= mmin)
-                    strip_ends<V, MODE, RA>(P, u, H, i, any_own, snap, sh, [&](int l) { return own[l]; });
+                    strip_ends<V, MODE, RA>(P, u, H, i, any_own, snap, sh, own_row);
                 if (MODE == M_GLOBAL_FREE && NL == 2 && i == cut_at) strip_cut<RA, kBlock>(H, cut);
             }
         }
