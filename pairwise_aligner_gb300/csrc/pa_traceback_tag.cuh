@@ -19,10 +19,10 @@
 // holds a word per lane (ra <= 8) or two; row k of a lane's first word is its nibble k (of a
 // shorter strip: k + 8 - ra), rows 8.. are in the second (nibble k - 8 + 16 - ra).
 //
-// Bound: the integer ALU pipe and, with eight strip heights instead of four, the instruction cache
-// (neighbouring warps run last passes of different heights): 4,096 global pairs of 500-2,000 rows
-// 16.96 ms per call with one pair per warp and compares, 7.6 with heights in steps of 2, 6.4 in
-// steps of 4.
+// Bound: the integer ALU pipe, 76 % busy over the 4.74 ms of k_tb_dp (the last passes are padded to
+// 128 rows), and the host copies around it: 4,096 global pairs of 500-2,000 rows 6.4 ms per call, 17.0
+// with one pair per warp and compares.  Strip heights in steps of 2 instead of 4: 7.6, as eight bodies
+// do not stay in the instruction cache (neighbouring warps run last passes of different heights).
 #pragma once
 #include "pa_long.cuh"
 
