@@ -246,7 +246,9 @@ pa_status pa_mlp_to_bf16(const float *src, int rows, int cols, int ld_dst, void 
 /* Pairs with at least `cells` = m * n cells are long: their row passes are spread over
  * many warps (unitary DNA scores: one queue of passes for the whole GPU; other scores:
  * the warps of a block) instead of running on one group of lanes; default 2^20.  1 makes
- * every pair long, UINT64_MAX none. */
+ * every pair long, UINT64_MAX none.  At 2^20 and above, pairs of at most 128 rows (few
+ * pairs) or 384 columns (a batch full of narrow, tall pairs) that would have a group of 32
+ * lanes stay there: one warp runs them as well. */
 pa_status pa_set_cta_threshold(pa_ctx *ctx, uint64_t cells);
 
 /* Calls the context keeps captured as CUDA graphs (replayed when a call repeats the
@@ -336,8 +338,7 @@ pa_status pa_align_batch_banded(pa_ctx *ctx, const pa_config *config,
  * and pair-size class: size class s = 0..3 when n_pairs < 2^(12 + 2s), else 4; pair-size
  * class h = 0..2 when the mean m*n per pair < 2^(14 + 2h), else 3.  An entry with
  * group_threads 0 falls back to variant_s16 / group_threads_s16; when that group size is
- * 0 too and variant_s16 is a short-pair variant, the rule also picks its rows per thread
- * (32 for groups of up to 8 lanes, else 16). */
+ * 0 too and variant_s16 is a short-pair variant, it runs with 32 rows per thread. */
 #define PA_TUNE_SIZES 5
 #define PA_TUNE_SHAPES 4
 typedef struct pa_tune_entry {
